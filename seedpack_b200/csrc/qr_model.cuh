@@ -55,22 +55,22 @@ SG_DEVINL int u16(const uchar* b) { return b[0] | (b[1] << 8); }
 SG_DEVINL unsigned u32(const uchar* b) { return b[0] | (b[1] << 8) | (b[2] << 16) | ((unsigned)b[3] << 24); }
 SG_DEVINL float h2f(const uchar* p) { return h2fv((unsigned)u16(p)); }
 
-__host__ SG_DEVINL int qk_of(int T) { return (T == 2 || T == 3 || T == 6 || T == 7 || T == 8 || T == 20) ? 32 : T == 42 ? 64 : 256; }
-SG_DEVINL int bs_of(int T) {
+constexpr __host__ SG_DEVINL int qk_of(int T) { return (T == 2 || T == 3 || T == 6 || T == 7 || T == 8 || T == 20) ? 32 : T == 42 ? 64 : 256; }
+constexpr __host__ SG_DEVINL int bs_of(int T) {
     switch (T) { case 2: return 18; case 3: return 20; case 6: return 22; case 7: return 24; case 8: return 34; case 10: return 84;
                  case 11: return 110; case 12: return 144; case 13: return 176; case 14: return 210; case 20: return 18;
                  case 23: return 136; case 42: return 18; case 16: return 66; case 17: return 74; case 18: return 98;
                  case 19: return 50; case 21: return 110; case 22: return 82; case 29: return 56; }
     return 1;
 }
-__host__ SG_DEVINL bool is_grid(int T) { return T == 16 || T == 17 || T == 18 || T == 19 || T == 21 || T == 22 || T == 29; }
-SG_DEVINL int qmin_of(int T) { return T == 8 ? -128 : 0; }
-SG_DEVINL int qmax_of(int T) {
+constexpr __host__ SG_DEVINL bool is_grid(int T) { return T == 16 || T == 17 || T == 18 || T == 19 || T == 21 || T == 22 || T == 29; }
+constexpr __host__ SG_DEVINL int qmin_of(int T) { return T == 8 ? -128 : 0; }
+constexpr __host__ SG_DEVINL int qmax_of(int T) {
     switch (T) { case 10: case 42: return 3; case 11: return 7; case 6: case 7: case 13: return 31; case 14: return 63; case 8: return 127; }
     return 15;
 }
-SG_DEVINL bool nonlin(int T) { return T == 20 || T == 23; }
-SG_DEVINL int sublen_of(int T) { return (T == 10 || T == 11 || T == 14) ? 16 : 32; }
+constexpr __host__ SG_DEVINL bool nonlin(int T) { return T == 20 || T == 23; }
+constexpr __host__ SG_DEVINL int sublen_of(int T) { return (T == 10 || T == 11 || T == 14) ? 16 : 32; }
 
 SG_DEVINL void scale_min_k4(int j, const uchar* q, int& sc, int& m) {
     if (j < 4) { sc = q[j] & 63; m = q[j + 4] & 63; }
@@ -131,14 +131,14 @@ SG_DEVINL void put_code(int T, uchar* b, int w, int q) {
 // ---- scale fields ------------------------------------------------------------------------------------------
 // A block's scale fields as an integer vector: [0] fp16 scale (bits), [1] fp16 min where the type has one, then
 // the sub-block scales (and sub-block mins).  unpack_fields / pack_fields are inverse on every valid block.
-__host__ SG_DEVINL int nfield(int T) {
+constexpr __host__ SG_DEVINL int nfield(int T) {
     switch (T) { case 2: case 6: case 8: case 20: case 42: return 1; case 3: case 7: return 2; case 10: return 34;
                  case 11: case 14: return 17; case 12: case 13: return 18; case 23: return 9;
                  case 16: case 18: case 19: case 21: return 9; case 17: case 22: case 29: return 17; }
     return 0;
 }
 // 0 fp16 scale, 1 fp16 min, 2 sub-scale, 3 sub-min
-SG_DEVINL int fkind(int T, int k) {
+constexpr __host__ SG_DEVINL int fkind(int T, int k) {
     if (k == 0) return 0;
     const bool has_min = T == 3 || T == 7 || T == 10 || T == 12 || T == 13;
     if (k == 1 && has_min) return 1;
@@ -328,11 +328,11 @@ SG_DEVINL void predict_code(int T, float a, float c, const uchar* pblk, int w, f
 
 // ==== grid (IQ) types ===========================================================================================
 // A unit = 8 consecutive weights: one lattice point (IQ3: two points of 4), one sign group, one scale.
-SG_DEVINL int grid_size(int T) {
+constexpr __host__ SG_DEVINL int grid_size(int T) {
     switch (T) { case 16: case 18: return 256; case 17: case 21: return 512; case 22: return 1024; }
     return 2048;
 }
-SG_DEVINL bool parity_type(int T) { return T == 16 || T == 17 || T == 18; }      // 7 stored sign bits + parity
+constexpr __host__ SG_DEVINL bool parity_type(int T) { return T == 16 || T == 17 || T == 18; }      // 7 stored sign bits + parity
 
 // where the index of lattice group g is kept: 8 low bits in a byte, the rest (1-3 bits) elsewhere
 struct GidxLoc { int lo_byte, hi_byte, hi_shift, hi_bits; };
