@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(32) k_chain_enc(const uint8_t* __restrict__ sy
         if (wr.ptr() < slot + 32) { out_len[c] = LEN_OVERFLOW; return; }
     }
     rans_flush(x, wr);
-    wr.flush(slot);
+    wr.flush();
     out_len[c] = wr.bad ? (unsigned long long)LEN_NOFREQ : (unsigned long long)(end - wr.ptr());
 }
 

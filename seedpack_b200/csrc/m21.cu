@@ -23,28 +23,22 @@ namespace m21 {
 struct Meta { int first, nblocks, nb_row, grp, colbase, rowbase, off, qset; };
 
 // ByteWriterDown that knows where its slot begins: the reference sizes these slots for typical data (68 bytes a block)
-// and does not look; here a window that would land below the slot is not stored and the segment reports an overflow
-struct SlotWriter {
-    uint8_t* base; unsigned long long lo, hi; int pos; unsigned bad; uint8_t* lim; bool over;
-    SG_DEVINL void init(uint8_t* end, uint8_t* slot_begin) { base = end - 16; lo = hi = 0; pos = 16; bad = 0; lim = slot_begin; over = false; }
-    SG_DEVINL void put(unsigned b) {
-        --pos;
-        if (pos >= 8) hi |= (unsigned long long)b << (8 * (pos - 8));
-        else          lo |= (unsigned long long)b << (8 * pos);
-        if (pos == 0) {
-            if (base >= lim) *reinterpret_cast<ulonglong2*>(base) = make_ulonglong2(lo, hi); else over = true;
-            base -= 16; lo = hi = 0; pos = 16;
+// and does not look; here a word that would land below the slot is not stored and the segment reports an overflow
+struct SlotWriter : ByteWriterDown {
+    uint8_t* lim; bool over;
+    SG_DEVINL void init(uint8_t* end, uint8_t* slot_begin) { ByteWriterDown::init(end); lim = slot_begin; over = false; }
+    SG_DEVINL void emit(unsigned x, int n) {
+        if (push(x, n)) {
+            cnt -= 4;
+            if (over || p - 4 < lim) over = true;
+            else { p -= 4; *reinterpret_cast<unsigned*>(p) = (unsigned)(acc >> (8 * cnt)); }
         }
     }
-    SG_DEVINL uint8_t* ptr() const { return base + pos; }
-    // the partial window; -> the segment's length, or the overflow mark
+    // the pending bytes; -> the segment's length, or the overflow mark
     SG_DEVINL unsigned finish(uint8_t* end) {
         if (over || ptr() < lim) return LEN_OVERFLOW;
-        if (pos < 16) {
-            if (base >= lim) *reinterpret_cast<ulonglong2*>(base) = make_ulonglong2(lo, hi);
-            else for (int k = pos; k < 16; ++k) base[k] = (uint8_t)((k >= 8 ? hi >> (8 * (k - 8)) : lo >> (8 * k)) & 0xff);
-        }
-        return bad ? LEN_NOFREQ : (unsigned)(end - ptr());
+        flush();
+        return bad ? LEN_NOFREQ : (unsigned)(end - p);
     }
 };
 

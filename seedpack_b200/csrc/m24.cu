@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(64) k_enc(const unsigned char* __restrict__ fi
         if (--j < 0) { j = T.rowlen - 1; --r; if (k > 0) rf = sd.rfi[T.rowbase + r]; }
     }
     rans_flush(x, wr);
-    wr.flush(slot);
+    wr.flush();
     out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
 }
 

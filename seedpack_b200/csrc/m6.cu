@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(128) k_enc(const unsigned char* __restrict__ b
         if (wr.ptr() < slot + 96) { out_len[s] = LEN_OVERFLOW; return; }         // a block writes at most 70 bytes
     }
     rans_flush(x, wr);
-    wr.flush(slot);
+    wr.flush();
     out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
 }
 

@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(QR_TPB) k_qr_enc(const Args a, const RansSym* 
     }
     if (c.ovf) { out_len[s] = 0xffffffffu; return; }
     rans_flush(c.x, c.wr);
-    c.wr.flush(c.slot);
+    c.wr.flush();
     out_len[s] = c.wr.bad ? LEN_NOFREQ : (unsigned)(c.slot + cap - c.wr.ptr());
 }
 
@@ -688,35 +688,59 @@ __global__ void __launch_bounds__(256) k_qr_stage_hist(long long nblocks, const 
     }
 }
 
-// the coder proper: one lane per segment, blocks last to first, each block's staged pairs in order
-__global__ void __launch_bounds__(QR_TPB) k_qr_stage_code(const SG* __restrict__ sg, int nseg, const unsigned* __restrict__ stage,
-                                                           const unsigned short* __restrict__ cnt, int capb, const RansSym* __restrict__ enc,
-                                                           uchar* __restrict__ out, size_t cap, unsigned* __restrict__ out_len) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
+// The coder proper: one lane per segment, blocks last to first, each block's staged pairs in order.  Bound by the lane's
+// chain: pairs are taken eight at a time, asked for two groups ahead, their table entries one group ahead; a block's last
+// group is filled with entries that leave the state as it is, so that the step has no branch.
+__global__ void __launch_bounds__(32) k_qr_stage_code(const SG* __restrict__ sg, int nseg, const unsigned* __restrict__ stage,
+                                                      const unsigned short* __restrict__ cnt, int capb, const RansSym* __restrict__ enc,
+                                                      uchar* __restrict__ out, size_t cap, unsigned* __restrict__ out_len, int spw) {
+    const int s = blockIdx.x * spw + threadIdx.x;
+    if ((int)threadIdx.x >= spw || s >= nseg) return;
     const SG g = sg[s];
     uchar* slot = out + (size_t)s * cap;
     ByteWriterDown wr; wr.init(slot + cap);
     unsigned x = RANS_L;
-    bool ovf = false;
-    for (long long b = g.b0 + g.nb - 1; b >= g.b0 && !ovf; --b) {
-        const int n = cnt[b];
-        const unsigned* p = stage + (size_t)b * capb;
-        int i = 0;
-        for (; i + 4 <= n; i += 4) {            // table entries do not depend on the coder state: four loads in flight
-            const uint4 e4 = *reinterpret_cast<const uint4*>(p + i);
-            const RansSym s0 = enc[e4.x], s1 = enc[e4.y], s2 = enc[e4.z], s3 = enc[e4.w];
-            rans_put<12>(x, wr, s0); rans_put<12>(x, wr, s1); rans_put<12>(x, wr, s2); rans_put<12>(x, wr, s3);
-            if (wr.ptr() < slot + 64) { ovf = true; break; }
+    long long b = g.b0 + g.nb;                          // block of the group asked for last
+    int i = 0, n = 0, nn = g.nb > 0 ? cnt[b - 1] : 0;   // next pair of it, its pairs, the pairs of the block before it
+    uint4 pa = make_uint4(0, 0, 0, 0), pc = pa;
+    int m0 = 0;
+    auto load = [&]() {                                 // m0 = 0: no group left (a block has one pair at least)
+        if (i >= n) {
+            --b; i = 0;
+            n = b >= g.b0 ? nn : 0;
+            if (b - 1 >= g.b0) nn = cnt[b - 1];
         }
-        for (; i < n && !ovf; ++i) {
-            rans_put<12>(x, wr, enc[p[i]]);
-            if (wr.ptr() < slot + 64) ovf = true;
-        }
+        m0 = min(8, n - i);
+        if (m0 > 0) {
+            const unsigned* p = stage + (size_t)b * capb + i;
+            pa = *reinterpret_cast<const uint4*>(p);
+            if (m0 > 4) pc = *reinterpret_cast<const uint4*>(p + 4);
+        } else { m0 = 0; n = i = 0; b = g.b0; }
+        i += 8;
+    };
+    const RansSym nop = {RANS_NOP_RCP, 4096u};
+    auto look = [&](RansSym (&e)[8]) {
+        const unsigned w[8] = {pa.x, pa.y, pa.z, pa.w, pc.x, pc.y, pc.z, pc.w};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { e[k] = nop; if (k < m0) e[k] = enc[w[k]]; }
+    };
+    RansSym cur[8], nxt[8];
+    load();
+    look(cur);
+    int m = m0;
+    load();
+    while (m > 0) {
+        look(nxt);
+        m = m0;
+        load();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) rans_put<12>(x, wr, cur[k]);
+        if (wr.ptr() < slot + 64) { out_len[s] = LEN_OVERFLOW; return; }       // 8 symbols write at most 16 bytes
+#pragma unroll
+        for (int k = 0; k < 8; ++k) cur[k] = nxt[k];
     }
-    if (ovf) { out_len[s] = 0xffffffffu; return; }
     rans_flush(x, wr);
-    wr.flush(slot);
+    wr.flush();
     out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
 }
 
@@ -861,8 +885,9 @@ extern "C" int sg_qr_stage_encode(int device, void* stream, int T, long long nbl
     if (nseg == 0) return SG_OK;
     int rc = use_device(device);
     if (rc != SG_OK) return rc;
-    k_qr_stage_code<<<(nseg + QR_TPB - 1) / QR_TPB, QR_TPB, 0, (cudaStream_t)stream>>>(
+    const int spw = segs_per_warp(nseg);
+    k_qr_stage_code<<<(nseg + spw - 1) / spw, 32, 0, (cudaStream_t)stream>>>(
         (const SG*)sgp, nseg, (const unsigned*)((const uchar*)stage + stage_cnt_bytes(nblocks)), (const unsigned short*)stage, capb,
-        (const RansSym*)enc_tab, slots, cap, out_len);
+        (const RansSym*)enc_tab, slots, cap, out_len, spw);
     return cuda_ok(cudaGetLastError());
 }

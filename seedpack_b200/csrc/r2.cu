@@ -16,7 +16,6 @@ namespace sg {
 namespace r2 {
 
 constexpr int PB = 15;
-constexpr int TPB = 64;
 
 struct TB { long long doff; int rowlen, rowbase, colbase, tab, rmap, pad; };       // bf16v2.py:158
 struct SG { int t, n; long long i0; };                                             // bf16v2.py:159
@@ -129,150 +128,261 @@ __global__ void __launch_bounds__(R2H_WARPS * 32) k_r2_hist(const unsigned char*
         }
 }
 
-// Encoder: a few lanes per segment, like the decoder below.  The table entries of a weight's three symbols depend on the
-// data only, not on the coder state: for every 32 weights (taken from the segment's end backwards) the lanes look
-// them up side by side into shared memory, and lane 0 runs the chain over the 96 staged entries.  Four lanes per segment:
-// the chain is what a warp spends its issue slots on, and a warp instruction of the chain then serves eight segments.
-constexpr int EG = 4, EB = 32, ESEG = 32, EW = EB / EG;          // lanes per segment, weights per batch, segments per CTA, weights per lane
-__global__ void __launch_bounds__(EG * ESEG) k_r2_enc(const unsigned char* __restrict__ dev, const TB* __restrict__ tb, const SG* __restrict__ sg,
+// Encoder.  What a weight's three symbols are coded with depends on the data only, not on the coder state, and a segment's
+// state is one chain.  So the CTA's first warp runs the chains of its 32 segments, a segment per lane, over table entries
+// staged in shared memory, while four more warps stage the next 32 weights of every segment (from the segments' ends
+// backwards; four lanes a segment, three dependent loads a weight): the loads' latency is hidden behind the chains.
+// Bound by the chain of 96 steps per batch.
+constexpr int EB = 32, ESEG = 32, EG = 4, EW = EB / EG;          // weights per batch, segments per CTA, staging lanes per segment
+constexpr int E_THREADS = 32 + EG * ESEG, E_PITCH = EB * 3 + 1;  // padded: the chain lanes read the same weight of their rows together
+constexpr int E_SMEM = 2 * ESEG * E_PITCH * (int)sizeof(RansSym);
+__global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __restrict__ dev, const TB* __restrict__ tb, const SG* __restrict__ sg,
                                                       int nseg, Ctx c, const RansSym* __restrict__ enc, unsigned char* __restrict__ out, size_t cap,
                                                       unsigned* __restrict__ out_len) {
-    // per weight of the batch: sign, mantissa, exponent entries (coding order); a row is padded by one entry so that the
-    // chain lanes of a warp's segments, which read the same weight of their rows together, hit different banks
-    __shared__ RansSym s_e[ESEG][EB * 3 + 1];
-    const int grp = threadIdx.x / EG, gl = threadIdx.x % EG;
+    // per weight of a batch: sign, mantissa, exponent entries (coding order); two batches
+    extern __shared__ __align__(16) RansSym s_e[];
+    __shared__ int s_nmax;
+    const bool chain = threadIdx.x < 32;
+    const int grp = chain ? threadIdx.x : (threadIdx.x - 32) / EG, gl = (threadIdx.x - 32) % EG;
     const int s = blockIdx.x * ESEG + grp;
     const bool live = s < nseg;
     SG g; g.t = 0; g.n = 0; g.i0 = 0;
     if (live) g = sg[s];
     const TB T = tb[g.t];
-    int nmax = g.n;
-    for (int o = 16; o; o >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
+    if (threadIdx.x == 0) s_nmax = 0;
+    __syncthreads();
+    if (chain) atomicMax(&s_nmax, g.n);
+    __syncthreads();
+    const int nb_max = (s_nmax + EB - 1) / EB;
     unsigned char* slot = out + (size_t)(live ? s : 0) * cap;
     ByteWriterDown wr; wr.init(slot + cap);
     unsigned x = RANS_L;
     bool full = false;
     const unsigned short* base = reinterpret_cast<const unsigned short*>(dev + T.doff);
-    // batches of 32 weights, the last one first; this lane's first weight of the batch: compact row rc, column j
-    const int nb_max = (nmax + EB - 1) / EB;
+    // batches of 32 weights, the last one first; a staging lane's first weight of the batch: compact row rc, column j
     int rc = 0, j = 0;
-    {
+    if (!chain && live) {
         const long long i = g.i0 + (long long)(nb_max - 1) * EB + EW * gl;
-        if (live) { rc = (int)(i / T.rowlen); j = (int)(i % T.rowlen); }
+        rc = (int)(i / T.rowlen); j = (int)(i % T.rowlen);
     }
-    for (int b = nb_max - 1; b >= 0; --b) {
-        const int k0 = b * EB;
-        {
-            int r = rc, col = j, have = -1, orow = 0;
+    for (int it = 0; it <= nb_max; ++it) {
+        if (!chain) {
+            const int k0 = (nb_max - 1 - it) * EB;
+            RansSym* row = s_e + ((it & 1) * ESEG + grp) * E_PITCH + 3 * EW * gl;
+            if (live && k0 >= 0 && k0 < g.n) {
+                int r = rc, col = j, have = -1, orow = 0;
 #pragma unroll
-            for (int v = 0; v < EW; ++v) {
-                const int k = k0 + EW * gl + v;
-                if (live && k < g.n) {
-                    if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
-                    const unsigned u = base[(size_t)orow * T.rowlen + col];
-                    const int ex = (u >> 7) & 255, man = u & 127, sgn = u >> 15;
-                    int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
-                    s_e[grp][3 * (EW * gl + v)] = enc[(size_t)(T.tab + 640 + sc) * 256 + sgn];
-                    s_e[grp][3 * (EW * gl + v) + 1] = enc[(size_t)(T.tab + 512 + mctx(ex, pred)) * 256 + man];
-                    s_e[grp][3 * (EW * gl + v) + 2] = enc[(size_t)(T.tab + pe) * 256 + ex];
-                    if (++col == T.rowlen) { col = 0; ++r; }
+                for (int v = 0; v < EW; ++v) {
+                    const int k = k0 + EW * gl + v;
+                    if (k < g.n) {
+                        if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
+                        const unsigned u = base[(size_t)orow * T.rowlen + col];
+                        const int ex = (u >> 7) & 255, man = u & 127, sgn = u >> 15;
+                        int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
+                        row[3 * v] = enc[(size_t)(T.tab + 640 + sc) * 256 + sgn];
+                        row[3 * v + 1] = enc[(size_t)(T.tab + 512 + mctx(ex, pred)) * 256 + man];
+                        row[3 * v + 2] = enc[(size_t)(T.tab + pe) * 256 + ex];
+                        if (++col == T.rowlen) { col = 0; ++r; }
+                    }
                 }
             }
-        }
-        __syncwarp();
-        if (live && gl == 0 && !full && k0 < g.n) {
-            const int n = min(EB, g.n - k0);
+            j -= EB;
+            if (live) while (j < 0) { j += T.rowlen; --rc; }
+        } else if (it > 0 && live && !full) {
+            const int n = min(EB, g.n - (nb_max - it) * EB);
+            const RansSym* row = s_e + (((it - 1) & 1) * ESEG + grp) * E_PITCH;
+#pragma unroll 4
             for (int w = n - 1; w >= 0; --w) {
-                rans_put<PB>(x, wr, s_e[grp][3 * w]);
-                rans_put<PB>(x, wr, s_e[grp][3 * w + 1]);
-                rans_put<PB>(x, wr, s_e[grp][3 * w + 2]);
-                if ((w & 3) == 0 && wr.ptr() < slot + 64) { full = true; break; }
+                rans_put<PB>(x, wr, row[3 * w]);
+                rans_put<PB>(x, wr, row[3 * w + 1]);
+                rans_put<PB>(x, wr, row[3 * w + 2]);
+                if (wr.ptr() < slot + 64) { full = true; break; }
             }
         }
-        __syncwarp();
-        j -= EB;
-        if (live) while (j < 0) { j += T.rowlen; --rc; }
+        __syncthreads();
     }
-    if (live && gl == 0) {
+    if (chain && live) {
         if (full) out_len[s] = LEN_OVERFLOW;
         else {
             rans_flush(x, wr);
-            wr.flush(slot);
+            wr.flush();
             out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
         }
     }
 }
 
-// Decoder: a segment is one rANS chain by format, but what a weight's symbols are decoded WITH - the exponent's and the
-// sign's tables, the prediction the mantissa's table is picked by - depends on its row and column only.  Four lanes
-// share a segment: for every 32 weights they look the contexts up side by side (eight weights each) into shared memory,
-// lane 0 then runs the chain over the staged contexts - three table walks per weight and nothing else - and all four
-// store the 32 decoded weights.  Eight segments per warp decode in lockstep.
-constexpr int DG = 4, DB = 32, DSEG = 32, DW = DB / DG;          // lanes per segment, weights per batch, segments per CTA, weights per lane
-__global__ void __launch_bounds__(DG * DSEG) k_r2_dec(const unsigned char* __restrict__ in, const unsigned long long* __restrict__ in_off,
-                                                      const unsigned long long* __restrict__ in_end, unsigned char* __restrict__ dev,
-                                                      const TB* __restrict__ tb, const SG* __restrict__ sg, int nseg, Ctx c,
-                                                      const RansSym* __restrict__ enc, const unsigned char* __restrict__ lut, int* __restrict__ status) {
-    // rows padded: the chain lanes of a warp's segments touch the same weight of their rows together
-    __shared__ int s_t0[DSEG][DB + 1], s_pred[DSEG][DB + 1], s_t2[DSEG][DB + 1];
-    __shared__ unsigned short s_out[DSEG][DB + 2];
-    const int grp = threadIdx.x / DG, gl = threadIdx.x % DG;
-    const int s = blockIdx.x * DSEG + grp;
-    const bool live = s < nseg;
+// Decoder.  A segment is one rANS chain by format, but what a weight's symbols are decoded WITH - the exponent's and the
+// sign's tables, the prediction the mantissa's table is picked by - depends on its row and column only.  A CTA (one per SM)
+// takes up to 64 segments, as few as fill the SMs: four warps run the chains, a segment per lane, over contexts that eight
+// more warps (four lanes a segment) stage for the next 32 weights while they store the 32 weights before.
+// The chain is three table searches per weight, and what they cost is the memory the tables are in: 656 tables do not fit
+// the L1.  In shared memory are, of the role of the CTA's first segment, the 128 mantissa tables, 16 sign tables and the
+// exponent tables of 128 contexts (16 octaves) around that segment's first weight, each as the cumulated frequencies plus
+// the symbol that holds every 128th slot; anything else goes through the tables in global memory.
+constexpr int DB = 32, DSEG = 64, DG = 4, DW = DB / DG;          // weights per batch, segments per CTA, staging lanes per segment and their weights
+constexpr int D_CHAIN = 128, D_THREADS = D_CHAIN + DG * DSEG;
+constexpr int D_ECTX = 128, D_MCTX = 128, D_MP = 256 + 260, D_EP = 256 + 516;       // bytes per table: 256 coarse, 130 / 258 cumulated
+struct DecSmem {
+    unsigned ring[RING_WORDS * DSEG];
+    unsigned ctx[2][DSEG][DB + 1];                               // pe | sc << 9 | pred << 16; rows padded
+    unsigned sign[16];                                           // frequency of symbol 0 | of symbol 1 << 16
+    unsigned short out[2][DSEG][DB + 2];
+    uint8_t mant[D_MCTX * D_MP], expo[D_ECTX * D_EP];
+    int nmax, pe0, bad;
+};
+// stage a compact table; false: it has symbols from `nsym` on, or is not a whole distribution (an unused one)
+SG_DEVINL void stage_table(const uint8_t* __restrict__ ct, uint8_t* dst, int nsym, int lane, int& bad) {
+    const unsigned* __restrict__ words = reinterpret_cast<const unsigned*>(ct + 256);
+    for (int i = lane; i < 64; i += 32) reinterpret_cast<unsigned*>(dst)[i] = reinterpret_cast<const unsigned*>(ct)[i];
+    unsigned short* cum = reinterpret_cast<unsigned short*>(dst + 256);
+    for (int i = lane; i < nsym; i += 32) cum[i] = (unsigned short)(words[i] >> 16);
+    if (lane == 0) {
+        const unsigned w = words[nsym - 1];
+        const unsigned tot = (w >> 16) + (w & 0xffffu);
+        cum[nsym] = (unsigned short)tot;
+        cum[nsym + 1] = 0xffff;
+        if (tot != (1u << PB)) bad = 1;
+    }
+}
+template <int NSYM> SG_DEVINL unsigned get_staged(unsigned& x, RingReader& r, const uint8_t* t) {
+    const unsigned short* cum = reinterpret_cast<const unsigned short*>(t + 256);
+    const unsigned slot = x & ((1u << PB) - 1);
+    unsigned s = min((unsigned)t[slot >> (PB - 8)], (unsigned)NSYM - 1);
+    unsigned lo = cum[s], hi = cum[s + 1], nx = cum[s + 2];
+    if (slot >= hi) { ++s; lo = hi; hi = nx; }                   // (selects: the usual bucket holds two symbols at most)
+#pragma unroll 1
+    while (slot >= hi && s < NSYM - 1) { ++s; lo = hi; hi = cum[s + 1]; }
+    x = (hi - lo) * (x >> PB) + slot - lo;
+    r.renorm(x);
+    return s;
+}
+SG_DEVINL unsigned get_global(unsigned& x, RingReader& r, const uint8_t* __restrict__ ct) {
+    const unsigned* __restrict__ words = reinterpret_cast<const unsigned*>(ct + 256);
+    const unsigned slot = x & ((1u << PB) - 1);
+    unsigned s = ct[slot >> (PB - 8)];
+    unsigned fc = words[s];
+#pragma unroll 1
+    while (slot >= (fc >> 16) + (fc & 0xffffu) && s < 255u) fc = words[++s];
+    x = (fc & 0xffffu) * (x >> PB) + slot - (fc >> 16);
+    r.renorm(x);
+    return s;
+}
+__global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __restrict__ in, const unsigned long long* __restrict__ in_off,
+                                                         const unsigned long long* __restrict__ in_end, unsigned char* __restrict__ dev,
+                                                         const TB* __restrict__ tb, const SG* __restrict__ sg, int nseg, int per, Ctx c,
+                                                         const unsigned char* __restrict__ lut, int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    DecSmem& m = *reinterpret_cast<DecSmem*>(dsm);
+    const bool chain = threadIdx.x < D_CHAIN;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = blockIdx.x * per;
+    const int grp = chain ? (lane < DSEG / 4 ? 4 * lane + warp : DSEG) : (threadIdx.x - D_CHAIN) / DG, gl = threadIdx.x % DG;
+    const int s = first + grp;
+    const bool live = grp < per && s < nseg;
     SG g; g.t = 0; g.n = 0; g.i0 = 0;
     if (live) g = sg[s];
     const TB T = tb[g.t];
-    int nmax = g.n;
-    for (int o = 16; o; o >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
-    ByteReaderUp rd; rd.over = false; rd.p = rd.end = nullptr;
-    unsigned x = RANS_L;
-    if (live && gl == 0) { rd.init(in + in_off[s], in + in_end[s]); x = rans_init(rd); }
-    unsigned short* base = reinterpret_cast<unsigned short*>(dev + T.doff);
-    // this lane's first weight of the batch: compact row rc, column j; 32 weights further every batch
-    int rc = 0, j = 0;
-    if (live) { const long long i = g.i0 + DW * gl; rc = (int)(i / T.rowlen); j = (int)(i % T.rowlen); }
-    bool bad = false;
-    for (int k0 = 0; k0 < nmax; k0 += DB) {
-        size_t at[DW];
-        {
-            int r = rc, col = j, have = -1, orow = 0;
-#pragma unroll
-            for (int v = 0; v < DW; ++v) {
-                const int k = k0 + DW * gl + v;
-                at[v] = 0;
-                if (live && k < g.n) {
-                    if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
-                    int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
-                    s_t0[grp][DW * gl + v] = T.tab + pe; s_pred[grp][DW * gl + v] = pred; s_t2[grp][DW * gl + v] = T.tab + 640 + sc;
-                    at[v] = (size_t)orow * T.rowlen + col;
-                    if (++col == T.rowlen) { col = 0; ++r; }
-                }
-            }
-        }
-        __syncwarp();
-        if (live && gl == 0 && !bad) {
-            const int n = min(DB, g.n - k0);
-#pragma unroll 2
-            for (int w = 0; w < n; ++w) {
-                const int t0 = s_t0[grp][w], pred = s_pred[grp][w], t2 = s_t2[grp][w];
-                const int ex = (int)rans_get_compact<PB>(x, rd, lut + (size_t)t0 * RANS_COMPACT);
-                const int t1 = T.tab + 512 + mctx(ex, pred);
-                const int man = (int)rans_get_compact<PB>(x, rd, lut + (size_t)t1 * RANS_COMPACT);
-                const int sgn = (int)rans_get_bit<PB>(x, rd, lut + (size_t)t2 * RANS_COMPACT);
-                s_out[grp][w] = (unsigned short)((sgn << 15) | (ex << 7) | man);
-            }
-            bad = rd.over;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int v = 0; v < DW; ++v) {
-            const int k = k0 + DW * gl + v;
-            if (live && k < g.n) base[at[v]] = s_out[grp][DW * gl + v];
-        }
-        j += DB;
-        if (live) while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
+    const int cta_tab = tb[sg[first].t].tab;
+    if (threadIdx.x == 0) {
+        const SG f = sg[first];
+        const TB F = tb[f.t];
+        const int rc = (int)(f.i0 / F.rowlen), j = (int)(f.i0 % F.rowlen);
+        int pred, pe, sc; contexts(c, F, F.rmap >= 0 ? c.rowmap[F.rmap + rc] : rc, j, pred, pe, sc);
+        m.pe0 = min(max(pe - D_ECTX / 2, 0), 512 - D_ECTX);
+        m.nmax = 0; m.bad = 0;
     }
-    if (live && gl == 0 && (bad || rd.over || x != RANS_L || rd.p != rd.end)) atomicOr(status, SG_ST_CORRUPT);
+    __syncthreads();
+    const int pe0 = m.pe0;
+    if (chain && live) atomicMax(&m.nmax, g.n);
+    for (int t = warp; t < D_MCTX + D_ECTX; t += D_THREADS / 32) {
+        if (t < D_MCTX) {
+            const uint8_t* ct = lut + (size_t)(cta_tab + 512 + t) * RANS_COMPACT;
+            int bad = 0;
+            stage_table(ct, m.mant + t * D_MP, 128, lane, bad);
+            // a used table whose distribution goes on past symbol 127 (no encoder writes one): this CTA stays with global memory
+            const unsigned w = reinterpret_cast<const unsigned*>(ct + 256)[255];
+            if (bad && (w >> 16) + (w & 0xffffu) == (1u << PB)) m.bad = 1;
+        } else {
+            int bad = 0;
+            stage_table(lut + (size_t)(cta_tab + pe0 + t - D_MCTX) * RANS_COMPACT, m.expo + (t - D_MCTX) * D_EP, 256, lane, bad);
+        }
+    }
+    if (threadIdx.x < 16) {
+        const unsigned* w = reinterpret_cast<const unsigned*>(lut + (size_t)(cta_tab + 640 + threadIdx.x) * RANS_COMPACT + 256);
+        m.sign[threadIdx.x] = (w[0] & 0xffffu) | (w[1] << 16);
+    }
+    __syncthreads();
+    const bool staged = T.tab == cta_tab && !m.bad;
+    const int nbatch = (m.nmax + DB - 1) / DB;
+    RingReader rd; rd.pos = rd.len = 0;
+    unsigned x = RANS_L;
+    bool bad = false;
+    if (chain && live) { rd.init(in + in_off[s], in + in_end[s], m.ring + grp, DSEG); x = rd.state(); }
+    unsigned short* base = reinterpret_cast<unsigned short*>(dev + T.doff);
+    // a staging lane's first weight of the batch to stage and of the batch to store: compact row, column
+    int rc = 0, j = 0, orc = 0, oj = 0;
+    if (!chain && live) { const long long i = g.i0 + DW * gl; orc = rc = (int)(i / T.rowlen); oj = j = (int)(i % T.rowlen); }
+    for (int it = 0; it < nbatch + 2; ++it) {
+        if (!chain) {
+            if (live && it >= 2) {                               // store the batch that was decoded in the last turn
+                int r = orc, col = oj, have = -1, orow = 0;
+#pragma unroll
+                for (int v = 0; v < DW; ++v) {
+                    if ((it - 2) * DB + DW * gl + v < g.n) {
+                        if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
+                        base[(size_t)orow * T.rowlen + col] = m.out[it & 1][grp][DW * gl + v];
+                        if (++col == T.rowlen) { col = 0; ++r; }
+                    }
+                }
+                oj += DB;
+                while (oj >= T.rowlen) { oj -= T.rowlen; ++orc; }
+            }
+            if (live && it < nbatch) {
+                int r = rc, col = j, have = -1, orow = 0;
+#pragma unroll
+                for (int v = 0; v < DW; ++v) {
+                    if (it * DB + DW * gl + v < g.n) {
+                        if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
+                        int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
+                        // (mctx() is constant outside of +-4000)
+                        m.ctx[it & 1][grp][DW * gl + v] = (unsigned)pe | (unsigned)sc << 9 | (unsigned)clampi(pred, -4000, 4000) << 16;
+                        if (++col == T.rowlen) { col = 0; ++r; }
+                    }
+                }
+                j += DB;
+                while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
+            }
+        } else if (live && it >= 1 && !bad) {
+            const int n = min(DB, g.n - (it - 1) * DB);
+            const unsigned* cx = m.ctx[(it - 1) & 1][grp];
+            unsigned short* o = m.out[(it - 1) & 1][grp];
+#pragma unroll 1
+            for (int w = 0; w < n; ++w) {
+                if ((w & 3) == 0) rd.top_up();                   // four weights take 24 bytes at most
+                const unsigned e = cx[w];
+                const int pe = e & 511, sc = (e >> 9) & 15, pred = (int)e >> 16;
+                unsigned ex, man;
+                if (staged && (unsigned)(pe - pe0) < (unsigned)D_ECTX) ex = get_staged<256>(x, rd, m.expo + (pe - pe0) * D_EP);
+                else ex = get_global(x, rd, lut + (size_t)(T.tab + pe) * RANS_COMPACT);
+                const int mc = mctx((int)ex, pred);
+                if (staged) man = get_staged<128>(x, rd, m.mant + mc * D_MP);
+                else man = get_global(x, rd, lut + (size_t)(T.tab + 512 + mc) * RANS_COMPACT);
+                unsigned f01 = m.sign[sc];
+                if (!staged) {
+                    const unsigned* sw = reinterpret_cast<const unsigned*>(lut + (size_t)(T.tab + 640 + sc) * RANS_COMPACT + 256);
+                    f01 = (sw[0] & 0xffffu) | (sw[1] << 16);
+                }
+                const unsigned slot = x & ((1u << PB) - 1), f0 = f01 & 0xffffu;
+                const bool neg = slot >= f0;                     // (two symbols: the second one starts where the first ends)
+                x = (neg ? f01 >> 16 : f0) * (x >> PB) + slot - (neg ? f0 : 0u);
+                rd.renorm(x);
+                o[w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
+            }
+            bad = rd.over();
+        }
+        __syncthreads();
+    }
+    if (chain && live && (bad || rd.over() || x != RANS_L || !rd.at_end())) atomicOr(status, SG_ST_CORRUPT);
 }
 
 // 64-bit row fingerprints for duplicate-row detection (bf16v2.py:148-155): an order-dependent integer recurrence, one
@@ -460,7 +570,9 @@ extern "C" int sg_r2_encode(int device, void* stream, const unsigned char* dev, 
     rc = use_device(device);
     if (rc != SG_OK) return rc;
     Ctx c = {rfi, cfi, scl, rowmap};
-    k_r2_enc<<<(nseg + ESEG - 1) / ESEG, EG * ESEG, 0, (cudaStream_t)stream>>>(dev, (const TB*)tb, (const SG*)sgp, nseg, c, (const RansSym*)enc_tab,
+    rc = cuda_ok(cudaFuncSetAttribute(k_r2_enc, cudaFuncAttributeMaxDynamicSharedMemorySize, E_SMEM));
+    if (rc != SG_OK) return rc;
+    k_r2_enc<<<(nseg + ESEG - 1) / ESEG, E_THREADS, E_SMEM, (cudaStream_t)stream>>>(dev, (const TB*)tb, (const SG*)sgp, nseg, c, (const RansSym*)enc_tab,
                                                                        slots, cap, out_len);
     return cuda_ok(cudaGetLastError());
 }
@@ -476,8 +588,11 @@ extern "C" int sg_r2_decode(int device, void* stream, const unsigned char* in, c
     rc = use_device(device);
     if (rc != SG_OK) return rc;
     Ctx c = {rfi, cfi, scl, rowmap};
-    k_r2_dec<<<(nseg + DSEG - 1) / DSEG, DG * DSEG, 0, (cudaStream_t)stream>>>(in, in_off, in_end, dev, (const TB*)tb, (const SG*)sgp, nseg, c,
-                                                                       (const RansSym*)enc_tab, lut, status_word(device));
+    rc = cuda_ok(cudaFuncSetAttribute(k_r2_dec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecSmem)));
+    if (rc != SG_OK) return rc;
+    const int want = (nseg + 147) / 148, per = want > DSEG ? DSEG : want;
+    k_r2_dec<<<(nseg + per - 1) / per, D_THREADS, sizeof(DecSmem), (cudaStream_t)stream>>>(in, in_off, in_end, dev, (const TB*)tb, (const SG*)sgp,
+                                                                                           nseg, per, c, lut, status_word(device));
     return cuda_ok(cudaGetLastError());
 }
 

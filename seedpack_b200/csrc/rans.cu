@@ -82,43 +82,61 @@ __global__ void __launch_bounds__(256) k_rans_hist(const uint8_t* __restrict__ s
 }
 
 // ---- encode ----------------------------------------------------------------------------------------------
+// Bound by the chain of a lane (one per segment) - x, comparisons, reciprocal, multiply-add - as long as nothing else is on
+// it: symbols and table ids are loaded three batches of 16 symbols ahead, the table's entry for 0 two, the other entries
+// one.  Most residual symbols are 0: only lanes with another symbol load (the lanes of a warp use different tables: a load
+// by all of them touches 32 lines).  `spw` segments per warp: few segments are spread over all SMs' schedulers.
 template <int PB>
-__global__ void __launch_bounds__(64) k_rans_encode(const uint8_t* __restrict__ sym, const uint16_t* __restrict__ block_tab,
+__global__ void __launch_bounds__(32) k_rans_encode(const uint8_t* __restrict__ sym, const uint16_t* __restrict__ block_tab,
                                                     int block_len, long long nsym, int seg_len, const RansSym* __restrict__ enc,
-                                                    uint8_t* __restrict__ out, size_t cap, unsigned* __restrict__ out_len, int nseg) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
+                                                    uint8_t* __restrict__ out, size_t cap, unsigned* __restrict__ out_len, int nseg, int spw) {
+    const long long sl = (long long)blockIdx.x * spw + threadIdx.x;
+    if ((int)threadIdx.x >= spw || sl >= nseg) return;
+    const int s = (int)sl;
     const long long s0 = (long long)s * seg_len;
-    const long long n = min((long long)seg_len, nsym - s0);            // multiple of 16
+    const int n = (int)min((long long)seg_len, nsym - s0), nb = n / 16;            // n: a multiple of 16
+    const int sub = block_len / 16;                                                // 16 | block_len: one table per batch of 16
+    const uint4* __restrict__ src = reinterpret_cast<const uint4*>(sym + s0);
+    const uint16_t* __restrict__ bt = block_tab + s0 / block_len;
     uint8_t* slot = out + (size_t)s * cap;
     ByteWriterDown w;
     w.init(slot + cap);
     unsigned x = RANS_L;
-    const RansSym* tab = nullptr;
-    RansSym e0 = {0, 0};
-    long long cur_block = -1;
-    // The lanes of a warp sit in different segments, hence different tables: a table look-up by all lanes touches 32
-    // cache lines, and with one per symbol the kernel is bound by the L1's line rate, not by its chains.  Most residual
-    // symbols are 0: the current table's entry for 0 is kept in registers, and only the lanes with another symbol load.
-    for (long long i = n - 16; i >= 0; i -= 16) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(sym + s0 + i));
-        const unsigned wv[4] = {v.x, v.y, v.z, v.w};
-        const long long blk = (s0 + i) / block_len;                     // 16 | block_len: one table per 16 symbols
-        if (blk != cur_block) { cur_block = blk; tab = enc + (size_t)block_tab[blk] * 256; e0 = tab[0]; }
+    int li = nb - 1, lblk = li / sub, lrem = li - lblk * sub;                      // next batch to load
+    uint4 v0, v1;                                                                  // symbols: just asked for / with their table known
+    unsigned t0 = 0;
+    const RansSym* tab1 = enc;
+    RansSym e01;
+    auto load = [&]() {
+        if (li >= 0) { v0 = __ldg(src + li); t0 = __ldg(bt + lblk); }
+        --li;
+        if (--lrem < 0) { lrem = sub - 1; --lblk; }
+    };
+    auto table = [&]() { v1 = v0; tab1 = enc + (size_t)t0 * 256; e01 = tab1[0]; };
+    auto look = [&](RansSym (&e)[16]) {
+        const unsigned wv[4] = {v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
-        for (int k = 3; k >= 0; --k) {
-#pragma unroll
-            for (int j = 3; j >= 0; --j) {
-                const unsigned sy = (wv[k] >> (8 * j)) & 0xff;
-                RansSym e = e0;
-                if (sy) e = tab[sy];
-                rans_put<PB>(x, w, e);
-            }
+        for (int k = 0; k < 16; ++k) {
+            const unsigned sy = (wv[k >> 2] >> (8 * (k & 3))) & 0xff;
+            e[k] = e01;
+            if (sy) e[k] = tab1[sy];
         }
-        if (w.ptr() < slot + 64) { out_len[s] = 0xffffffffu; return; }   // 16 symbols write at most 32 bytes
+    };
+    RansSym cur[16], nxt[16];
+    load(); table(); load();
+    look(cur);
+    table(); load();
+    for (int i = nb - 1; i >= 0; --i) {
+        if (i > 0) look(nxt);
+        table(); load();
+#pragma unroll
+        for (int k = 15; k >= 0; --k) rans_put<PB>(x, w, cur[k]);
+        if (w.ptr() < slot + 64) { out_len[s] = 0xffffffffu; return; }             // 16 symbols write at most 32 bytes
+#pragma unroll
+        for (int k = 0; k < 16; ++k) cur[k] = nxt[k];
     }
     rans_flush(x, w);
-    w.flush(slot);
+    w.flush();
     out_len[s] = w.bad ? LEN_NOFREQ : (unsigned)(slot + cap - w.ptr());
 }
 
@@ -201,16 +219,19 @@ __global__ void __launch_bounds__(64) k_rans_decode(const uint8_t* __restrict__ 
 // shared memory.  The other slots of a table - [freq(0), 2^PB), few when zeros dominate - get one 4-byte entry each,
 // symbol | (freq - 1) << 8 | (slot - cum) << 20, also in shared memory as far as they fit (tables in id order; the rest
 // keep the two dependent global loads lut[slot] -> enc[symbol]).  Every CTA builds the entries from enc / lut itself
-// (a few per cent of its decoding time): the caller passes no further buffer.  One CTA of 512 lanes per SM.
+// (a few per cent of its decoding time; all 512 threads): the caller passes no further buffer.  One CTA per SM, whose first
+// `per` threads then decode a segment each: the segments are spread over all SMs before a CTA takes more of them.
 constexpr unsigned NOFIT = 0xffffffffu;
 template <int PB>
 __global__ void __launch_bounds__(512, 1) k_rans_decode_sm(const uint8_t* __restrict__ in, const unsigned long long* __restrict__ off,
                                                            const uint16_t* __restrict__ block_tab, int block_len, long long nsym, int seg_len,
                                                            const RansSym* __restrict__ enc, const uint8_t* __restrict__ lut,
-                                                           uint8_t* __restrict__ sym, int nseg, int ntab, unsigned cap, int* __restrict__ status) {
+                                                           uint8_t* __restrict__ sym, int nseg, int ntab, unsigned cap, int per,
+                                                           int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned smem[];
     unsigned* base = smem;                                   // [ntab] first entry of the table, NOFIT if not staged
-    unsigned* ent = smem + ntab;                             // [cap]
+    unsigned* ring = smem + ntab;                            // [RING_WORDS][per]
+    unsigned* ent = ring + RING_WORDS * per;                 // [cap]
     unsigned short* f0 = reinterpret_cast<unsigned short*>(ent + cap);     // [ntab] freq(0)
     constexpr unsigned SLOTS = 1u << PB;
     for (int t = threadIdx.x; t < ntab; t += blockDim.x) {
@@ -240,45 +261,51 @@ __global__ void __launch_bounds__(512, 1) k_rans_decode_sm(const uint8_t* __rest
         }
     }
     __syncthreads();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
+    const long long sl = (long long)blockIdx.x * per + threadIdx.x;
+    if ((int)threadIdx.x >= per || sl >= nseg) return;
+    const int s = (int)sl;
     const long long s0 = (long long)s * seg_len;
-    const long long n = min((long long)seg_len, nsym - s0);
-    ByteReaderUp r;
-    r.init(in + off[s], in + off[s + 1]);
-    unsigned x = rans_init(r);
-    unsigned tf0 = 0, tb = NOFIT, tid = 0;
-    long long cur_block = -1;
-    for (long long i = 0; i < n; i += 16) {
-        const long long blk = (s0 + i) / block_len;
-        if (blk != cur_block) { cur_block = blk; tid = block_tab[blk]; tf0 = f0[tid]; tb = base[tid]; }
-        unsigned wv[4];
+    const int n = (int)min((long long)seg_len, nsym - s0);
+    RingReader r;
+    r.init(in + off[s], in + off[s + 1], ring + threadIdx.x, per);
+    unsigned x = r.state();
+    const uint16_t* __restrict__ bt = block_tab + s0 / block_len;
+    const int nblk = n / block_len;
+    unsigned tid_next = bt[0];
+    for (int b = 0; b < nblk; ++b) {
+        const unsigned tid = tid_next, tf0 = f0[tid], tb = base[tid];
+        if (b + 1 < nblk) tid_next = __ldg(bt + b + 1);
+        const unsigned tb0 = tb == NOFIT ? 0u : tb;
+        for (int i = 0; i < block_len; i += 16) {
+            r.top_up();
+            unsigned wv[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            unsigned word = 0;
+            for (int k = 0; k < 4; ++k) {
+                unsigned word = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const unsigned slot = x & (SLOTS - 1);
-                unsigned sy = 0;
-                if (slot < tf0) x = tf0 * (x >> PB) + slot;
-                else if (tb != NOFIT) {
-                    const unsigned e = ent[tb + slot - tf0];
-                    sy = e & 0xffu;
-                    x = (((e >> 8) & 0xfffu) + 1u) * (x >> PB) + (e >> 20);
-                } else {
-                    sy = lut[((size_t)tid << PB) + slot];
-                    const unsigned fc = enc[(size_t)tid * 256 + sy].fc;
-                    x = (fc & 0xffffu) * (x >> PB) + slot - (fc >> 16);
+                for (int j = 0; j < 4; ++j) {
+                    // both kinds of slot without a branch: with 32 segments in a warp some lane meets a symbol other than 0
+                    // at most steps.  ent[] is read within bounds whatever the slot (an unstaged table reads its start)
+                    const unsigned slot = x & (SLOTS - 1);
+                    const bool nz = slot >= tf0;
+                    const unsigned e = ent[tb0 + (nz && tb != NOFIT ? slot - tf0 : 0u)];
+                    unsigned sy = nz ? e & 0xffu : 0u, f = nz ? ((e >> 8) & 0xfffu) + 1u : tf0, d = nz ? e >> 20 : slot;
+                    if (nz && tb == NOFIT) {
+                        sy = lut[((size_t)tid << PB) + slot];
+                        const unsigned fc = enc[(size_t)tid * 256 + sy].fc;
+                        f = fc & 0xffffu; d = slot - (fc >> 16);
+                    }
+                    x = f * (x >> PB) + d;
+                    r.renorm(x);
+                    word |= sy << (8 * j);
                 }
-                if (x < RANS_L) { x = (x << 8) | r.get(); if (x < RANS_L) x = (x << 8) | r.get(); }
-                word |= sy << (8 * j);
+                wv[k] = word;
             }
-            wv[k] = word;
+            *reinterpret_cast<uint4*>(sym + s0 + (long long)b * block_len + i) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+            if (r.over()) { atomicOr(status, SG_ST_CORRUPT); return; }
         }
-        *reinterpret_cast<uint4*>(sym + s0 + i) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-        if (r.over) { atomicOr(status, SG_ST_CORRUPT); return; }
     }
-    if (x != RANS_L || r.p != r.end) atomicOr(status, SG_ST_CORRUPT);     // a well-formed segment ends in the initial state
+    if (x != RANS_L || !r.at_end()) atomicOr(status, SG_ST_CORRUPT);      // a well-formed segment ends in the initial state
 }
 
 }  // namespace sg
@@ -328,8 +355,9 @@ extern "C" int sg_rans_encode(int device, void* stream, const unsigned char* sym
     if (rc != SG_OK) return rc;
     const long long nseg = (nsym + seg_len - 1) / seg_len;
     if (nseg > 0x7fffffffLL) return SG_ERR_LIMIT;
-    k_rans_encode<12><<<(unsigned)((nseg + 63) / 64), 64, 0, (cudaStream_t)stream>>>(sym, block_tab, block_len, nsym, seg_len,
-                                                                                     (const RansSym*)enc_tab, slots, cap, out_len, (int)nseg);
+    const int spw = segs_per_warp(nseg);
+    k_rans_encode<12><<<(unsigned)((nseg + spw - 1) / spw), 32, 0, (cudaStream_t)stream>>>(
+        sym, block_tab, block_len, nsym, seg_len, (const RansSym*)enc_tab, slots, cap, out_len, (int)nseg, spw);
     return cuda_ok(cudaGetLastError());
 }
 
@@ -360,19 +388,23 @@ extern "C" int sg_rans_decode(int device, void* stream, const unsigned char* in,
     if (nseg > 0x7fffffffLL) return SG_ERR_LIMIT;
     cudaStream_t st = (cudaStream_t)stream;
     // tables staged in shared memory when their number is given and small enough to leave room for entries
-    const size_t smem_max = 200 * 1024;
-    if (ntab > 0 && (size_t)ntab * 6 + 8192 <= smem_max) {
-        const unsigned cap = (unsigned)((smem_max - (size_t)ntab * 6 - 16) / 4);
-        const size_t smem = (size_t)ntab * 4 + (size_t)cap * 4 + (size_t)ntab * 2 + 16;
+    const size_t smem_max = 220 * 1024;
+    if (ntab > 0 && (size_t)ntab * 6 + 8192 + 256 * RING_WORDS * 4 <= smem_max) {
+        // segments per CTA: as few as fill the SMs (a warp's worth at least), 256 at most (their rings take 128 bytes each)
+        long long per = (nseg + 147) / 148;
+        per = per <= 32 ? 32 : per >= 256 ? 256 : (per + 31) / 32 * 32;
+        const size_t ring = (size_t)per * RING_WORDS * 4;
+        const unsigned cap = (unsigned)((smem_max - (size_t)ntab * 6 - 16 - ring) / 4);
+        const size_t smem = (size_t)ntab * 4 + ring + (size_t)cap * 4 + (size_t)ntab * 2 + 16;
         static bool configured[64] = {false};
         if (device < 64 && !configured[device]) {
             rc = cuda_ok(cudaFuncSetAttribute(k_rans_decode_sm<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max + 1024));
             if (rc != SG_OK) return rc;
             configured[device] = true;
         }
-        k_rans_decode_sm<12><<<(unsigned)((nseg + 511) / 512), 512, smem, st>>>(in, off, block_tab, block_len, nsym, seg_len,
-                                                                            (const RansSym*)enc_tab, lut, sym_out, (int)nseg, ntab, cap,
-                                                                            status_word(device));
+        k_rans_decode_sm<12><<<(unsigned)((nseg + per - 1) / per), 512, smem, st>>>(in, off, block_tab, block_len, nsym, seg_len,
+                                                                                (const RansSym*)enc_tab, lut, sym_out, (int)nseg, ntab, cap,
+                                                                                (int)per, status_word(device));
         return cuda_ok(cudaGetLastError());
     }
     k_rans_decode<12><<<(unsigned)((nseg + 63) / 64), 64, 0, st>>>(in, off, block_tab, block_len, nsym, seg_len,

@@ -9,8 +9,9 @@
 // What differs from the reference is only how a lane gets there:
 //   * x / f and x % f use a per-(table, symbol) 32-bit reciprocal (exact for x < 2^31, which the
 //     renormalisation guarantees) instead of integer division;
-//   * bytes move through a 16-byte register window per lane, so that global memory only sees aligned
-//     16-byte loads and stores.
+//   * a coder step has no branch: the number of bytes it moves (0, 1 or 2) is two comparisons, the bytes enter or
+//     leave a shift register.  The lanes of a warp sit in different segments and renormalise at different symbols, so
+//     that a branch per byte ran on nearly every symbol of the warp: 280 - 360 cycles a symbol before, see the kernels.
 #pragma once
 #include "common.cuh"
 
@@ -25,41 +26,28 @@ struct __align__(8) RansSym { unsigned rcp, fc; };
 
 SG_DEVINL unsigned rans_shift(unsigned freq) { return freq < 2 ? 0u : 32u - __clz(freq - 1); }
 
-// quotient x / freq for x < 2^31, 1 <= freq <= 2^15
-SG_DEVINL unsigned rans_div(unsigned x, unsigned freq, unsigned rcp) {
-    if (freq < 2) return x;
-    const unsigned s = rans_shift(freq);            // >= 1
-    return __umulhi(x, rcp) >> (s - 1);
-}
-
 // ---- downward byte writer ----------------------------------------------------------------------------
-// Writes bytes at decreasing addresses ending at `end` (16-byte aligned).  Holds the 16-byte window that
-// contains the next byte; full windows are stored with one 16-byte store.
+// Writes bytes at decreasing addresses ending at `end` (4-byte aligned).  Pending bytes sit in `acc`, the last one lowest;
+// whenever four are there the oldest four leave as one aligned word.
 struct ByteWriterDown {
-    uint8_t* base;                 // address of the current window
-    unsigned long long lo, hi;     // window contents (byte k of the window at bits 8k of lo / hi)
-    int pos;                       // bytes still free in the window: next byte goes to index pos - 1
+    uint8_t* p;                    // lowest address stored so far
+    unsigned long long acc;        // pending bytes (what is above them has left already)
+    int cnt;                       // how many: 0 .. 3 between calls
     unsigned bad;                  // set when a symbol with frequency 0 was coded (tables not made from these symbols)
-    SG_DEVINL void init(uint8_t* end) { base = end - 16; lo = hi = 0; pos = 16; bad = 0; }
-    SG_DEVINL void put(unsigned b) {
-        --pos;
-        if (pos >= 8) hi |= (unsigned long long)b << (8 * (pos - 8));
-        else          lo |= (unsigned long long)b << (8 * pos);
-        if (pos == 0) {
-            *reinterpret_cast<ulonglong2*>(base) = make_ulonglong2(lo, hi);
-            base -= 16; lo = hi = 0; pos = 16;
-        }
+    SG_DEVINL void init(uint8_t* end) { p = end; acc = 0; cnt = 0; bad = 0; }
+    SG_DEVINL bool push(unsigned x, int n) {                   // the n <= 2 low bytes of x, the lowest first
+        const unsigned v = n == 2 ? __byte_perm(x, 0, 0x4401) : n ? x & 0xffu : 0u;
+        acc = (acc << (8 * n)) | v;
+        cnt += n;
+        return cnt >= 4;
+    }
+    SG_DEVINL void emit(unsigned x, int n) {
+        if (push(x, n)) { cnt -= 4; p -= 4; *reinterpret_cast<unsigned*>(p) = (unsigned)(acc >> (8 * cnt)); }
     }
     // bytes written so far end at this address (the lowest written byte)
-    SG_DEVINL uint8_t* ptr() const { return base + pos; }
-    // store the partial window; the bytes below ptr() inside it are zero filler in the lane's private slot
-    SG_DEVINL void flush(uint8_t* slot_begin) {
-        if (pos < 16 && base >= slot_begin) *reinterpret_cast<ulonglong2*>(base) = make_ulonglong2(lo, hi);
-        else if (pos < 16) {       // window straddles the slot start: byte stores for the part inside the slot
-            for (int k = pos; k < 16; ++k)
-                base[k] = (uint8_t)((k >= 8 ? hi >> (8 * (k - 8)) : lo >> (8 * k)) & 0xff);
-        }
-    }
+    SG_DEVINL uint8_t* ptr() const { return p - cnt; }
+    // store the pending bytes
+    SG_DEVINL void flush() { for (; cnt > 0; --cnt) *--p = (uint8_t)(acc >> (8 * (cnt - 1))); }
 };
 
 // ---- forward byte reader -----------------------------------------------------------------------------
@@ -98,21 +86,96 @@ struct ByteReaderUp {
     }
 };
 
+// ---- forward reader through a ring in shared memory --------------------------------------------------------
+// For kernels whose lanes decode side by side.  A register that is refilled by a load when a lane has used it up makes
+// the whole warp wait for that load, and with 8 - 32 segments per warp some lane refills at almost every symbol.  Here all
+// lanes top their rings up together, every few symbols, with the 32 bytes that were asked for at the last top-up; a
+// symbol takes its next four bytes from two shared-memory words, off the state's own chain.
+// A lane's ring: 32 words at a stride of `pitch` words.  Between two top-ups a lane may take 32 bytes (16 symbols).
+constexpr int RING_WORDS = 32;
+struct RingReader {
+    const uint8_t* src;            // next 32 bytes to ask for (16-byte aligned)
+    const uint8_t* end;
+    uint4 c0, c1;                  // the 32 bytes asked for last
+    unsigned* ring; int pitch;
+    int pos, have, len;            // bytes from the aligned start: taken, put into the ring, in the stream
+    unsigned top;                  // the next four bytes, the first one highest
+    SG_DEVINL void fetch() {
+        c0 = c1 = make_uint4(0, 0, 0, 0);
+        if (src < end) c0 = *reinterpret_cast<const uint4*>(src);
+        if (src + 16 < end) c1 = *reinterpret_cast<const uint4*>(src + 16);
+        src += 32;
+    }
+    SG_DEVINL void put(const uint4 v, int w) {
+        const unsigned a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ring[((w + i) & (RING_WORDS - 1)) * pitch] = __byte_perm(a[i], 0, 0x0123);
+    }
+    SG_DEVINL void top_up() {
+        if (have - pos <= 4 * RING_WORDS - 32) {
+            put(c0, have >> 2); put(c1, (have >> 2) + 4);
+            have += 32;
+            fetch();
+        }
+    }
+    SG_DEVINL void look() {
+        const unsigned hi = ring[((pos >> 2) & (RING_WORDS - 1)) * pitch], lo = ring[((pos >> 2) + 1 & (RING_WORDS - 1)) * pitch];
+        top = __funnelshift_l(lo, hi, 8 * (pos & 3));
+    }
+    SG_DEVINL void init(const uint8_t* begin, const uint8_t* e, unsigned* r, int stride) {
+        ring = r; pitch = stride;
+        src = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(begin) & ~(uintptr_t)15);
+        pos = (int)(begin - src); have = 0;
+        end = e > begin ? e : begin;
+        len = (int)min((long long)(end - src), 0x7fffff00LL);
+        if (end == begin) end = src;                           // nothing to read
+        fetch();
+        top_up(); top_up(); top_up();
+        look();
+    }
+    SG_DEVINL bool over() const { return pos > len; }
+    SG_DEVINL bool at_end() const { return pos == len; }
+    // x after a step: take bytes until x >= 2^23 (a stream that was coded needs at most two)
+    SG_DEVINL void renorm(unsigned& x) {
+        int n = x < (1u << 15) ? 2 : x < RANS_L ? 1 : 0;
+        x = __funnelshift_l(top, x, 8 * n);
+        pos += n;
+        look();
+        if (x < RANS_L && n) {                                 // damaged streams only
+#pragma unroll 1
+            for (int guard = 0; guard < 2 && x < RANS_L; ++guard) { x = __funnelshift_l(top, x, 8); ++pos; look(); }
+        }
+    }
+    SG_DEVINL unsigned state() { const unsigned x = top; pos += 4; look(); return x; }
+};
+
 // ---- coder steps -------------------------------------------------------------------------------------
+// The chain from state to state: two comparisons, a shift, the reciprocal's high product, a shift, one multiply-add.  What
+// depends on the entry alone (xm, the shift, the bias) is off it.  f = 1: the reciprocal 2^32 - 1 gives x - 1, made up
+// for in the bias.
+// Segments per warp of a kernel with one lane per segment: its time is that of one lane's chain, so a warp takes more than 8
+// only once every scheduler of the 148 SMs has one.
+inline int segs_per_warp(long long nseg) {
+    const long long n = (nseg + 148 * 4 - 1) / (148 * 4);
+    return n <= 8 ? 8 : n >= 32 ? 32 : (int)n;
+}
+constexpr unsigned RANS_NOP_RCP = 1u << 31;        // with freq = 2^12, cum = 0 (12 bits): an entry that leaves the state as it is
 template <int PB, class W>
 SG_DEVINL void rans_put(unsigned& x, W& w, const RansSym e) {
     const unsigned f = e.fc & 0xffffu, c = e.fc >> 16;
-    const unsigned xm = ((RANS_L >> PB) << 8) * f;
-    // x < 2^31 and xm >= 2^(31 - PB) for f >= 1: at most two bytes leave per symbol (PB <= 15).  Written as two steps,
-    // not a loop: a zero frequency (xm = 0) would never end it; such a symbol marks the segment instead.
+    const unsigned xm = f << (31 - PB);
+    // x < 2^31 and xm >= 2^(31 - PB) for f >= 1: at most two bytes leave per symbol (PB <= 15); a zero frequency marks the segment
     w.bad |= (unsigned)(f == 0);
-    if (x >= xm) { w.put(x & 0xff); x >>= 8; if (x >= xm) { w.put(x & 0xff); x >>= 8; } }
-    const unsigned q = rans_div(x, f, e.rcp);
-    x = (q << PB) + (x - q * f) + c;
+    const int n = x >= xm ? ((x >> 8) >= xm ? 2 : 1) : 0;
+    w.emit(x, n);
+    x >>= 8 * n;
+    const unsigned sh = f < 2 ? 0u : 31u - __clz(f - 1), bias = f < 2 ? c + (1u << PB) - 1u : c;
+    const unsigned q = __umulhi(x, e.rcp) >> sh;
+    x = q * ((1u << PB) - f) + (x + bias);
 }
 template <class W> SG_DEVINL void rans_flush(unsigned x, W& w) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { w.put(x & 0xff); x >>= 8; }
+    for (int i = 0; i < 4; ++i) { w.emit(x, 1); x >>= 8; }
 }
 template <class R> SG_DEVINL unsigned rans_init(R& r) {
     unsigned x = 0;
@@ -144,18 +207,6 @@ SG_DEVINL unsigned rans_get_compact(unsigned& x, R& r, const uint8_t* __restrict
     unsigned fc = words[s];
 #pragma unroll 1
     while (slot >= (fc >> 16) + (fc & 0xffffu) && s < 255u) fc = words[++s];
-    x = (fc & 0xffffu) * (x >> PB) + slot - (fc >> 16);
-#pragma unroll 1
-    for (int guard = 0; guard < 4 && x < RANS_L; ++guard) x = (x << 8) | r.get();
-    return s;
-}
-// a table of two symbols (a sign): both words in one 8-byte load, no coarse entry
-template <int PB, class R>
-SG_DEVINL unsigned rans_get_bit(unsigned& x, R& r, const uint8_t* __restrict__ ct) {
-    const unsigned slot = x & ((1u << PB) - 1);
-    const uint2 e = *reinterpret_cast<const uint2*>(ct + 256);
-    const unsigned s = slot >= (e.x & 0xffffu) ? 1u : 0u;
-    const unsigned fc = s ? e.y : e.x;
     x = (fc & 0xffffu) * (x >> PB) + slot - (fc >> 16);
 #pragma unroll 1
     for (int guard = 0; guard < 4 && x < RANS_L; ++guard) x = (x << 8) | r.get();

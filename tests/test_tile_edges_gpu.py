@@ -42,3 +42,74 @@ def test_dequantize_values():
     y = np.concatenate([d.view(np.uint8).reshape(-1, 2), q4[:, :16] | (q4[:, 16:] << 4)], 1)
     want = (q4.astype(np.float32) - 8) * d.astype(np.float32)[:, None]
     assert np.array_equal(gq.dequantize(2, torch.from_numpy(y).cuda()).cpu().numpy().reshape(-1, 32), want)
+
+
+R2_SHAPES = [(1, 1, 0), (5, 37, 0), (3, 16384, 0), (64, 1000, 1), (700, 4099, 1)]
+
+
+@pytest.mark.parametrize("rows,cols,spread", R2_SHAPES)
+def test_base_codec_round_trip(rows, cols, spread):
+    """two tensors of different roles in one launch: segments of one weight and of ragged batches, and (spread) rows over more
+    octaves than the decoder stages tables for, zeros and infinities among them: the weights come back bit for bit"""
+    import ctypes
+
+    import torch
+    from seedpack_b200 import _lib
+    from seedpack_b200.rans import normalize
+    L, dev = _lib.lib(), torch.device("cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    call = lambda name, *a: _lib.check(getattr(L, name)(torch.cuda.current_device(), st, *a), name)
+    g = torch.Generator(device="cuda").manual_seed(rows * cols)
+    w = torch.randn(2, rows, cols, generator=g, device=dev)
+    if spread:
+        w *= torch.exp2(torch.randint(-40, 40, (2, rows, 1), generator=g, device=dev).float())
+        w[:, ::7, ::11] = 0
+        w[1, 0, 0] = float("inf")
+    w = w.to(torch.bfloat16).view(torch.int16).reshape(-1)
+    n, ntab = rows * cols, 2 * 656
+    tb = np.zeros(2, np.dtype([("doff", "<i8"), ("rowlen", "<i4"), ("rowbase", "<i4"), ("colbase", "<i4"), ("tab", "<i4"), ("rmap", "<i4"), ("pad", "<i4")]))
+    segs = []
+    for i in range(2):
+        tb[i] = (2 * i * n, cols, i * rows, i * cols, i * 656, -1, 0)
+        segs += [(i, min(16384, n - a), a) for a in range(0, n, 16384)]
+    sg = np.array(segs, np.dtype([("t", "<i4"), ("n", "<i4"), ("i0", "<i8")]))
+    tb, sg, nseg = torch.from_numpy(tb.view(np.uint8)).cuda(), torch.from_numpy(sg.view(np.uint8)).cuda(), len(sg)
+    rfi, cfi = torch.empty(2 * rows, dtype=torch.int16, device=dev), torch.empty(2 * cols, dtype=torch.int16, device=dev)
+    scl = torch.empty(2 * cols, dtype=torch.int8, device=dev)
+    scratch = torch.empty(L.sg_r2_stats_scratch_bytes(rows, cols), dtype=torch.uint8, device=dev)
+    for i in range(2):
+        call("sg_r2_stats", p(w[i * n:]), rows, cols, p(rfi[i * rows:]), p(cfi[i * cols:]), p(scl[i * cols:]), p(scratch), scratch.numel())
+    none = torch.zeros(1, dtype=torch.int32, device=dev)
+    side = (p(rfi), p(cfi), p(scl), p(none))
+    counts = torch.zeros(ntab * 256, dtype=torch.int32, device=dev)
+    call("sg_r2_hist", p(w), p(tb), p(sg), nseg, *side, p(counts))
+    h = counts.cpu().numpy().reshape(ntab, 256)
+    assert h.sum() == 6 * n
+    # the histogram against NumPy, over the side information the device made
+    u = w.cpu().numpy().view(np.uint16).reshape(2, rows, cols).astype(np.int64)
+    pred = rfi.cpu().numpy().reshape(2, rows, 1).astype(np.int64) + cfi.cpu().numpy().reshape(2, 1, cols)
+    ex, base = (u >> 7) & 255, np.arange(2).reshape(2, 1, 1) * 656
+    want = np.zeros(ntab * 256, np.int64)
+    for tab, sym in ((np.clip(pred + 256, 0, 511), ex), (512 + np.clip(8 * ex - pred - 952, 0, 127), u & 127),
+                     (640 + np.clip(scl.cpu().numpy().reshape(2, 1, cols).astype(np.int64), 0, 15) + 0 * ex, u >> 15)):
+        want += np.bincount(((base + tab) * 256 + sym).reshape(-1), minlength=ntab * 256)
+    assert np.array_equal(h.reshape(-1), want)
+    freq, used = normalize(h, 1 << 15)
+    full = np.zeros((ntab, 256), np.uint16)
+    full[used] = freq
+    f = torch.from_numpy(full.view(np.int16)).cuda()
+    enc, lut = torch.empty(ntab * 512, dtype=torch.int32, device=dev), torch.empty(ntab * 1280, dtype=torch.uint8, device=dev)
+    call("sg_rans_tables", p(f), ntab, 15, p(enc), p(lut))
+    cap = 16384 * 4 + 1024
+    slots, lens = torch.empty(nseg * cap, dtype=torch.uint8, device=dev), torch.empty(nseg, dtype=torch.int32, device=dev)
+    call("sg_r2_encode", p(w), p(tb), p(sg), nseg, *side, p(enc), p(slots), cap, p(lens))
+    total = int(lens.cpu().numpy().view(np.uint32).astype(np.int64).sum())
+    assert 0 < total < nseg * cap
+    stream, off = torch.zeros((total + 31) // 16 * 16, dtype=torch.uint8, device=dev), torch.empty(nseg + 1, dtype=torch.int64, device=dev)
+    call("sg_scan_gather", p(slots), cap, p(lens), nseg, p(stream), total, p(off))
+    back = torch.full_like(w, -1)
+    call("sg_r2_decode", p(stream), p(off), p(off[1:]), p(back), p(tb), p(sg), nseg, *side, p(enc), p(lut))
+    bits = ctypes.c_int(0)
+    _lib.check(L.sg_status_fetch(torch.cuda.current_device(), st, ctypes.byref(bits)), "sg_status_fetch")
+    assert bits.value == 0 and torch.equal(back, w)
