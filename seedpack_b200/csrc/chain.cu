@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(32) k_chain_enc(const uint8_t* __restrict__ sy
     }
     rans_flush(x, wr);
     wr.flush();
-    out_len[c] = wr.bad ? (unsigned long long)LEN_NOFREQ : (unsigned long long)(end - wr.ptr());
+    out_len[c] = wr.bad() ? (unsigned long long)LEN_NOFREQ : (unsigned long long)(end - wr.ptr());
 }
 
 template <class C>

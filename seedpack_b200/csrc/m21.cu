@@ -27,18 +27,17 @@ struct Meta { int first, nblocks, nb_row, grp, colbase, rowbase, off, qset; };
 struct SlotWriter : ByteWriterDown {
     uint8_t* lim; bool over;
     SG_DEVINL void init(uint8_t* end, uint8_t* slot_begin) { ByteWriterDown::init(end); lim = slot_begin; over = false; }
-    SG_DEVINL void emit(unsigned x, int n) {
-        if (push(x, n)) {
-            cnt -= 4;
-            if (over || p - 4 < lim) over = true;
-            else { p -= 4; *reinterpret_cast<unsigned*>(p) = (unsigned)(acc >> (8 * cnt)); }
-        }
+    SG_DEVINL void drain() {
+        if (bits < 32) return;
+        if (over || p - 4 < lim) over = true;
+        else { p -= 4; *reinterpret_cast<unsigned*>(p) = oldest(); }
+        bits -= 32;
     }
     // the pending bytes; -> the segment's length, or the overflow mark
     SG_DEVINL unsigned finish(uint8_t* end) {
         if (over || ptr() < lim) return LEN_OVERFLOW;
         flush();
-        return bad ? LEN_NOFREQ : (unsigned)(end - p);
+        return bad() ? LEN_NOFREQ : (unsigned)(end - p);
     }
 };
 

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(128) k_enc(const unsigned char* __restrict__ b
     }
     rans_flush(x, wr);
     wr.flush();
-    out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
+    out_len[s] = wr.bad() ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
 }
 
 __global__ void __launch_bounds__(128) k_dec(const unsigned char* __restrict__ in, const unsigned long long* __restrict__ in_off,

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(QR_TPB) k_qr_enc(const Args a, const RansSym* 
     if (c.ovf) { out_len[s] = 0xffffffffu; return; }
     rans_flush(c.x, c.wr);
     c.wr.flush();
-    out_len[s] = c.wr.bad ? LEN_NOFREQ : (unsigned)(c.slot + cap - c.wr.ptr());
+    out_len[s] = c.wr.bad() ? LEN_NOFREQ : (unsigned)(c.slot + cap - c.wr.ptr());
 }
 
 // ---- decoder of the scalar-code types: a warp per segment ------------------------------------------------------------
@@ -734,14 +734,14 @@ __global__ void __launch_bounds__(32) k_qr_stage_code(const SG* __restrict__ sg,
         m = m0;
         load();
 #pragma unroll
-        for (int k = 0; k < 8; ++k) rans_put<12>(x, wr, cur[k]);
+        for (int k = 0; k < 8; k += 2) rans_put2<12>(x, wr, cur[k], cur[k + 1]);
         if (wr.ptr() < slot + 64) { out_len[s] = LEN_OVERFLOW; return; }       // 8 symbols write at most 16 bytes
 #pragma unroll
         for (int k = 0; k < 8; ++k) cur[k] = nxt[k];
     }
     rans_flush(x, wr);
     wr.flush();
-    out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
+    out_len[s] = wr.bad() ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
 }
 
 }  // namespace qr

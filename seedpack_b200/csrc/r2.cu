@@ -135,13 +135,14 @@ __global__ void __launch_bounds__(R2H_WARPS * 32) k_r2_hist(const unsigned char*
 // Bound by the chain of 96 steps per batch.
 constexpr int EB = 32, ESEG = 32, EG = 4, EW = EB / EG;          // weights per batch, segments per CTA, staging lanes per segment
 constexpr int E_THREADS = 32 + EG * ESEG, E_PITCH = EB * 3 + 1;  // padded: the chain lanes read the same weight of their rows together
-constexpr int E_SMEM = 2 * ESEG * E_PITCH * (int)sizeof(RansSym);
+constexpr int E_SMEM = 2 * ESEG * E_PITCH * (int)sizeof(RansStep);
 __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __restrict__ dev, const TB* __restrict__ tb, const SG* __restrict__ sg,
                                                       int nseg, Ctx c, const RansSym* __restrict__ enc, unsigned char* __restrict__ out, size_t cap,
                                                       unsigned* __restrict__ out_len) {
     // per weight of a batch: sign, mantissa, exponent entries (coding order); two batches
-    extern __shared__ __align__(16) RansSym s_e[];
+    extern __shared__ __align__(16) RansStep s_e[];
     __shared__ int s_nmax;
+    __shared__ unsigned s_bad[ESEG];
     const bool chain = threadIdx.x < 32;
     const int grp = chain ? threadIdx.x : (threadIdx.x - 32) / EG, gl = (threadIdx.x - 32) % EG;
     const int s = blockIdx.x * ESEG + grp;
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
     if (live) g = sg[s];
     const TB T = tb[g.t];
     if (threadIdx.x == 0) s_nmax = 0;
+    if (chain) s_bad[grp] = 0;
     __syncthreads();
     if (chain) atomicMax(&s_nmax, g.n);
     __syncthreads();
@@ -168,35 +170,73 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
     for (int it = 0; it <= nb_max; ++it) {
         if (!chain) {
             const int k0 = (nb_max - 1 - it) * EB;
-            RansSym* row = s_e + ((it & 1) * ESEG + grp) * E_PITCH + 3 * EW * gl;
+            RansStep* row = s_e + ((it & 1) * ESEG + grp) * E_PITCH + 3 * EW * gl;
             if (live && k0 >= 0 && k0 < g.n) {
-                int r = rc, col = j, have = -1, orow = 0;
+                // loads in three waves, each for all of the lane's weights (past the segment's end: its last weight again)
+                int r[EW], col[EW], orow[EW];
+                unsigned u[EW];
+                int pred[EW], pe[EW], sc[EW];
+                RansSym e[3 * EW];
 #pragma unroll
                 for (int v = 0; v < EW; ++v) {
-                    const int k = k0 + EW * gl + v;
-                    if (k < g.n) {
-                        if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
-                        const unsigned u = base[(size_t)orow * T.rowlen + col];
-                        const int ex = (u >> 7) & 255, man = u & 127, sgn = u >> 15;
-                        int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
-                        row[3 * v] = enc[(size_t)(T.tab + 640 + sc) * 256 + sgn];
-                        row[3 * v + 1] = enc[(size_t)(T.tab + 512 + mctx(ex, pred)) * 256 + man];
-                        row[3 * v + 2] = enc[(size_t)(T.tab + pe) * 256 + ex];
-                        if (++col == T.rowlen) { col = 0; ++r; }
+                    r[v] = v ? r[v - 1] : rc; col[v] = v ? col[v - 1] : j;
+                    if (v && k0 + EW * gl + v < g.n && ++col[v] == T.rowlen) { col[v] = 0; ++r[v]; }
+                }
+                if (k0 + EW * gl < g.n) {
+#pragma unroll
+                    for (int v = 0; v < EW; ++v) orow[v] = T.rmap >= 0 ? c.rowmap[T.rmap + r[v]] : r[v];
+#pragma unroll
+                    for (int v = 0; v < EW; ++v) {
+                        u[v] = base[(size_t)orow[v] * T.rowlen + col[v]];
+                        contexts(c, T, orow[v], col[v], pred[v], pe[v], sc[v]);
                     }
+                    const RansSym* et = enc + (size_t)T.tab * 256;
+#pragma unroll
+                    for (int v = 0; v < EW; ++v) {
+                        const int ex = (u[v] >> 7) & 255;
+                        e[3 * v] = et[(640 + sc[v]) * 256 + (u[v] >> 15)];
+                        e[3 * v + 1] = et[(512 + mctx(ex, pred[v])) * 256 + (u[v] & 127)];
+                        e[3 * v + 2] = et[pe[v] * 256 + ex];
+                    }
+                    bool none = false;
+#pragma unroll
+                    for (int i = 0; i < 3 * EW; ++i) {
+                        none |= (e[i].fc & 0xffffu) == 0;
+                        row[i] = rans_step_of<PB>(e[i]);
+                    }
+                    if (none) s_bad[grp] = 1;
                 }
             }
             j -= EB;
             if (live) while (j < 0) { j += T.rowlen; --rc; }
         } else if (it > 0 && live && !full) {
             const int n = min(EB, g.n - (nb_max - it) * EB);
-            const RansSym* row = s_e + (((it - 1) & 1) * ESEG + grp) * E_PITCH;
-#pragma unroll 4
-            for (int w = n - 1; w >= 0; --w) {
-                rans_put<PB>(x, wr, row[3 * w]);
-                rans_put<PB>(x, wr, row[3 * w + 1]);
-                rans_put<PB>(x, wr, row[3 * w + 2]);
+            const RansStep* row = s_e + (((it - 1) & 1) * ESEG + grp) * E_PITCH;
+            int w = n - 1;
+            // two weights, six steps, at a time; a look at the slot's room every 16 weights, of 6 bytes at most each
+            for (; (w & 15) != 15; --w) {
+                if (w < 0) break;
+                rans_put(x, wr, row[3 * w]); rans_put(x, wr, row[3 * w + 1]); wr.drain();
+                rans_put(x, wr, row[3 * w + 2]); wr.drain();
                 if (wr.ptr() < slot + 64) { full = true; break; }
+            }
+            for (; w >= 15 && !full; w -= 16) {
+                if (wr.ptr() < slot + 64 + 96) {                 // near the slot's start: weight by weight
+                    for (int v = 0; v < 16 && !full; ++v) {
+                        const RansStep* q = row + 3 * (w - v);
+                        rans_put(x, wr, q[0]); rans_put(x, wr, q[1]); wr.drain();
+                        rans_put(x, wr, q[2]); wr.drain();
+                        full = wr.ptr() < slot + 64;
+                    }
+                    continue;
+                }
+#pragma unroll
+                for (int v = 0; v < 16; v += 2) {
+                    const RansStep* q = row + 3 * (w - v);
+                    rans_put(x, wr, q[0]); rans_put(x, wr, q[1]); wr.drain();
+                    rans_put(x, wr, q[2]); rans_put(x, wr, q[-3]); wr.drain();
+                    rans_put(x, wr, q[-2]); rans_put(x, wr, q[-1]); wr.drain();
+                }
             }
         }
         __syncthreads();
@@ -206,7 +246,7 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
         else {
             rans_flush(x, wr);
             wr.flush();
-            out_len[s] = wr.bad ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
+            out_len[s] = s_bad[grp] ? LEN_NOFREQ : (unsigned)(slot + cap - wr.ptr());
         }
     }
 }
@@ -223,7 +263,7 @@ constexpr int DB = 32, DSEG = 64, DG = 4, DW = DB / DG;          // weights per 
 constexpr int D_CHAIN = 128, D_THREADS = D_CHAIN + DG * DSEG;
 constexpr int D_ECTX = 128, D_MCTX = 128, D_MP = 256 + 260, D_EP = 256 + 516;       // bytes per table: 256 coarse, 130 / 258 cumulated
 struct DecSmem {
-    unsigned ring[RING_WORDS * DSEG];
+    unsigned ring[RING_ROWS * DSEG];
     unsigned ctx[2][DSEG][DB + 1];                               // pe | sc << 9 | pred << 16; rows padded
     unsigned sign[16];                                           // frequency of symbol 0 | of symbol 1 << 16
     unsigned short out[2][DSEG][DB + 2];
@@ -240,23 +280,27 @@ SG_DEVINL void stage_table(const uint8_t* __restrict__ ct, uint8_t* dst, int nsy
         const unsigned w = words[nsym - 1];
         const unsigned tot = (w >> 16) + (w & 0xffffu);
         cum[nsym] = (unsigned short)tot;
-        cum[nsym + 1] = 0xffff;
+        cum[nsym + 1] = (unsigned short)tot;
         if (tot != (1u << PB)) bad = 1;
     }
 }
-template <int NSYM> SG_DEVINL unsigned get_staged(unsigned& x, RingReader& r, const uint8_t* t) {
+typedef RingReader<DSEG> DecRing;
+// The staged search stops at the second symbol of a bucket: a third one (rare symbols share a bucket) sets `miss`, and the
+// weight is decoded again from the tables in global memory.  So the steps have no branch.
+template <int NSYM> SG_DEVINL unsigned get_staged(unsigned& x, DecRing& r, const uint8_t* t, bool& miss) {
     const unsigned short* cum = reinterpret_cast<const unsigned short*>(t + 256);
-    const unsigned slot = x & ((1u << PB) - 1);
-    unsigned s = min((unsigned)t[slot >> (PB - 8)], (unsigned)NSYM - 1);
-    unsigned lo = cum[s], hi = cum[s + 1], nx = cum[s + 2];
-    if (slot >= hi) { ++s; lo = hi; hi = nx; }                   // (selects: the usual bucket holds two symbols at most)
-#pragma unroll 1
-    while (slot >= hi && s < NSYM - 1) { ++s; lo = hi; hi = cum[s + 1]; }
-    x = (hi - lo) * (x >> PB) + slot - lo;
+    const unsigned slot = x & ((1u << PB) - 1), xs = x >> PB;
+    unsigned s = t[slot >> (PB - 8)];
+    if (NSYM < 256) s &= NSYM - 1;                               // (an unused table's place holds anything)
+    const unsigned c0 = cum[s], c1 = cum[s + 1], c2 = cum[s + 2];
+    const bool up = slot >= c1;
+    miss |= slot >= c2;
+    const unsigned lo = up ? c1 : c0, hi = up ? c2 : c1;
+    x = (hi - lo) * xs + (slot - lo);
     r.renorm(x);
-    return s;
+    return s + up;
 }
-SG_DEVINL unsigned get_global(unsigned& x, RingReader& r, const uint8_t* __restrict__ ct) {
+SG_DEVINL unsigned get_global(unsigned& x, DecRing& r, const uint8_t* __restrict__ ct) {
     const unsigned* __restrict__ words = reinterpret_cast<const unsigned*>(ct + 256);
     const unsigned slot = x & ((1u << PB) - 1);
     unsigned s = ct[slot >> (PB - 8)];
@@ -314,10 +358,10 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
     __syncthreads();
     const bool staged = T.tab == cta_tab && !m.bad;
     const int nbatch = (m.nmax + DB - 1) / DB;
-    RingReader rd; rd.pos = rd.len = 0;
+    DecRing rd; rd.pos = rd.len = 0;
     unsigned x = RANS_L;
     bool bad = false;
-    if (chain && live) { rd.init(in + in_off[s], in + in_end[s], m.ring + grp, DSEG); x = rd.state(); }
+    if (chain && live) { rd.init(in + in_off[s], in + in_end[s], m.ring + grp); x = rd.state(); }
     unsigned short* base = reinterpret_cast<unsigned short*>(dev + T.doff);
     // a staging lane's first weight of the batch to stage and of the batch to store: compact row, column
     int rc = 0, j = 0, orc = 0, oj = 0;
@@ -338,16 +382,22 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
                 while (oj >= T.rowlen) { oj -= T.rowlen; ++orc; }
             }
             if (live && it < nbatch) {
-                int r = rc, col = j, have = -1, orow = 0;
+                int r[DW], col[DW];                              // (past the segment's end: its last weight again)
 #pragma unroll
                 for (int v = 0; v < DW; ++v) {
-                    if (it * DB + DW * gl + v < g.n) {
-                        if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
-                        int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
+                    r[v] = v ? r[v - 1] : rc; col[v] = v ? col[v - 1] : j;
+                    if (v && it * DB + DW * gl + v < g.n && ++col[v] == T.rowlen) { col[v] = 0; ++r[v]; }
+                }
+                if (it * DB + DW * gl < g.n) {
+                    unsigned e[DW];
+#pragma unroll
+                    for (int v = 0; v < DW; ++v) {
+                        int pred, pe, sc; contexts(c, T, T.rmap >= 0 ? c.rowmap[T.rmap + r[v]] : r[v], col[v], pred, pe, sc);
                         // (mctx() is constant outside of +-4000)
-                        m.ctx[it & 1][grp][DW * gl + v] = (unsigned)pe | (unsigned)sc << 9 | (unsigned)clampi(pred, -4000, 4000) << 16;
-                        if (++col == T.rowlen) { col = 0; ++r; }
+                        e[v] = (unsigned)pe | (unsigned)sc << 9 | (unsigned)clampi(pred, -4000, 4000) << 16;
                     }
+#pragma unroll
+                    for (int v = 0; v < DW; ++v) m.ctx[it & 1][grp][DW * gl + v] = e[v];
                 }
                 j += DB;
                 while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
@@ -361,20 +411,24 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
                 if ((w & 3) == 0) rd.top_up();                   // four weights take 24 bytes at most
                 const unsigned e = cx[w];
                 const int pe = e & 511, sc = (e >> 9) & 15, pred = (int)e >> 16;
-                unsigned ex, man;
-                if (staged && (unsigned)(pe - pe0) < (unsigned)D_ECTX) ex = get_staged<256>(x, rd, m.expo + (pe - pe0) * D_EP);
-                else ex = get_global(x, rd, lut + (size_t)(T.tab + pe) * RANS_COMPACT);
-                const int mc = mctx((int)ex, pred);
-                if (staged) man = get_staged<128>(x, rd, m.mant + mc * D_MP);
-                else man = get_global(x, rd, lut + (size_t)(T.tab + 512 + mc) * RANS_COMPACT);
+                // staged: exponent and mantissa; `miss`: from the start again, through global memory
+                const unsigned x0 = x, top0 = rd.top;
+                const int pos0 = rd.pos;
+                bool miss = !staged || (unsigned)(pe - pe0) >= (unsigned)D_ECTX;
+                unsigned ex = get_staged<256>(x, rd, m.expo + (miss ? 0 : pe - pe0) * D_EP, miss);
+                unsigned man = get_staged<128>(x, rd, m.mant + mctx((int)ex, pred) * D_MP, miss);
                 unsigned f01 = m.sign[sc];
-                if (!staged) {
-                    const unsigned* sw = reinterpret_cast<const unsigned*>(lut + (size_t)(T.tab + 640 + sc) * RANS_COMPACT + 256);
+                if (miss) {
+                    x = x0; rd.top = top0; rd.pos = pos0;
+                    const uint8_t* tl = lut + (size_t)T.tab * RANS_COMPACT;
+                    ex = get_global(x, rd, tl + (size_t)pe * RANS_COMPACT);
+                    man = get_global(x, rd, tl + (size_t)(512 + mctx((int)ex, pred)) * RANS_COMPACT);
+                    const unsigned* sw = reinterpret_cast<const unsigned*>(tl + (size_t)(640 + sc) * RANS_COMPACT + 256);
                     f01 = (sw[0] & 0xffffu) | (sw[1] << 16);
                 }
                 const unsigned slot = x & ((1u << PB) - 1), f0 = f01 & 0xffffu;
                 const bool neg = slot >= f0;                     // (two symbols: the second one starts where the first ends)
-                x = (neg ? f01 >> 16 : f0) * (x >> PB) + slot - (neg ? f0 : 0u);
+                x = (neg ? f01 >> 16 : f0) * (x >> PB) + (slot - (neg ? f0 : 0u));
                 rd.renorm(x);
                 o[w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
             }

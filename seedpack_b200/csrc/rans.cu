@@ -130,14 +130,14 @@ __global__ void __launch_bounds__(32) k_rans_encode(const uint8_t* __restrict__ 
         if (i > 0) look(nxt);
         table(); load();
 #pragma unroll
-        for (int k = 15; k >= 0; --k) rans_put<PB>(x, w, cur[k]);
+        for (int k = 15; k >= 0; k -= 2) rans_put2<PB>(x, w, cur[k], cur[k - 1]);
         if (w.ptr() < slot + 64) { out_len[s] = 0xffffffffu; return; }             // 16 symbols write at most 32 bytes
 #pragma unroll
         for (int k = 0; k < 16; ++k) cur[k] = nxt[k];
     }
     rans_flush(x, w);
     w.flush();
-    out_len[s] = w.bad ? LEN_NOFREQ : (unsigned)(slot + cap - w.ptr());
+    out_len[s] = w.bad() ? LEN_NOFREQ : (unsigned)(slot + cap - w.ptr());
 }
 
 // ---- scan + gather ---------------------------------------------------------------------------------------
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(64) k_rans_decode(const uint8_t* __restrict__ 
 // The same decoder with the tables it needs in shared memory.  A residual stream is mostly the symbol 0, whose slots are
 // [0, freq(0)) of every table: for those the step is x = freq(0) (x >> PB) + slot with freq(0) from a small array in
 // shared memory.  The other slots of a table - [freq(0), 2^PB), few when zeros dominate - get one 4-byte entry each,
-// symbol | (freq - 1) << 8 | (slot - cum) << 20, also in shared memory as far as they fit (tables in id order; the rest
+// symbol | (slot - cum) << 8 | (freq - 1) << 20, also in shared memory as far as they fit (tables in id order; the rest
 // keep the two dependent global loads lut[slot] -> enc[symbol]).  Every CTA builds the entries from enc / lut itself
 // (a few per cent of its decoding time; all 512 threads): the caller passes no further buffer.  One CTA per SM, whose first
 // `per` threads then decode a segment each: the segments are spread over all SMs before a CTA takes more of them.
@@ -229,11 +229,11 @@ __global__ void __launch_bounds__(512, 1) k_rans_decode_sm(const uint8_t* __rest
                                                            uint8_t* __restrict__ sym, int nseg, int ntab, unsigned cap, int per,
                                                            int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned smem[];
-    unsigned* base = smem;                                   // [ntab] first entry of the table, NOFIT if not staged
-    unsigned* ring = smem + ntab;                            // [RING_WORDS][per]
-    unsigned* ent = ring + RING_WORDS * per;                 // [cap]
-    unsigned short* f0 = reinterpret_cast<unsigned short*>(ent + cap);     // [ntab] freq(0)
     constexpr unsigned SLOTS = 1u << PB;
+    unsigned* base = smem;                                   // [ntab] first entry of the table, NOFIT if not staged
+    unsigned* ring = smem + ntab;                            // [per / 32][RING_ROWS][32]
+    unsigned* ent = smem + max((int)SLOTS, ntab + RING_ROWS * per);        // [cap]; SLOTS words before it can be read
+    unsigned short* f0 = reinterpret_cast<unsigned short*>(ent + cap);     // [ntab] freq(0)
     for (int t = threadIdx.x; t < ntab; t += blockDim.x) {
         const unsigned first = enc[(size_t)t * 256].fc & 0xffffu, last = enc[(size_t)t * 256 + 255].fc;
         const bool used = (last >> 16) + (last & 0xffffu) == SLOTS;
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(512, 1) k_rans_decode_sm(const uint8_t* __rest
         for (unsigned slot = f + (threadIdx.x & 31); slot < SLOTS; slot += 32) {
             const unsigned s = lut[((size_t)t << PB) + slot];
             const unsigned fc = enc[(size_t)t * 256 + s].fc;
-            ent[b + slot - f] = s | (((fc & 0xffffu) - 1u) << 8) | ((slot - (fc >> 16)) << 20);
+            ent[b + slot - f] = s | ((slot - (fc >> 16)) << 8) | (((fc & 0xffffu) - 1u) << 20);
         }
     }
     __syncthreads();
@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(512, 1) k_rans_decode_sm(const uint8_t* __rest
     const int s = (int)sl;
     const long long s0 = (long long)s * seg_len;
     const int n = (int)min((long long)seg_len, nsym - s0);
-    RingReader r;
-    r.init(in + off[s], in + off[s + 1], ring + threadIdx.x, per);
+    RingReader<32> r;
+    r.init(in + off[s], in + off[s + 1], ring + (threadIdx.x >> 5) * (RING_ROWS * 32) + (threadIdx.x & 31));
     unsigned x = r.state();
     const uint16_t* __restrict__ bt = block_tab + s0 / block_len;
     const int nblk = n / block_len;
@@ -275,31 +275,35 @@ __global__ void __launch_bounds__(512, 1) k_rans_decode_sm(const uint8_t* __rest
     for (int b = 0; b < nblk; ++b) {
         const unsigned tid = tid_next, tf0 = f0[tid], tb = base[tid];
         if (b + 1 < nblk) tid_next = __ldg(bt + b + 1);
-        const unsigned tb0 = tb == NOFIT ? 0u : tb;
+        // both kinds of slot without a branch: with 32 segments in a warp some lane meets a symbol other than 0 at most
+        // steps.  ent[] is read whatever the slot: for a slot of the symbol 0 that is some word before the table's entries
+        const unsigned* te = ent + (int)(tb == NOFIT ? 0u : tb) - (int)tf0;
+        const unsigned e0 = (tf0 - 1u) << 20;
         for (int i = 0; i < block_len; i += 16) {
             r.top_up();
             unsigned wv[4];
+            if (tb != NOFIT) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                unsigned word = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    // both kinds of slot without a branch: with 32 segments in a warp some lane meets a symbol other than 0
-                    // at most steps.  ent[] is read within bounds whatever the slot (an unstaged table reads its start)
-                    const unsigned slot = x & (SLOTS - 1);
-                    const bool nz = slot >= tf0;
-                    const unsigned e = ent[tb0 + (nz && tb != NOFIT ? slot - tf0 : 0u)];
-                    unsigned sy = nz ? e & 0xffu : 0u, f = nz ? ((e >> 8) & 0xfffu) + 1u : tf0, d = nz ? e >> 20 : slot;
-                    if (nz && tb == NOFIT) {
-                        sy = lut[((size_t)tid << PB) + slot];
-                        const unsigned fc = enc[(size_t)tid * 256 + sy].fc;
-                        f = fc & 0xffffu; d = slot - (fc >> 16);
-                    }
-                    x = f * (x >> PB) + d;
+                for (int k = 0; k < 16; ++k) {
+                    const unsigned slot = x & (SLOTS - 1), xs = x >> PB, en = te[slot];
+                    const unsigned e = slot >= tf0 ? en : e0 + (slot << 8);
+                    x = (e >> 20) * xs + (xs + ((e >> 8) & (SLOTS - 1)));
                     r.renorm(x);
-                    word |= sy << (8 * j);
+                    wv[k >> 2] = (k & 3) == 0 ? e & 0xffu : wv[k >> 2] | (e & 0xffu) << (8 * (k & 3));
                 }
-                wv[k] = word;
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) {
+                    unsigned word = 0;
+#pragma unroll 1
+                    for (int j = 0; j < 4; ++j) {
+                        const unsigned slot = x & (SLOTS - 1), sy = lut[((size_t)tid << PB) + slot], fc = enc[(size_t)tid * 256 + sy].fc;
+                        x = (fc & 0xffffu) * (x >> PB) + slot - (fc >> 16);
+                        r.renorm(x);
+                        word |= sy << (8 * j);
+                    }
+                    wv[0] = k == 0 ? word : wv[0]; wv[1] = k == 1 ? word : wv[1]; wv[2] = k == 2 ? word : wv[2]; wv[3] = k == 3 ? word : wv[3];
+                }
             }
             *reinterpret_cast<uint4*>(sym + s0 + (long long)b * block_len + i) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
             if (r.over()) { atomicOr(status, SG_ST_CORRUPT); return; }
@@ -389,13 +393,13 @@ extern "C" int sg_rans_decode(int device, void* stream, const unsigned char* in,
     cudaStream_t st = (cudaStream_t)stream;
     // tables staged in shared memory when their number is given and small enough to leave room for entries
     const size_t smem_max = 220 * 1024;
-    if (ntab > 0 && (size_t)ntab * 6 + 8192 + 256 * RING_WORDS * 4 <= smem_max) {
+    if (ntab > 0 && (size_t)ntab * 6 + 16384 + 256 * RING_ROWS * 4 <= smem_max) {
         // segments per CTA: as few as fill the SMs (a warp's worth at least), 256 at most (their rings take 128 bytes each)
         long long per = (nseg + 147) / 148;
         per = per <= 32 ? 32 : per >= 256 ? 256 : (per + 31) / 32 * 32;
-        const size_t ring = (size_t)per * RING_WORDS * 4;
-        const unsigned cap = (unsigned)((smem_max - (size_t)ntab * 6 - 16 - ring) / 4);
-        const size_t smem = (size_t)ntab * 4 + ring + (size_t)cap * 4 + (size_t)ntab * 2 + 16;
+        const size_t head = (size_t)ntab * 4 + (size_t)per * RING_ROWS * 4, front = head > (4 << 12) ? head : 4 << 12;
+        const unsigned cap = (unsigned)((smem_max - front - (size_t)ntab * 2 - 16) / 4);
+        const size_t smem = front + (size_t)cap * 4 + (size_t)ntab * 2 + 16;
         static bool configured[64] = {false};
         if (device < 64 && !configured[device]) {
             rc = cuda_ok(cudaFuncSetAttribute(k_rans_decode_sm<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max + 1024));

@@ -27,27 +27,34 @@ struct __align__(8) RansSym { unsigned rcp, fc; };
 SG_DEVINL unsigned rans_shift(unsigned freq) { return freq < 2 ? 0u : 32u - __clz(freq - 1); }
 
 // ---- downward byte writer ----------------------------------------------------------------------------
-// Writes bytes at decreasing addresses ending at `end` (4-byte aligned).  Pending bytes sit in `acc`, the last one lowest;
-// whenever four are there the oldest four leave as one aligned word.
+// Writes bytes at decreasing addresses ending at `end` (4-byte aligned).  Pending bytes sit at the top of a 64-bit register,
+// the last one highest: a step shifts the low bytes of its state in (two funnel shifts).  Whenever four are pending the
+// oldest four leave as one aligned word; two steps between flushes are the most that fits.
 struct ByteWriterDown {
     uint8_t* p;                    // lowest address stored so far
-    unsigned long long acc;        // pending bytes (what is above them has left already)
-    int cnt;                       // how many: 0 .. 3 between calls
-    unsigned bad;                  // set when a symbol with frequency 0 was coded (tables not made from these symbols)
-    SG_DEVINL void init(uint8_t* end) { p = end; acc = 0; cnt = 0; bad = 0; }
-    SG_DEVINL bool push(unsigned x, int n) {                   // the n <= 2 low bytes of x, the lowest first
-        const unsigned v = n == 2 ? __byte_perm(x, 0, 0x4401) : n ? x & 0xffu : 0u;
-        acc = (acc << (8 * n)) | v;
-        cnt += n;
-        return cnt >= 4;
+    unsigned hi, lo;               // pending bytes
+    int bits;                      // 8 x how many
+    unsigned minf;                 // smallest frequency coded: 0 = tables not made from these symbols
+    SG_DEVINL void init(uint8_t* end) { p = end; hi = lo = 0; bits = 0; minf = 1; }
+    SG_DEVINL void push(unsigned x, int n8) {                  // the n8 / 8 <= 2 low bytes of x, the lowest first
+        lo = __funnelshift_r(lo, hi, n8);
+        hi = __funnelshift_r(hi, x, n8);
+        bits += n8;
     }
-    SG_DEVINL void emit(unsigned x, int n) {
-        if (push(x, n)) { cnt -= 4; p -= 4; *reinterpret_cast<unsigned*>(p) = (unsigned)(acc >> (8 * cnt)); }
+    SG_DEVINL unsigned oldest() const { return __byte_perm(__funnelshift_rc(lo, hi, 64 - bits), 0, 0x0123); }       // bits >= 32
+    SG_DEVINL void drain() {
+        if (bits >= 32) { p -= 4; *reinterpret_cast<unsigned*>(p) = oldest(); bits -= 32; }
     }
+    SG_DEVINL bool bad() const { return minf == 0; }
     // bytes written so far end at this address (the lowest written byte)
-    SG_DEVINL uint8_t* ptr() const { return p - cnt; }
+    SG_DEVINL uint8_t* ptr() const { return p - (bits >> 3); }
     // store the pending bytes
-    SG_DEVINL void flush() { for (; cnt > 0; --cnt) *--p = (uint8_t)(acc >> (8 * (cnt - 1))); }
+    SG_DEVINL void flush() {
+        drain();
+        const int n = bits >> 3;
+        for (int k = 0; k < n; ++k) p[-1 - k] = (uint8_t)(hi >> (32 - bits + 8 * k));
+        p -= n; bits = 0;
+    }
 };
 
 // ---- forward byte reader -----------------------------------------------------------------------------
@@ -91,14 +98,16 @@ struct ByteReaderUp {
 // the whole warp wait for that load, and with 8 - 32 segments per warp some lane refills at almost every symbol.  Here all
 // lanes top their rings up together, every few symbols, with the 32 bytes that were asked for at the last top-up; a
 // symbol takes its next four bytes from two shared-memory words, off the state's own chain.
-// A lane's ring: 32 words at a stride of `pitch` words.  Between two top-ups a lane may take 32 bytes (16 symbols).
-constexpr int RING_WORDS = 32;
+// A lane's ring: 32 words and a copy of the first (a read takes two neighbours) at a pitch of P words.  Between two
+// top-ups a lane may take 32 bytes (16 symbols).
+constexpr int RING_WORDS = 32, RING_ROWS = RING_WORDS + 1;
+template <int P>
 struct RingReader {
     const uint8_t* src;            // next 32 bytes to ask for (16-byte aligned)
     const uint8_t* end;
     uint4 c0, c1;                  // the 32 bytes asked for last
-    unsigned* ring; int pitch;
-    int pos, have, len;            // bytes from the aligned start: taken, put into the ring, in the stream
+    unsigned* ring;
+    int pos, have, len;            // bits from the aligned start: taken, put into the ring, in the stream
     unsigned top;                  // the next four bytes, the first one highest
     SG_DEVINL void fetch() {
         c0 = c1 = make_uint4(0, 0, 0, 0);
@@ -106,28 +115,29 @@ struct RingReader {
         if (src + 16 < end) c1 = *reinterpret_cast<const uint4*>(src + 16);
         src += 32;
     }
-    SG_DEVINL void put(const uint4 v, int w) {
-        const unsigned a[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ring[((w + i) & (RING_WORDS - 1)) * pitch] = __byte_perm(a[i], 0, 0x0123);
-    }
     SG_DEVINL void top_up() {
-        if (have - pos <= 4 * RING_WORDS - 32) {
-            put(c0, have >> 2); put(c1, (have >> 2) + 4);
-            have += 32;
+        if (have - pos <= 8 * (4 * RING_WORDS - 32)) {
+            const int w = (have >> 5) & (RING_WORDS - 1);      // a multiple of 8
+            unsigned* r = ring + w * P;
+            const unsigned a[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i * P] = __byte_perm(a[i], 0, 0x0123);
+            if (w == 0) ring[RING_WORDS * P] = __byte_perm(a[0], 0, 0x0123);
+            have += 256;
             fetch();
         }
     }
     SG_DEVINL void look() {
-        const unsigned hi = ring[((pos >> 2) & (RING_WORDS - 1)) * pitch], lo = ring[((pos >> 2) + 1 & (RING_WORDS - 1)) * pitch];
-        top = __funnelshift_l(lo, hi, 8 * (pos & 3));
+        const unsigned off = (P >= 8 ? (unsigned)pos * (P / 8) : (unsigned)pos / (8 / P)) & ((RING_WORDS - 1) * P * 4);
+        const unsigned* r = reinterpret_cast<const unsigned*>(reinterpret_cast<const char*>(ring) + off);
+        top = __funnelshift_l(r[P], r[0], pos);                // (the shift counts modulo 32)
     }
-    SG_DEVINL void init(const uint8_t* begin, const uint8_t* e, unsigned* r, int stride) {
-        ring = r; pitch = stride;
+    SG_DEVINL void init(const uint8_t* begin, const uint8_t* e, unsigned* r) {
+        ring = r;
         src = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(begin) & ~(uintptr_t)15);
-        pos = (int)(begin - src); have = 0;
+        pos = 8 * (int)(begin - src); have = 0;
         end = e > begin ? e : begin;
-        len = (int)min((long long)(end - src), 0x7fffff00LL);
+        len = 8 * (int)min((long long)(end - src), 1LL << 27); // (a segment's symbols take far less)
         if (end == begin) end = src;                           // nothing to read
         fetch();
         top_up(); top_up(); top_up();
@@ -135,18 +145,15 @@ struct RingReader {
     }
     SG_DEVINL bool over() const { return pos > len; }
     SG_DEVINL bool at_end() const { return pos == len; }
-    // x after a step: take bytes until x >= 2^23 (a stream that was coded needs at most two)
+    // x after a step: the bytes that bring it to 2^23 or more.  A coder's state is 2^23 or more before a step, hence 2^8 or
+    // more after it: two bytes at most.  (A damaged stream may leave it smaller; it is found out at the segment's end.)
     SG_DEVINL void renorm(unsigned& x) {
-        int n = x < (1u << 15) ? 2 : x < RANS_L ? 1 : 0;
-        x = __funnelshift_l(top, x, 8 * n);
-        pos += n;
+        const int n8 = x < (1u << 15) ? 16 : x < RANS_L ? 8 : 0;
+        x = __funnelshift_l(top, x, n8);
+        pos += n8;
         look();
-        if (x < RANS_L && n) {                                 // damaged streams only
-#pragma unroll 1
-            for (int guard = 0; guard < 2 && x < RANS_L; ++guard) { x = __funnelshift_l(top, x, 8); ++pos; look(); }
-        }
     }
-    SG_DEVINL unsigned state() { const unsigned x = top; pos += 4; look(); return x; }
+    SG_DEVINL unsigned state() { const unsigned x = top; pos += 32; look(); return x; }
 };
 
 // ---- coder steps -------------------------------------------------------------------------------------
@@ -160,22 +167,39 @@ inline int segs_per_warp(long long nseg) {
     return n <= 8 ? 8 : n >= 32 ? 32 : (int)n;
 }
 constexpr unsigned RANS_NOP_RCP = 1u << 31;        // with freq = 2^12, cum = 0 (12 bits): an entry that leaves the state as it is
+// what a step needs of an entry
+struct RansStep { unsigned xm, rcp, sh_comp, bias; };                              // sh_comp = shift | (2^PB - freq) << 5
+template <int PB> SG_DEVINL RansStep rans_step_of(const RansSym e) {
+    const unsigned f = e.fc & 0xffffu, c = e.fc >> 16;
+    const unsigned sh = f < 2 ? 0u : 31u - __clz(f - 1);
+    return {e.fc << (31 - PB), e.rcp, sh | ((1u << PB) - f) << 5, f < 2 ? c + (1u << PB) - 1u : c};
+}
+template <class W>
+SG_DEVINL void rans_put(unsigned& x, W& w, const RansStep t) {
+    // x < 2^31 and xm >= 2^(31 - PB) for f >= 1: at most two bytes leave per symbol (PB <= 15)
+    const int n8 = (x >> 8) >= t.xm ? 16 : x >= t.xm ? 8 : 0;
+    w.push(x, n8);
+    x >>= n8;
+    const unsigned q = __umulhi(x, t.rcp) >> (t.sh_comp & 31u);
+    x = q * (t.sh_comp >> 5) + (x + t.bias);
+}
+// one symbol, or two with one look at the pending bytes
 template <int PB, class W>
 SG_DEVINL void rans_put(unsigned& x, W& w, const RansSym e) {
-    const unsigned f = e.fc & 0xffffu, c = e.fc >> 16;
-    const unsigned xm = f << (31 - PB);
-    // x < 2^31 and xm >= 2^(31 - PB) for f >= 1: at most two bytes leave per symbol (PB <= 15); a zero frequency marks the segment
-    w.bad |= (unsigned)(f == 0);
-    const int n = x >= xm ? ((x >> 8) >= xm ? 2 : 1) : 0;
-    w.emit(x, n);
-    x >>= 8 * n;
-    const unsigned sh = f < 2 ? 0u : 31u - __clz(f - 1), bias = f < 2 ? c + (1u << PB) - 1u : c;
-    const unsigned q = __umulhi(x, e.rcp) >> sh;
-    x = q * ((1u << PB) - f) + (x + bias);
+    w.minf = min(w.minf, e.fc & 0xffffu);
+    rans_put(x, w, rans_step_of<PB>(e));
+    w.drain();
+}
+template <int PB, class W>
+SG_DEVINL void rans_put2(unsigned& x, W& w, const RansSym e, const RansSym f) {
+    w.minf = min(w.minf, min(e.fc & 0xffffu, f.fc & 0xffffu));
+    rans_put(x, w, rans_step_of<PB>(e));
+    rans_put(x, w, rans_step_of<PB>(f));
+    w.drain();
 }
 template <class W> SG_DEVINL void rans_flush(unsigned x, W& w) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { w.emit(x, 1); x >>= 8; }
+    for (int i = 0; i < 4; ++i) { w.push(x, 8); w.drain(); x >>= 8; }
 }
 template <class R> SG_DEVINL unsigned rans_init(R& r) {
     unsigned x = 0;
