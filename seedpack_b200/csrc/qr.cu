@@ -428,19 +428,50 @@ __global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, con
     if (have && sub == 0 && !c.finished()) atomicOr(status, SG_ST_CORRUPT);
 }
 
-// ---- decoder of the lattice types: a warp per segment ------------------------------------------------------------------
+// ---- decoder of the lattice types: a CTA per segment -------------------------------------------------------------------
 // What makes these blocks expensive is the ordering of all 256 - 2048 lattice points by their weighted distance to the
-// seed, once per group of 4 / 8 weights.  Here the 32 lanes of the warp share that: every lane measures the points
-// lane, lane + 32, ... and keeps its own 16 closest in order; the warp's closest, second closest, ... come out of
-// rounds of an arg-min over the lanes' list heads (only as many rounds as the decoded rank needs).  Everything that is
-// one chain (flag, fields, ranks, signs) is decoded by all lanes in lockstep.
-struct GridWarpSmem {
-    unsigned fblk[28], pblk[28];            // block sizes <= 110 bytes
-    float xs[256];                          // the block's seed values
-    float tab[128];                         // pair tables of the group being ranked: [pair][levels]
-    float dist[2048];                       // distance of every lattice point of the group being ranked
-    float gu[256], gw[256];                 // per weight: seed value over the unit's scale (sign-folded), search weight
-    unsigned char pn[32];                   // per unit of 8 weights: which seed values count as negative
+// seed, once per group of 4 / 8 weights.  It depends on the seed and on the block's scale fields only, so that once the
+// fields are decoded the eight warps rank all groups of the block side by side (four units of 8 weights each): the closest
+// four points and the gap context of every group go to shared memory.  The first warp then runs the chain - ranks and
+// signs - over them, all lanes in lockstep, while the others fetch the next block and sum its squares.  A rank beyond the
+// fourth is looked up when it occurs.  (One warp per segment that ranked a group when the chain came to it: 6100 cycles
+// a group, 13.2 ms for the 1024 x 3072 weights of an IQ3_S tensor.)
+constexpr int GW = 8, GTOP = 4;                    // warps per CTA; ranked points kept per group
+struct GridSmem {
+    unsigned f01[NTAB2];                           // per table: frequency of symbol 0 | of symbol 1 << 16
+    unsigned ring[RING_ROWS];
+    unsigned fblk[28], pblk[2][28];                // block sizes <= 110 bytes
+    float xs[2][256];                              // the block's seed values; this block and the next
+    float sx2[2];
+    float tab[GW][128];                            // pair tables of the group a warp ranks: [pair][levels]
+    float dist[2048];                              // distance of every lattice point (ranks beyond GTOP)
+    float gu[256], gw[256];                        // per weight: seed value over the unit's scale (sign-folded), search weight
+    unsigned short gk[2048];                       // the lattice's points
+    unsigned short top[2][64][GTOP];               // [IQ1_M's shift bit][group]: closest points in order, 0xffff: none
+    unsigned char gap[2][64];
+    unsigned char pn[32], neg[32], shift[32];      // per unit: negative seed values; decoded sign symbols, shift bit
+    unsigned short tg[64];
+    int tv[MAXF];
+    int eq;
+};
+struct GridDec {
+    unsigned x; RingReader<1> r; const RansSym* enc; const uchar* lut; const unsigned* f01;
+    // w = f01[tab].  Symbols 0 and 1 without a load
+    SG_DEVINL int step(int tab, unsigned w) {
+        const unsigned slot = x & 4095u, f0 = w & 0xffffu, f1 = w >> 16;
+        const bool one = slot >= f0;
+        int s = one;
+        unsigned f = one ? f1 : f0, d = one ? slot - f0 : slot;
+        if (slot >= f0 + f1) {
+            s = lut[((size_t)tab << 12) + slot];
+            const unsigned fc = enc[tab * 256 + s].fc;
+            f = fc & 0xffffu; d = slot - (fc >> 16);
+        }
+        x = f * (x >> 12) + d;
+        r.renorm(x);
+        return s;
+    }
+    SG_DEVINL int get(int tab) { return step(tab, f01[tab]); }
 };
 template <int N> SG_DEVINL float point_dist_w(const float* tab, unsigned key) {
     constexpr int B = N == 8 ? 2 : 3, E = 1 << (2 * B);
@@ -449,175 +480,263 @@ template <int N> SG_DEVINL float point_dist_w(const float* tab, unsigned key) {
     for (int p = 0; p < N / 2; ++p) d = d + tab[p * E + ((key >> (2 * B * p)) & (E - 1))];
     return isnan(d) ? __int_as_float(0x7f800000) : d;
 }
-template <int N, bool SGN>
-SG_DEVINL void grid_block_warp(WarpDec& c, GridWarpSmem& m, int lane, int T, int mv, const int* tv, const uint16_t* __restrict__ gk,
-                               long long gw0, int cols, const float* im) {
-    constexpr int B = N == 8 ? 2 : 3, ng = 8 / N, L = 1 << B, E = L * L;
-    const float inf = __int_as_float(0x7f800000);
-    uchar* fb = reinterpret_cast<uchar*>(m.fblk);
-    const uchar* pb = reinterpret_cast<const uchar*>(m.pblk);
-    const int gs = grid_size(T);
-    const bool par = parity_type(T);
-    float sx2 = 0.f;
-    for (int i = 0; i < 256; ++i) { const float xv = m.xs[i]; sx2 += xv * xv; }
-    const float sigma2 = (T == 16 || T == 17) ? sx2 * (1.0f / 256.f) : 2.f * sx2 * (1.0f / 256.f);
-    const long long col0 = cols > 0 ? gw0 % cols : 0;
-    // what a unit's ranking needs from the seed, one unit per lane: weights, sign folding with the parity repair, values
-    // over the unit's scale (the scale does not depend on IQ1_M's shift bit, only the level offset does)
-    {
-        const int u = lane;
-        float gs_, gdl0;
-        gscale(T, fb, tv, u, gs_, gdl0);
-        float x[8], v[8], wv[8];
-        int pnb = 0;
-        for (int i = 0; i < 8; ++i) {
-            x[i] = m.xs[8 * u + i];
-            float wi = sqrtf(sigma2 + x[i] * x[i]);
-            if (im) wi = wi * im[(gw0 + 8 * u + i) % cols];
-            wv[i] = wi;
-            if (x[i] < 0.f) pnb |= 1 << i;
-            v[i] = SGN ? fabsf(x[i]) : x[i];
-        }
-        if (SGN && par && (__popc(pnb) & 1)) {         // an odd number of negatives: the least weighty one flips back
-            int imin = 0; float mn = wv[0] * x[0] * x[0];
-            for (int i = 1; i < 8; ++i) { const float a = wv[i] * x[i] * x[i]; if (a < mn) { mn = a; imin = i; } }
-            pnb ^= 1 << imin;
-            for (int i = 0; i < 8; ++i) if (i == imin) v[i] = -v[i];
-        }
-        for (int i = 0; i < 8; ++i) { m.gu[8 * u + i] = v[i] / gs_; m.gw[8 * u + i] = wv[i]; }
-        m.pn[u] = (unsigned char)pnb;
-    }
-    __syncwarp();
-    for (int u = 0; u < 32; ++u) {
-        const int p4 = pos4(col0 + 8 * u, cols);
-        const int rank0 = mv >= 2 ? GRANK2 + 4 * p4 : GRID_RANK;
-        const int sign0 = mv >= 2 ? GSIGN2 + 16 * p4 : GRID_SIGN;
-        if (T == 29) { if (c.get(GRID_SHIFT) ^ get_shift(pb, u)) { if (lane == 0) put_shift(fb, u); } __syncwarp(); }
-        float gu[8], gw[8], gs_, gdl;
-        int pn[8];
-        gscale(T, fb, tv, u, gs_, gdl);
-        for (int i = 0; i < 8; ++i) { gu[i] = m.gu[8 * u + i]; gw[i] = m.gw[8 * u + i]; pn[i] = (m.pn[u] >> i) & 1; }
-        int tg[2] = {0, 0};
-        for (int gg = 0; gg < ng; ++gg) {
-            // pair tables of this group, entries spread over the lanes
-            __syncwarp();
-            for (int e = lane; e < (N / 2) * E; e += 32) {
-                const int p = e / E, ee = e % E, la = ee & (L - 1), lb = ee >> B;
-                const float qa = SGN ? (float)(2 * la + 1) : (float)(la - 1) + gdl;
-                const float qb = SGN ? (float)(2 * lb + 1) : (float)(lb - 1) + gdl;
-                float ua = 0.f, ub = 0.f, wa = 0.f, wb = 0.f;
+// pair tables of the group of weights w0 .. w0 + N - 1, entries spread over the lanes
+template <int N, bool SGN> SG_DEVINL void group_tables(float* tab, const GridSmem& m, int w0, float gdl, int lane) {
+    constexpr int B = N == 8 ? 2 : 3, L = 1 << B, E = L * L;
 #pragma unroll
-                for (int i = 0; i < N / 2; ++i) if (i == p) { ua = gu[gg * N + 2 * i]; ub = gu[gg * N + 2 * i + 1]; wa = gw[gg * N + 2 * i]; wb = gw[gg * N + 2 * i + 1]; }
-                const float ea = qa - ua, eb = qb - ub;
-                m.tab[e] = wa * (ea * ea) + wb * (eb * eb);
-            }
-            __syncwarp();
-            // distances of all points; every lane remembers the closest of its own (points lane, lane + 32, ...)
-            float md = inf; int mk = 0x7fffffff;
-            for (int k = lane; k < gs; k += 32) {
-                const float d = point_dist_w<N>(m.tab, __ldg(gk + k));
-                m.dist[k] = d;
-                if (d < md) { md = d; mk = k; }
-            }
-            // the warp's next closest point in the order (distance, index): arg-min over the lanes' closest; the winning
-            // lane strikes its point out and looks for its next one.  Points at infinite distance never come up.
-            auto next = [&](float& bd, int& bk) {
-                bd = md; bk = mk;
-#pragma unroll
-                for (int sft = 16; sft > 0; sft >>= 1) {
-                    const float od = __shfl_xor_sync(0xffffffffu, bd, sft);
-                    const int ok = __shfl_xor_sync(0xffffffffu, bk, sft);
-                    if (od < bd || (od == bd && ok < bk)) { bd = od; bk = ok; }
-                }
-                if (bk == mk && bk != 0x7fffffff) {
-                    m.dist[mk] = inf;
-                    md = inf; mk = 0x7fffffff;
-                    for (int k = lane; k < gs; k += 32) { const float d = m.dist[k]; if (d < md) { md = d; mk = k; } }
-                }
-            };
-            float d1, d2; int k1, k2;
-            next(d1, k1); next(d2, k2);
-            const int r = c.get(rank0 + gapctx(d1, d2));
-            int t;
-            if (r >= TOPK) { const int lo = c.get(FESC_LO), hi = c.get(FESC_HI); t = (lo | (hi << 8)) % gs; }
-            else {
-                // slot r of the ordered list; slots beyond the points at finite distance keep their own number
-                t = r == 0 ? k1 : k2;
-                for (int j = 2; j <= r; ++j) { float dj; next(dj, t); }
-                if (t == 0x7fffffff) t = r;
-            }
-            if (lane == 0) put_gidx(T, fb, u * ng + gg, t);
-            tg[gg] = t;
-        }
-        __syncwarp();
-        if (SGN) for (int j = 0; j < 8; ++j) {
-            if (par && j == 7) continue;
-            const int lev = (gk[tg[j / N]] >> (B * (j % N))) & ((1 << B) - 1);
-            const float m4 = fabsf(gu[j]) * 4.f;
-            const int sctx = sign0 + (lev == 0) * 8 + (m4 < 7.f ? (int)m4 : 7);
-            if (c.get(sctx) ^ pn[j]) { if (lane == 0) put_neg(T, fb, 8 * u + j); }
-        }
-        __syncwarp();
-        if (c.over) return;
+    for (int e = lane; e < (N / 2) * E; e += 32) {
+        const int p = e / E, ee = e % E, la = ee & (L - 1), lb = ee >> B;
+        const float qa = SGN ? (float)(2 * la + 1) : (float)(la - 1) + gdl;
+        const float qb = SGN ? (float)(2 * lb + 1) : (float)(lb - 1) + gdl;
+        const float ea = qa - m.gu[w0 + 2 * p], eb = qb - m.gu[w0 + 2 * p + 1];
+        tab[e] = m.gw[w0 + 2 * p] * (ea * ea) + m.gw[w0 + 2 * p + 1] * (eb * eb);
     }
 }
+// a float's bits in an unsigned order (no NaN comes here)
+SG_DEVINL unsigned ordered_bits(float d) { const unsigned u = __float_as_uint(d); return u ^ ((unsigned)((int)u >> 31) | 0x80000000u); }
 
-__global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_grid_warp(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
-                                                                    const RansSym* __restrict__ enc, const uchar* __restrict__ lut,
-                                                                    uchar* __restrict__ F, int* __restrict__ status) {
-    __shared__ unsigned short f0[NTAB2];
-    __shared__ GridWarpSmem wsm[DW_WARPS];
-    for (int t = threadIdx.x; t < NTAB2; t += blockDim.x) f0[t] = (unsigned short)(enc[t * 256].fc & 0xffffu);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, s = blockIdx.x * DW_WARPS + (threadIdx.x >> 5);
-    if (s >= a.nseg) return;
-    GridWarpSmem& m = wsm[threadIdx.x >> 5];
-    const int T = a.T, mv = a.mv;
+// Closest GTOP points of one group in the order (distance, index), and its gap context.  Every lane keeps the closest of
+// its own points (lane, lane + 32, ...; met in index order, so that on equal distances the earlier one stays ahead);
+// the warp's next one is then an arg-min over the lanes' lists.  Points at infinite distance never come up.
+template <int N, bool SGN> SG_DEVINL void rank_group(GridSmem& m, float* tab, int gs, int w0, float gdl, int lane, unsigned short* top, unsigned char* gap) {
+    const float inf = __int_as_float(0x7f800000);
+    __syncwarp();
+    group_tables<N, SGN>(tab, m, w0, gdl, lane);
+    __syncwarp();
+    float D[GTOP]; int K[GTOP];
+#pragma unroll
+    for (int l = 0; l < GTOP; ++l) { D[l] = inf; K[l] = 0xffff; }
+#pragma unroll 4
+    for (int k0 = 0; k0 < gs; k0 += 32) {
+        float d = point_dist_w<N>(tab, m.gk[k0 + lane]);
+        int k = k0 + lane;
+#pragma unroll
+        for (int l = 0; l < GTOP; ++l) {
+            const bool lt = d < D[l];
+            const float dm = D[l]; const int km = K[l];
+            D[l] = lt ? d : dm; K[l] = lt ? k : km;
+            d = lt ? dm : d; k = lt ? km : k;
+        }
+    }
+    float d1 = inf, d2 = inf;
+#pragma unroll
+    for (int j = 0; j < GTOP; ++j) {
+        const unsigned key = ordered_bits(D[0]), best = __reduce_min_sync(0xffffffffu, key);
+        const unsigned bk = __reduce_min_sync(0xffffffffu, key == best ? (unsigned)K[0] : 0xffffu);
+        if (lane == 0) top[j] = (unsigned short)bk;
+        if (j < 2) {
+            const float d = __uint_as_float(best ^ ((best >> 31) ? 0x80000000u : 0xffffffffu));
+            if (j == 0) d1 = d; else d2 = d;
+        }
+        if (key == best && (unsigned)K[0] == bk) {
+#pragma unroll
+            for (int l = 0; l + 1 < GTOP; ++l) { D[l] = D[l + 1]; K[l] = K[l + 1]; }
+            D[GTOP - 1] = inf; K[GTOP - 1] = 0xffff;
+        }
+    }
+    if (lane == 0) *gap = (unsigned char)gapctx(d1, d2);
+}
+// the point of rank r >= GTOP, by the first warp: distances to shared memory, then r + 1 rounds of an arg-min
+template <int N, bool SGN> SG_DEVINL int deep_rank(GridSmem& m, int gs, int w0, float gdl, int r, int lane) {
+    const float inf = __int_as_float(0x7f800000);
+    __syncwarp();
+    group_tables<N, SGN>(m.tab[0], m, w0, gdl, lane);
+    __syncwarp();
+    float md = inf; int mk = 0x7fffffff;
+    for (int k = lane; k < gs; k += 32) {
+        const float d = point_dist_w<N>(m.tab[0], m.gk[k]);
+        m.dist[k] = d;
+        if (d < md) { md = d; mk = k; }
+    }
+    int bk = 0x7fffffff;
+    for (int j = 0; j <= r; ++j) {
+        float bd = md; bk = mk;
+#pragma unroll
+        for (int sft = 16; sft > 0; sft >>= 1) {
+            const float od = __shfl_xor_sync(0xffffffffu, bd, sft);
+            const int ok = __shfl_xor_sync(0xffffffffu, bk, sft);
+            if (od < bd || (od == bd && ok < bk)) { bd = od; bk = ok; }
+        }
+        if (bk == mk && bk != 0x7fffffff) {
+            m.dist[mk] = inf;
+            md = inf; mk = 0x7fffffff;
+            for (int k = lane; k < gs; k += 32) { const float d = m.dist[k]; if (d < md) { md = d; mk = k; } }
+        }
+        __syncwarp();
+    }
+    return bk == 0x7fffffff ? r : bk;              // slots beyond the points at finite distance keep their own number
+}
+
+template <int T>
+__global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
+                                                         const RansSym* __restrict__ enc, const uchar* __restrict__ lut,
+                                                         uchar* __restrict__ F, int* __restrict__ status) {
+    constexpr int N = T == 18 || T == 21 ? 4 : 8, ng = 8 / N, B = N == 8 ? 2 : 3, gs = grid_size(T), bs = bs_of(T), nf = nfield(T);
+    constexpr bool SGN = T != 19 && T != 29, par = parity_type(T);
+    __shared__ __align__(16) GridSmem m;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.x, mv = a.mv;
     const Setup u = setup(T, a.seed, a.tm, a.sg, s);
     const float* im = u.m.imx_off >= 0 ? a.imx + u.m.imx_off : nullptr;
-    WarpDec c; c.enc = enc; c.lut = lut; c.f0 = f0;
-    c.init(in + off[s], in + off[s + 1]);
-    uchar* fb = reinterpret_cast<uchar*>(m.fblk);
-    const uchar* pbs = reinterpret_cast<const uchar*>(m.pblk);
+    for (int t = threadIdx.x; t < NTAB2; t += GW * 32) m.f01[t] = (enc[t * 256].fc & 0xffffu) | (enc[t * 256 + 1].fc << 16);
+    for (int k = threadIdx.x; k < gs; k += GW * 32) m.gk[k] = a.gk[k];
+    // block j of the segment into buffer j & 1, by the threads of warps w0 .. GW - 1
+    auto fetch = [&](int j, int w0) {
+        const int t = (int)threadIdx.x - 32 * w0;
+        if (t < 0 || j >= u.g.nb) return;
+        const long long b = u.g.b0 + j, gw0 = (b - u.m.blk0) * 256;
+        for (int i = t; i < bs; i += 32 * (GW - w0)) reinterpret_cast<uchar*>(m.pblk[j & 1])[i] = a.P[b * bs + i];
+        for (int i = t; i < 256; i += 32 * (GW - w0)) { float xv, hv; seed_val(u.m.seed_type, u.sbase, gw0 + i, xv, hv, u.m.cols); m.xs[j & 1][i] = xv; }
+    };
+    auto sum_squares = [&](int j) {                // in order; one warp, every lane the same
+        float sx2 = 0.f;
+#pragma unroll 16
+        for (int i = 0; i < 256; ++i) { const float xv = m.xs[j & 1][i]; sx2 += xv * xv; }
+        if (lane == 0) m.sx2[j & 1] = sx2;
+    };
+    fetch(0, 0);
+    __syncthreads();
+    if (warp == 1) sum_squares(0);
+    GridDec c; c.enc = enc; c.lut = lut; c.f01 = m.f01;
     int prev = 1;
-    for (long long b = u.g.b0; b < u.g.b0 + u.g.nb && !c.over; ++b) {
-        const uchar* pg = a.P + b * u.bs;
-        uchar* fg = F + b * u.bs;
-        const int eq = c.get(FLAG + prev);
-        prev = eq;
-        if (eq) { for (int i = lane; i < u.bs; i += 32) fg[i] = pg[i]; continue; }
-        const long long gw0 = (b - u.m.blk0) * u.qk;
-        __syncwarp();
-        if (lane < 28) m.fblk[lane] = 0;
-        for (int i = lane; i < u.bs; i += 32) reinterpret_cast<uchar*>(m.pblk)[i] = pg[i];
-        for (int i = lane; i < 256; i += 32) { float xv, hv; seed_val(u.m.seed_type, u.sbase, gw0 + i, xv, hv, u.m.cols); m.xs[i] = xv; }
-        __syncwarp();
-        int tv[MAXF], pv[MAXF];
-        unpack_fields(T, pbs, pv);
-        int any = 0;
-        for (int k = 0; k < u.nf; ++k) {
-            const int kd = fkind(T, k);
-            const int pr = fpred(T, mv, pv, k, k > 0 ? tv[0] : 0, k > 1 ? tv[1] : 0);
-            const int sym = c.get(fctx(kd, any));
-            int t;
-            if (kd < 2 && sym == 128) { const int lo = c.get(FESC_LO), hi = c.get(FESC_HI); t = lo | (hi << 8); }
-            else {
-                t = pr + (int)(signed char)sym;
-                if (kd < 2) t &= 0xffff;
+    if (warp == 0) { c.r.init(in + off[s], in + off[s + 1], m.ring); c.x = c.r.state(); }
+    uchar* fb = reinterpret_cast<uchar*>(m.fblk);
+    for (int j = 0; j < u.g.nb; ++j) {
+        const long long b = u.g.b0 + j, gw0 = (b - u.m.blk0) * 256;
+        const uchar* pbs = reinterpret_cast<const uchar*>(m.pblk[j & 1]);
+        if (warp == 0) {
+            __syncwarp();                          // (the ring is one for all lanes: no lane runs ahead into a top-up)
+            c.r.top_up();
+            int eq = c.get(FLAG + prev);
+            prev = eq;
+            if (c.r.over()) eq = 2;                // a damaged stream: no more blocks
+            if (eq == 0) {
+                int pv[MAXF], tv[MAXF];
+                unpack_fields(T, pbs, pv);
+                int any = 0;
+#pragma unroll
+                for (int k = 0; k < nf; ++k) {
+                    if ((k & 3) == 0) { __syncwarp(); c.r.top_up(); }
+                    const int kd = fkind(T, k);
+                    const int pr = fpred(T, mv, pv, k, k > 0 ? tv[0] : 0, k > 1 ? tv[1] : 0);
+                    const int sym = c.get(fctx(kd, any));
+                    int t;
+                    if (kd < 2 && sym == 128) { const int lo = c.get(FESC_LO), hi = c.get(FESC_HI); t = lo | (hi << 8); }
+                    else {
+                        t = pr + (int)(signed char)sym;
+                        if (kd < 2) t &= 0xffff;
+                    }
+                    tv[k] = t; any |= t != pr;
+                }
+                if (lane < 28) m.fblk[lane] = 0;
+                __syncwarp();
+                if (lane == 0) {
+                    pack_fields(T, fb, tv);
+#pragma unroll
+                    for (int k = 0; k < nf; ++k) m.tv[k] = tv[k];
+                }
             }
-            tv[k] = t; any |= t != pr;
+            if (lane == 0) m.eq = eq;
         }
-        if (lane == 0) pack_fields(T, fb, tv);
-        __syncwarp();
-        switch (T) {
-            case 18: case 21: grid_block_warp<4, true>(c, m, lane, T, mv, tv, a.gk, gw0, u.m.cols, im); break;
-            case 19: case 29: grid_block_warp<8, false>(c, m, lane, T, mv, tv, a.gk, gw0, u.m.cols, im); break;
-            default: grid_block_warp<8, true>(c, m, lane, T, mv, tv, a.gk, gw0, u.m.cols, im);
+        __syncthreads();
+        const int eq = m.eq;
+        if (eq == 2) break;
+        const long long col0 = u.m.cols > 0 ? gw0 % u.m.cols : 0;
+        if (eq == 0) {
+            // this warp's four units, a weight per lane: search weight, sign folding with the parity repair, value over scale
+            const int un = 4 * warp + (lane >> 3), i = lane & 7, w = 32 * warp + lane;
+            const float sx2 = m.sx2[j & 1], sigma2 = (T == 16 || T == 17) ? sx2 * (1.0f / 256.f) : 2.f * sx2 * (1.0f / 256.f);
+            float gs_, gdl;
+            gscale(T, fb, m.tv, un, gs_, gdl);     // (the scale does not depend on IQ1_M's shift bit)
+            const float x = m.xs[j & 1][w];
+            float wi = sqrtf(sigma2 + x * x);
+            if (im) wi = wi * im[(gw0 + w) % u.m.cols];
+            float v = SGN ? fabsf(x) : x;
+            unsigned pnb = (__ballot_sync(0xffffffffu, x < 0.f) >> (8 * (lane >> 3))) & 255u;
+            if (SGN && par) {                      // an odd number of negatives: the least weighty one flips back
+                const float e = wi * x * x;
+                int imin = 0; float mn = __shfl_sync(0xffffffffu, e, 0, 8);
+#pragma unroll
+                for (int q = 1; q < 8; ++q) { const float o = __shfl_sync(0xffffffffu, e, q, 8); if (o < mn) { mn = o; imin = q; } }
+                if (__popc(pnb) & 1) { pnb ^= 1u << imin; if (i == imin) v = -v; }
+            }
+            m.gu[w] = v / gs_; m.gw[w] = wi;
+            if (i == 0) m.pn[un] = (unsigned char)pnb;
+            __syncwarp();
+#pragma unroll 1
+            for (int q = 0; q < 4 * ng; ++q) {
+                const int g = 4 * ng * warp + q;
+                float sc, dl;
+                gscale(T, fb, m.tv, g / ng, sc, dl);
+                if (T != 29) rank_group<N, SGN>(m, m.tab[warp], gs, N * g, dl, lane, m.top[0][g], &m.gap[0][g]);
+                else {                             // the level offset hangs on a shift bit that the chain decodes: both are ranked
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) rank_group<N, SGN>(m, m.tab[warp], gs, N * g, h ? -0.125f : 0.125f, lane, m.top[h][g], &m.gap[h][g]);
+                }
+            }
         }
-        __syncwarp();
-        for (int i = lane; i < u.bs; i += 32) fg[i] = fb[i];
+        __syncthreads();
+        if (warp > 0) {
+            fetch(j + 1, 1);
+            asm volatile("bar.sync 1, %0;" ::"n"((GW - 1) * 32) : "memory");
+            if (warp == 1 && j + 1 < u.g.nb) sum_squares(j + 1);
+        } else if (eq) {
+            for (int i = lane; i < bs; i += 32) F[b * bs + i] = pbs[i];
+        } else {
+#pragma unroll 1
+            for (int un = 0; un < 32; ++un) {
+                __syncwarp();
+                c.r.top_up();                      // a unit takes 14 symbols at most
+                const int p4 = pos4(col0 + 8 * un, u.m.cols);
+                const int rank0 = mv >= 2 ? GRANK2 + 4 * p4 : GRID_RANK;
+                const int sign0 = mv >= 2 ? GSIGN2 + 16 * p4 : GRID_SIGN;
+                int h = 0;
+                float gs_, gdl;
+                gscale(T, fb, m.tv, un, gs_, gdl);
+                if (T == 29) { h = (c.get(GRID_SHIFT) ^ get_shift(pbs, un)) != 0; gdl = h ? -0.125f : 0.125f; }
+                int tg[2] = {0, 0};
+#pragma unroll
+                for (int gg = 0; gg < ng; ++gg) {
+                    const int g = un * ng + gg;
+                    const int r = c.get(rank0 + m.gap[h][g]);
+                    int t;
+                    if (r >= TOPK) { const int lo = c.get(FESC_LO), hi = c.get(FESC_HI); t = (lo | (hi << 8)) % gs; }
+                    else if (r < GTOP) { t = m.top[h][g][r]; if (t == 0xffff) t = r; }
+                    else t = deep_rank<N, SGN>(m, gs, N * g, gdl, r, lane);
+                    tg[gg] = t;
+                }
+                unsigned neg = 0;
+                if (SGN) {
+                    // lane j works out the context of sign j; the chain then takes the contexts' tables from the lanes
+                    const int j8 = lane & 7, lev = (m.gk[ng == 2 && j8 >= 4 ? tg[1] : tg[0]] >> (B * (j8 % N))) & ((1 << B) - 1);
+                    const float m4 = fabsf(m.gu[8 * un + j8]) * 4.f;
+                    const int sctx = sign0 + (lev == 0) * 8 + (m4 < 7.f ? (int)m4 : 7);
+                    const unsigned sw = m.f01[sctx], pn = m.pn[un];
+#pragma unroll
+                    for (int q = 0; q < (par ? 7 : 8); ++q) {
+                        const int tq = __shfl_sync(0xffffffffu, sctx, q);
+                        const unsigned wq = __shfl_sync(0xffffffffu, sw, q);
+                        if (c.step(tq, wq) ^ (int)((pn >> q) & 1u)) neg |= 1u << q;
+                    }
+                }
+                if (lane < ng) m.tg[un * ng + lane] = (unsigned short)(lane ? tg[1] : tg[0]);
+                if (lane == 0) { m.neg[un] = (unsigned char)neg; m.shift[un] = (unsigned char)h; }
+                if (c.r.over()) break;
+            }
+            __syncwarp();
+            // the block's bytes, a unit per lane (lanes share bytes)
+            auto orb = [&](int i, unsigned v) { or_byte(m.fblk, i, v); };
+            if (!c.r.over()) {
+#pragma unroll
+                for (int gg = 0; gg < ng; ++gg) put_gidx(T, orb, lane * ng + gg, m.tg[lane * ng + gg]);
+                if (SGN) for (int q = 0; q < 8; ++q) if ((m.neg[lane] >> q) & 1) put_neg(T, orb, 8 * lane + q);
+                if (T == 29 && m.shift[lane]) put_shift(orb, lane);
+            }
+            __syncwarp();
+            for (int i = lane; i < bs; i += 32) F[b * bs + i] = fb[i];
+        }
+        __syncthreads();
     }
-    if (lane == 0 && !c.finished()) atomicOr(status, SG_ST_CORRUPT);
+    if (threadIdx.x == 0 && (c.r.over() || c.x != RANS_L || !c.r.at_end())) atomicOr(status, SG_ST_CORRUPT);
 }
 
 // ---- encoding in two steps ---------------------------------------------------------------------------------------
@@ -815,9 +934,18 @@ extern "C" int sg_qr_decode(int device, void* stream, int T, const unsigned char
     if (nseg == 0) return SG_OK;
     rc = use_device(device);
     if (rc != SG_OK) return rc;
-    if (qr::is_grid(T))
-        k_qr_dec_grid_warp<<<(nseg + DW_WARPS - 1) / DW_WARPS, DW_WARPS * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F,
-                                                                                                      status_word(device));
+    if (qr::is_grid(T)) {
+        auto run = [&](auto kernel) { kernel<<<nseg, GW * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F, status_word(device)); };
+        switch (T) {
+            case 16: run(k_qr_dec_grid<16>); break;
+            case 17: run(k_qr_dec_grid<17>); break;
+            case 18: run(k_qr_dec_grid<18>); break;
+            case 19: run(k_qr_dec_grid<19>); break;
+            case 21: run(k_qr_dec_grid<21>); break;
+            case 22: run(k_qr_dec_grid<22>); break;
+            default: run(k_qr_dec_grid<29>);
+        }
+    }
     else
     {
         constexpr int W = 8, per_cta = DW_WARPS * (32 / W);

@@ -355,16 +355,17 @@ SG_DEVINL int get_gidx(int T, const uchar* b, int g) {
     if (L.hi_bits) k |= ((b[L.hi_byte] >> L.hi_shift) & ((1 << L.hi_bits) - 1)) << 8;
     return k;
 }
-SG_DEVINL void put_gidx(int T, uchar* b, int g, int k) {
+// orb(i, v): OR the byte v into byte i of the block
+template <class O> SG_DEVINL void put_gidx(int T, O&& orb, int g, int k) {
     const GidxLoc L = gidx_loc(T, g);
-    if (T == 16 || T == 18) { b[L.lo_byte] |= (uchar)k; return; }
-    b[L.lo_byte] |= (uchar)(k & 255);
+    orb(L.lo_byte, (unsigned)(k & 255));
+    if (T == 16 || T == 18) return;
     if (T == 19) {
         const int v = ((k >> 8) & 7) << (3 * (g & 3));
-        b[34 + 2 * (g >> 2)] |= (uchar)(v & 255); b[35 + 2 * (g >> 2)] |= (uchar)(v >> 8);
+        orb(34 + 2 * (g >> 2), (unsigned)(v & 255)); orb(35 + 2 * (g >> 2), (unsigned)(v >> 8));
         return;
     }
-    b[L.hi_byte] |= (uchar)(((k >> 8) & ((1 << L.hi_bits) - 1)) << L.hi_shift);
+    orb(L.hi_byte, (unsigned)(((k >> 8) & ((1 << L.hi_bits) - 1)) << L.hi_shift));
 }
 // bit position (from the start of the block) of the stored sign of weight w; -1: the type stores no signs
 SG_DEVINL int sign_bit_pos(int T, int w) {
@@ -388,13 +389,13 @@ SG_DEVINL int get_neg(int T, const uchar* b, int w) {
     const int j = w & 7;
     return j < 7 ? (s7 >> j) & 1 : __popc(s7) & 1;
 }
-SG_DEVINL void put_neg(int T, uchar* b, int w) {         // parity types: only for w % 8 < 7
+template <class O> SG_DEVINL void put_neg(int T, O&& orb, int w) {         // parity types: only for w % 8 < 7
     const int p = sign_bit_pos(T, w);
-    if (p >= 0) b[p >> 3] |= (uchar)(1 << (p & 7));
+    if (p >= 0) orb(p >> 3, 1u << (p & 7));
 }
 // IQ1_M: shift bit of unit u (bit 3 or 7 of the qh byte of its pair of units)
 SG_DEVINL int get_shift(const uchar* b, int u) { return (b[32 + (u >> 1)] >> ((u & 1) ? 7 : 3)) & 1; }
-SG_DEVINL void put_shift(uchar* b, int u) { b[32 + (u >> 1)] |= (u & 1) ? 0x80 : 0x08; }
+template <class O> SG_DEVINL void put_shift(O&& orb, int u) { orb(32 + (u >> 1), (u & 1) ? 0x80u : 0x08u); }
 
 // scale of unit u and the IQ1 shift: value = s (2 l + 1), IQ1: s (l - 1 + dl).  The quantisers' fudge factors on
 // the stored fp16 are undone by multiplying with the rounded reciprocal (what the reference's GPU build does
