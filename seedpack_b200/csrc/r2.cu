@@ -47,28 +47,24 @@ SG_DEVINL void contexts(const Ctx& c, const TB& T, int orow, int j, int& pred, i
 }
 SG_DEVINL int mctx(int ex, int pred) { return clampi(8 * ex - pred - 1016 + 64, 0, 127); }
 
-// warp-aggregated histogram add: lanes hitting the same counter make one atomic
-SG_DEVINL void hadd(unsigned* counts, unsigned key) {
-    const unsigned m = __match_any_sync(__activemask(), key);
-    if ((threadIdx.x & 31) == (unsigned)(__ffs(m) - 1)) atomicAdd(counts + key, (unsigned)__popc(m));
-}
-
-// counts do not depend on the order of the weights: a warp per segment, lanes on consecutive weights (coalesced reads).
-// Exponent and sign symbols repeat inside a warp and are added once per distinct value; mantissa symbols are spread
-// over 128 x 128 counters per role, which a CTA collects in shared memory (64 KB) and adds to global memory at its end;
-// so are the exponent symbols inside a window of 128 contexts x 64 exponents around the CTA's first weight (weights
-// of one tensor keep to a few octaves; what falls outside the window goes to global memory directly).
-constexpr int R2H_WARPS = 8, R2H_SEGS = 8;         // segments per warp
-__global__ void __launch_bounds__(R2H_WARPS * 32) k_r2_hist(const unsigned char* __restrict__ dev, const TB* __restrict__ tb,
-                                                            const SG* __restrict__ sg, int nseg, Ctx c, unsigned* __restrict__ counts) {
+// Counts do not depend on the order of the weights.  A CTA takes `per` segments, as few as give two CTAs per SM their share,
+// and its 16 warps walk through a segment together (coalesced reads, four weights per lane in flight).  Bound by the shared
+// memory's atomics, three per weight.  Mantissa symbols are spread over 128 x 128 counters per role, which a CTA collects in
+// shared memory (64 KB) and adds to global memory at its end; so are the exponent symbols inside a window of 128 contexts x
+// 64 exponents around the CTA's first weight (weights of one tensor keep to a few octaves; what falls outside the window
+// goes to global memory directly).  Of the sign's 32 counters every lane has its own copy: they would collide on every step.
+constexpr int R2H_THREADS = 512, R2H_U = 4;
+constexpr int R2H_SMEM = (128 * 128 + 128 * 64 + 32 * 32) * 4;
+__global__ void __launch_bounds__(R2H_THREADS, 2) k_r2_hist(const unsigned char* __restrict__ dev, const TB* __restrict__ tb,
+                                                            const SG* __restrict__ sg, int nseg, int per, Ctx c, unsigned* __restrict__ counts) {
     extern __shared__ unsigned mhist[];            // [128 contexts][128 symbols] of the role of the CTA's first segment
     unsigned* ehist = mhist + 128 * 128;           // [128 contexts from pe0][64 exponents from ex0] of the same role
+    unsigned* shist = ehist + 128 * 64;            // [16 classes x sign][lane] of the same role
     __shared__ int win[2];
-    for (int i = threadIdx.x; i < 128 * 128 + 128 * 64; i += blockDim.x) mhist[i] = 0;
-    const int lane = threadIdx.x & 31;
-    const int first = blockIdx.x * (R2H_WARPS * R2H_SEGS);
-    const int cta_tab = first < nseg ? tb[sg[first].t].tab : -1;
-    if (threadIdx.x == 0 && first < nseg) {
+    for (int i = threadIdx.x; i < R2H_SMEM / 4; i += R2H_THREADS) mhist[i] = 0;
+    const int lane = threadIdx.x & 31, first = blockIdx.x * per;
+    const int cta_tab = tb[sg[first].t].tab;
+    if (threadIdx.x == 0) {
         const SG g = sg[first];
         const TB T = tb[g.t];
         const int rc = (int)(g.i0 / T.rowlen), j = (int)(g.i0 % T.rowlen);
@@ -79,53 +75,58 @@ __global__ void __launch_bounds__(R2H_WARPS * 32) k_r2_hist(const unsigned char*
     }
     __syncthreads();
     const int pe0 = win[0], ex0 = win[1];
-    for (int q = 0; q < R2H_SEGS; ++q) {
-        const int s = first + (threadIdx.x >> 5) * R2H_SEGS + q;
-        if (s >= nseg) break;
+    for (int s = first; s < min(nseg, first + per); ++s) {
         const SG g = sg[s];
         const TB T = tb[g.t];
         const bool local = T.tab == cta_tab;
-        // this lane's weight: compact row rc, column j; 32 weights further every turn (no division inside the loop)
-        int rc = (int)((g.i0 + lane) / T.rowlen), j = (int)((g.i0 + lane) % T.rowlen), orow = -1, have_rc = -1;
+        unsigned* gt = counts + (size_t)T.tab * 256;
+        // this lane's weight: compact row rc, column j; a CTA's width further every time (no division inside the loop)
+        const int dr = R2H_THREADS / T.rowlen, dj = R2H_THREADS % T.rowlen;
+        int rc = (int)((g.i0 + threadIdx.x) / T.rowlen), j = (int)((g.i0 + threadIdx.x) % T.rowlen);
         const unsigned short* base = reinterpret_cast<const unsigned short*>(dev + T.doff);
-        for (int k0 = 0; k0 < g.n; k0 += 32) {
-            const int k = k0 + lane;
-            const bool live = k < g.n;
-            unsigned e0 = 0xffffffffu, e2 = 0xffffffffu;
-            if (live) {
-                if (rc != have_rc) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + rc] : rc; have_rc = rc; }
-                const unsigned u = base[(size_t)orow * T.rowlen + j];
-                const int ex = (u >> 7) & 255, man = u & 127, sgn = u >> 15;
-                int pred, pe, sc; contexts(c, T, orow, j, pred, pe, sc);
-                if (local && (unsigned)(pe - pe0) < 128u && (unsigned)(ex - ex0) < 64u) atomicAdd(ehist + (pe - pe0) * 64 + (ex - ex0), 1u);
-                else e0 = (unsigned)(T.tab + pe) * 256 + ex;
-                e2 = (unsigned)(T.tab + 640 + sc) * 256 + sgn;
-                const int mc = mctx(ex, pred);
-                if (local) atomicAdd(mhist + mc * 128 + man, 1u);
-                else atomicAdd(counts + (size_t)(T.tab + 512 + mc) * 256 + man, 1u);
-                j += 32;
-                while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
+        for (int k0 = threadIdx.x; k0 < g.n; k0 += R2H_THREADS * R2H_U) {
+            unsigned u[R2H_U];
+            int pred[R2H_U], pe[R2H_U], sc[R2H_U];
+#pragma unroll
+            for (int v = 0; v < R2H_U; ++v) {
+                if (k0 + v * R2H_THREADS < g.n) {
+                    const int orow = T.rmap >= 0 ? c.rowmap[T.rmap + rc] : rc;
+                    u[v] = base[(size_t)orow * T.rowlen + j];
+                    contexts(c, T, orow, j, pred[v], pe[v], sc[v]);
+                }
+                j += dj; rc += dr;
+                if (j >= T.rowlen) { j -= T.rowlen; ++rc; }
             }
-            if (__any_sync(0xffffffffu, e0 != 0xffffffffu)) {
-                const unsigned m0 = __match_any_sync(0xffffffffu, e0);
-                if (e0 != 0xffffffffu && lane == __ffs(m0) - 1) atomicAdd(counts + e0, (unsigned)__popc(m0));
+#pragma unroll
+            for (int v = 0; v < R2H_U; ++v) {
+                if (k0 + v * R2H_THREADS >= g.n) break;
+                const int ex = (u[v] >> 7) & 255, man = u[v] & 127, sgn = u[v] >> 15, mc = mctx(ex, pred[v]);
+                if (local && (unsigned)(pe[v] - pe0) < 128u && (unsigned)(ex - ex0) < 64u) atomicAdd(ehist + (pe[v] - pe0) * 64 + (ex - ex0), 1u);
+                else atomicAdd(gt + pe[v] * 256 + ex, 1u);
+                if (local) {
+                    atomicAdd(mhist + mc * 128 + man, 1u);
+                    atomicAdd(shist + (sc[v] * 2 + sgn) * 32 + lane, 1u);
+                } else {
+                    atomicAdd(gt + (512 + mc) * 256 + man, 1u);
+                    atomicAdd(gt + (640 + sc[v]) * 256 + sgn, 1u);
+                }
             }
-            const unsigned m2 = __match_any_sync(0xffffffffu, e2);
-            if (live && lane == __ffs(m2) - 1) atomicAdd(counts + e2, (unsigned)__popc(m2));
         }
     }
     __syncthreads();
-    if (cta_tab >= 0)
-        for (int i = threadIdx.x; i < 128 * 128; i += blockDim.x) {
-            const unsigned v = mhist[i];
-            if (v) atomicAdd(counts + (size_t)(cta_tab + 512 + (i >> 7)) * 256 + (i & 127), v);
-        }
-    if (cta_tab >= 0)
-        for (int i = threadIdx.x; i < 128 * 64; i += blockDim.x) {
-            const unsigned v = ehist[i];
-            const int pe = pe0 + (i >> 6), ex = ex0 + (i & 63);
-            if (v) atomicAdd(counts + (size_t)(cta_tab + pe) * 256 + ex, v);
-        }
+    unsigned* gt = counts + (size_t)cta_tab * 256;
+    for (int i = threadIdx.x; i < 128 * 128; i += R2H_THREADS) {
+        const unsigned v = mhist[i];
+        if (v) atomicAdd(gt + (512 + (i >> 7)) * 256 + (i & 127), v);
+    }
+    for (int i = threadIdx.x; i < 128 * 64; i += R2H_THREADS) {
+        const unsigned v = ehist[i];
+        if (v) atomicAdd(gt + (pe0 + (i >> 6)) * 256 + ex0 + (i & 63), v);
+    }
+    for (int i = threadIdx.x >> 5; i < 32; i += R2H_THREADS / 32) {
+        const unsigned v = __reduce_add_sync(0xffffffffu, shist[i * 32 + lane]);
+        if (v && lane == 0) atomicAdd(gt + (640 + (i >> 1)) * 256 + (i & 1), v);
+    }
 }
 
 // Encoder.  What a weight's three symbols are coded with depends on the data only, not on the coder state, and a segment's
@@ -213,30 +214,22 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
             const int n = min(EB, g.n - (nb_max - it) * EB);
             const RansStep* row = s_e + (((it - 1) & 1) * ESEG + grp) * E_PITCH;
             int w = n - 1;
-            // two weights, six steps, at a time; a look at the slot's room every 16 weights, of 6 bytes at most each
-            for (; (w & 15) != 15; --w) {
+            // four weights, twelve steps, at a time; they take 24 bytes at most
+            for (; (w & 3) != 3; --w) {
                 if (w < 0) break;
                 rans_put(x, wr, row[3 * w]); rans_put(x, wr, row[3 * w + 1]); wr.drain();
                 rans_put(x, wr, row[3 * w + 2]); wr.drain();
                 if (wr.ptr() < slot + 64) { full = true; break; }
             }
-            for (; w >= 15 && !full; w -= 16) {
-                if (wr.ptr() < slot + 64 + 96) {                 // near the slot's start: weight by weight
-                    for (int v = 0; v < 16 && !full; ++v) {
-                        const RansStep* q = row + 3 * (w - v);
-                        rans_put(x, wr, q[0]); rans_put(x, wr, q[1]); wr.drain();
-                        rans_put(x, wr, q[2]); wr.drain();
-                        full = wr.ptr() < slot + 64;
-                    }
-                    continue;
-                }
+            for (; w >= 3 && !full; w -= 4) {
+                const RansStep* q = row + 3 * w;
 #pragma unroll
-                for (int v = 0; v < 16; v += 2) {
-                    const RansStep* q = row + 3 * (w - v);
+                for (int v = 0; v < 4; v += 2, q -= 6) {
                     rans_put(x, wr, q[0]); rans_put(x, wr, q[1]); wr.drain();
                     rans_put(x, wr, q[2]); rans_put(x, wr, q[-3]); wr.drain();
                     rans_put(x, wr, q[-2]); rans_put(x, wr, q[-1]); wr.drain();
                 }
+                full = wr.ptr() < slot + 64;
             }
         }
         __syncthreads();
@@ -253,14 +246,16 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
 
 // Decoder.  A segment is one rANS chain by format, but what a weight's symbols are decoded WITH - the exponent's and the
 // sign's tables, the prediction the mantissa's table is picked by - depends on its row and column only.  A CTA (one per SM)
-// takes up to 64 segments, as few as fill the SMs: four warps run the chains, a segment per lane, over contexts that eight
-// more warps (four lanes a segment) stage for the next 32 weights while they store the 32 weights before.
+// takes up to 64 segments, as few as fill the SMs: eight warps run the chains, a segment per lane, over contexts that eight
+// more warps (four lanes a segment) stage for the next 32 weights while they store the 32 weights before.  A chain warp and
+// its staging warp wait for each other only; few lanes to a chain warp, since one lane's walk through a bucket or top-up
+// of its ring holds up the others (four chain warps behind one barrier: 10.7 ms for 2 x 4096 x 12288 weights).
 // The chain is three table searches per weight, and what they cost is the memory the tables are in: 656 tables do not fit
 // the L1.  In shared memory are, of the role of the CTA's first segment, the 128 mantissa tables, 16 sign tables and the
 // exponent tables of 128 contexts (16 octaves) around that segment's first weight, each as the cumulated frequencies plus
 // the symbol that holds every 128th slot; anything else goes through the tables in global memory.
 constexpr int DB = 32, DSEG = 64, DG = 4, DW = DB / DG;          // weights per batch, segments per CTA, staging lanes per segment and their weights
-constexpr int D_CHAIN = 128, D_THREADS = D_CHAIN + DG * DSEG;
+constexpr int D_CHAIN = 256, D_THREADS = D_CHAIN + DG * DSEG;
 constexpr int D_ECTX = 128, D_MCTX = 128, D_MP = 256 + 260, D_EP = 256 + 516;       // bytes per table: 256 coarse, 130 / 258 cumulated
 struct DecSmem {
     unsigned ring[RING_ROWS * DSEG];
@@ -286,7 +281,7 @@ SG_DEVINL void stage_table(const uint8_t* __restrict__ ct, uint8_t* dst, int nsy
 }
 typedef RingReader<DSEG> DecRing;
 // The staged search stops at the second symbol of a bucket: a third one (rare symbols share a bucket) sets `miss`, and the
-// weight is decoded again from the tables in global memory.  So the steps have no branch.
+// weight is decoded again with a walk.  So the usual steps have no branch.
 template <int NSYM> SG_DEVINL unsigned get_staged(unsigned& x, DecRing& r, const uint8_t* t, bool& miss) {
     const unsigned short* cum = reinterpret_cast<const unsigned short*>(t + 256);
     const unsigned slot = x & ((1u << PB) - 1), xs = x >> PB;
@@ -299,6 +294,18 @@ template <int NSYM> SG_DEVINL unsigned get_staged(unsigned& x, DecRing& r, const
     x = (hi - lo) * xs + (slot - lo);
     r.renorm(x);
     return s + up;
+}
+template <int NSYM> SG_DEVINL unsigned get_walk(unsigned& x, DecRing& r, const uint8_t* t) {
+    const unsigned short* cum = reinterpret_cast<const unsigned short*>(t + 256);
+    const unsigned slot = x & ((1u << PB) - 1);
+    unsigned s = t[slot >> (PB - 8)];
+    if (NSYM < 256) s &= NSYM - 1;
+#pragma unroll 1
+    while (slot >= cum[s + 1] && s < NSYM - 1) ++s;
+    const unsigned lo = cum[s];
+    x = (cum[s + 1] - lo) * (x >> PB) + (slot - lo);
+    r.renorm(x);
+    return s;
 }
 SG_DEVINL unsigned get_global(unsigned& x, DecRing& r, const uint8_t* __restrict__ ct) {
     const unsigned* __restrict__ words = reinterpret_cast<const unsigned*>(ct + 256);
@@ -320,7 +327,8 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
     const bool chain = threadIdx.x < D_CHAIN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = blockIdx.x * per;
-    const int grp = chain ? (lane < DSEG / 4 ? 4 * lane + warp : DSEG) : (threadIdx.x - D_CHAIN) / DG, gl = threadIdx.x % DG;
+    const int pair = warp & 7, grp = chain ? (lane < DSEG / 8 ? 8 * lane + pair : DSEG) : 8 * (lane / DG) + pair, gl = lane % DG;
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); };
     const int s = first + grp;
     const bool live = grp < per && s < nseg;
     SG g; g.t = 0; g.n = 0; g.i0 = 0;
@@ -411,20 +419,26 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
                 if ((w & 3) == 0) rd.top_up();                   // four weights take 24 bytes at most
                 const unsigned e = cx[w];
                 const int pe = e & 511, sc = (e >> 9) & 15, pred = (int)e >> 16;
-                // staged: exponent and mantissa; `miss`: from the start again, through global memory
                 const unsigned x0 = x, top0 = rd.top;
                 const int pos0 = rd.pos;
-                bool miss = !staged || (unsigned)(pe - pe0) >= (unsigned)D_ECTX;
-                unsigned ex = get_staged<256>(x, rd, m.expo + (miss ? 0 : pe - pe0) * D_EP, miss);
+                const bool near = staged && (unsigned)(pe - pe0) < (unsigned)D_ECTX;
+                const uint8_t* te = m.expo + (near ? pe - pe0 : 0) * D_EP;
+                bool miss = !near;
+                unsigned ex = get_staged<256>(x, rd, te, miss);
                 unsigned man = get_staged<128>(x, rd, m.mant + mctx((int)ex, pred) * D_MP, miss);
                 unsigned f01 = m.sign[sc];
                 if (miss) {
                     x = x0; rd.top = top0; rd.pos = pos0;
-                    const uint8_t* tl = lut + (size_t)T.tab * RANS_COMPACT;
-                    ex = get_global(x, rd, tl + (size_t)pe * RANS_COMPACT);
-                    man = get_global(x, rd, tl + (size_t)(512 + mctx((int)ex, pred)) * RANS_COMPACT);
-                    const unsigned* sw = reinterpret_cast<const unsigned*>(tl + (size_t)(640 + sc) * RANS_COMPACT + 256);
-                    f01 = (sw[0] & 0xffffu) | (sw[1] << 16);
+                    if (near) {
+                        ex = get_walk<256>(x, rd, te);
+                        man = get_walk<128>(x, rd, m.mant + mctx((int)ex, pred) * D_MP);
+                    } else {
+                        const uint8_t* tl = lut + (size_t)T.tab * RANS_COMPACT;
+                        ex = get_global(x, rd, tl + (size_t)pe * RANS_COMPACT);
+                        man = get_global(x, rd, tl + (size_t)(512 + mctx((int)ex, pred)) * RANS_COMPACT);
+                        const unsigned* sw = reinterpret_cast<const unsigned*>(tl + (size_t)(640 + sc) * RANS_COMPACT + 256);
+                        f01 = (sw[0] & 0xffffu) | (sw[1] << 16);
+                    }
                 }
                 const unsigned slot = x & ((1u << PB) - 1), f0 = f01 & 0xffffu;
                 const bool neg = slot >= f0;                     // (two symbols: the second one starts where the first ends)
@@ -434,40 +448,9 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
             }
             bad = rd.over();
         }
-        __syncthreads();
+        pair_sync();
     }
     if (chain && live && (bad || rd.over() || x != RANS_L || !rd.at_end())) atomicOr(status, SG_ST_CORRUPT);
-}
-
-// 64-bit row fingerprints for duplicate-row detection (bf16v2.py:148-155): an order-dependent integer recurrence, one
-// lane per row
-__global__ void __launch_bounds__(128) k_row_hash(const unsigned short* __restrict__ w, int nrows, int rowlen, unsigned long long* __restrict__ h) {
-    // the recurrence runs along a row, one lane per row; the rows' data comes in through shared memory in tiles of
-    // 128 rows x 64 weights loaded with the lanes along the row (coalesced), read back with a 33-word row pitch
-    __shared__ unsigned tile[128][33];
-    const int r0 = blockIdx.x * 128, r = r0 + threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned long long a = 1469598103934665603ull;
-    if ((rowlen & 63) || (reinterpret_cast<uintptr_t>(w) & 3)) {           // odd shapes: straight from global memory
-        if (r < nrows) {
-            const unsigned short* p = w + (size_t)r * rowlen;
-            for (int j = 0; j < rowlen; ++j) { a ^= p[j]; a *= 1099511628211ull; a ^= a >> 29; }
-            h[r] = a;
-        }
-        return;
-    }
-    for (int c0 = 0; c0 < rowlen; c0 += 64) {
-        __syncthreads();
-        for (int rr = warp; rr < 128; rr += 4)
-            tile[rr][lane] = r0 + rr < nrows ? reinterpret_cast<const unsigned*>(w + (size_t)(r0 + rr) * rowlen + c0)[lane] : 0u;
-        __syncthreads();
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) {
-            const unsigned v = tile[threadIdx.x][i];
-            a ^= v & 0xffffu; a *= 1099511628211ull; a ^= a >> 29;
-            a ^= v >> 16;     a *= 1099511628211ull; a ^= a >> 29;
-        }
-    }
-    if (r < nrows) h[r] = a;
 }
 
 // duplicate rows copied from their source rows after decoding (bf16v2.py:475-480): pairs = (dup row, source row)
@@ -479,30 +462,93 @@ __global__ void __launch_bounds__(256) k_copy_rows(unsigned short* __restrict__ 
     for (int j = threadIdx.x; j < rowlen; j += blockDim.x) d[j] = s[j];
 }
 
-// ---- statistics ----------------------------------------------------------------------------------------------------
-// rfi[r] = rint(8 log2 rms(row r)), and rfa[r] = (float) 2^(log2 rms) used to normalise the row in the column pass.
-// One warp per row; the float64 sum of squares runs in column order (lane 0 extends the chain over staged squares).
-__global__ void __launch_bounds__(128) k_r2_rowstat(const unsigned short* __restrict__ w, int nrows, int rowlen, short* __restrict__ rfi,
-                                                    float* __restrict__ rfa) {
-    __shared__ double sq[4][256];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * 4 + warp;
-    if (r >= nrows) return;
-    const unsigned short* p = w + (size_t)r * rowlen;
-    double s = 0.0;
-    for (int c0 = 0; c0 < rowlen; c0 += 256) {
-        const int n = min(256, rowlen - c0);
-        for (int i = lane; i < n; i += 32) { const double v = (double)__uint_as_float((unsigned)p[c0 + i] << 16); sq[warp][i] = v * v; }
-        __syncwarp();
-        if (lane == 0) for (int i = 0; i < n; ++i) s = s + sq[warp][i];
-        __syncwarp();
-    }
-    if (lane == 0) {
+// ---- row recurrences: fingerprints and sums of squares --------------------------------------------------------------
+// Both run along a row, one lane per row, and the row's length is the chain.  The rows' data comes in through shared memory
+// in tiles of 32 rows x 64 weights, asked for three tiles ahead by three warps; the fourth runs the chains.  32 rows a CTA:
+// a projection's 4096 rows reach 128 SMs.
+constexpr int RC_ROWS = 32, RC_STAGES = 4, RC_PITCH = 9;          // 16-byte words per row and tile: 8, and one against bank conflicts
+// 64-bit row fingerprints for duplicate-row detection (bf16v2.py:148-155)
+struct RowHash {
+    unsigned long long* h;
+    unsigned long long a;
+    SG_DEVINL void init() { a = 1469598103934665603ull; }
+    SG_DEVINL void step(unsigned v) { a ^= v; a *= 1099511628211ull; a ^= a >> 29; }
+    SG_DEVINL void done(int r, int) { h[r] = a; }
+};
+// rfi[r] = rint(8 log2 rms(row r)), and rfa[r] = (float) 2^(log2 rms) used to normalise the row in the column pass; the
+// float64 sum of squares runs in column order
+struct RowRms {
+    short* rfi; float* rfa;
+    double s;
+    SG_DEVINL void init() { s = 0.0; }
+    SG_DEVINL void step(unsigned u) { const double v = (double)__uint_as_float(u << 16); s = s + v * v; }
+    SG_DEVINL void done(int r, int rowlen) {
         const double rf = dm::log2v(sqrt(s / (double)rowlen) + 1e-30);
         rfa[r] = (float)dm::exp2v(rf);
         rfi[r] = (short)fmin(fmax(rint(rf * 8.0), -32768.0), 32767.0);
     }
+};
+template <int CP, class Op>                                       // CP: bytes per asynchronous copy, what the rows are aligned to
+__global__ void __launch_bounds__(128) k_row_chain(const unsigned short* __restrict__ w, int nrows, int rowlen, Op op) {
+    __shared__ __align__(16) uint4 tile[RC_STAGES][RC_ROWS][RC_PITCH];
+    constexpr int PER = 128 / CP;                                 // copies per row and tile
+    const int r0 = blockIdx.x * RC_ROWS, lane = threadIdx.x & 31, ntile = (rowlen + 63) / 64;
+    auto ask = [&](int t) {
+        if (threadIdx.x >= 32 && t < ntile)
+            for (int i = threadIdx.x - 32; i < RC_ROWS * PER; i += 96) {
+                const int r = i / PER, col = t * 64 + i % PER * (CP / 2);
+                if (r0 + r < nrows && col < rowlen) {
+                    const unsigned dst = (unsigned)__cvta_generic_to_shared(reinterpret_cast<unsigned char*>(&tile[t % RC_STAGES][r][0]) + i % PER * CP);
+                    const unsigned short* src = w + (size_t)(r0 + r) * rowlen + col;
+                    if (CP == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+                    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+                }
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    op.init();
+    for (int t = 0; t < RC_STAGES - 1; ++t) ask(t);
+    for (int t = 0; t < ntile; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(RC_STAGES - 2) : "memory");
+        __syncthreads();
+        ask(t + RC_STAGES - 1);
+        if (threadIdx.x < 32 && r0 + lane < nrows) {
+            const uint4* p = tile[t % RC_STAGES][lane];
+            const int n = min(64, rowlen - t * 64);               // (even: the rows are 4-byte aligned)
+            if (n == 64) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint4 q = p[i];
+                    const unsigned v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) { op.step(v[k] & 0xffffu); op.step(v[k] >> 16); }
+                }
+            } else for (int i = 0; i < n / 2; ++i) { const unsigned v = reinterpret_cast<const unsigned*>(p)[i]; op.step(v & 0xffffu); op.step(v >> 16); }
+        }
+    }
+    if (threadIdx.x < 32 && r0 + lane < nrows) op.done(r0 + lane, rowlen);
 }
+// rows of an odd length or alignment: straight from global memory
+template <class Op>
+__global__ void __launch_bounds__(32) k_row_chain_any(const unsigned short* __restrict__ w, int nrows, int rowlen, Op op) {
+    const int r = blockIdx.x * 32 + threadIdx.x;
+    if (r >= nrows) return;
+    const unsigned short* p = w + (size_t)r * rowlen;
+    op.init();
+#pragma unroll 8
+    for (int j = 0; j < rowlen; ++j) op.step(p[j]);
+    op.done(r, rowlen);
+}
+template <class Op> static int row_chain(const void* w, int nrows, int rowlen, Op op, cudaStream_t st) {
+    const unsigned grid = (unsigned)((nrows + RC_ROWS - 1) / RC_ROWS);
+    const unsigned short* p = (const unsigned short*)w;
+    if (rowlen % 8 == 0 && (uintptr_t)w % 16 == 0) k_row_chain<16><<<grid, 128, 0, st>>>(p, nrows, rowlen, op);
+    else if (rowlen % 2 == 0 && (uintptr_t)w % 4 == 0) k_row_chain<4><<<grid, 128, 0, st>>>(p, nrows, rowlen, op);
+    else k_row_chain_any<<<grid, 32, 0, st>>>(p, nrows, rowlen, op);
+    return cuda_ok(cudaGetLastError());
+}
+
+// ---- statistics ----------------------------------------------------------------------------------------------------
 // per (row chunk, column): float64 sums of v^2 and v over the chunk's rows in row order, v = weight / rfa[row] in float32.
 // The sums are one dependent chain per column by format; what does not depend on the chain (load, the IEEE division,
 // the conversion) is done by all 256 threads of a CTA for a tile of 64 rows x 32 columns into shared memory, and the
@@ -603,13 +649,11 @@ extern "C" int sg_r2_hist(int device, void* stream, const unsigned char* dev, co
     rc = use_device(device);
     if (rc != SG_OK) return rc;
     Ctx c = {rfi, cfi, scl, rowmap};
-    {
-        rc = cuda_ok(cudaFuncSetAttribute(k_r2_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (128 * 128 + 128 * 64) * 4));
-        if (rc != SG_OK) return rc;
-        const int per_cta = R2H_WARPS * R2H_SEGS;
-        k_r2_hist<<<(nseg + per_cta - 1) / per_cta, R2H_WARPS * 32, (128 * 128 + 128 * 64) * 4, (cudaStream_t)stream>>>(dev, (const TB*)tb, (const SG*)sgp,
-                                                                                                           nseg, c, counts);
-    }
+    rc = cuda_ok(cudaFuncSetAttribute(k_r2_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, R2H_SMEM));
+    if (rc != SG_OK) return rc;
+    // clearing and adding up a CTA's counters costs about as much as a segment: at most 64 segments share it
+    const int want = (nseg + 2 * 148 - 1) / (2 * 148), per = want > 64 ? 64 : want;
+    k_r2_hist<<<(nseg + per - 1) / per, R2H_THREADS, R2H_SMEM, (cudaStream_t)stream>>>(dev, (const TB*)tb, (const SG*)sgp, nseg, per, c, counts);
     return cuda_ok(cudaGetLastError());
 }
 
@@ -655,8 +699,7 @@ extern "C" int sg_row_hash(int device, void* stream, const void* w, int nrows, i
     if (nrows == 0) return SG_OK;
     int rc = use_device(device);
     if (rc != SG_OK) return rc;
-    k_row_hash<<<(nrows + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const unsigned short*)w, nrows, rowlen, h);
-    return cuda_ok(cudaGetLastError());
+    return row_chain(w, nrows, rowlen, RowHash{h, 0}, (cudaStream_t)stream);
 }
 
 extern "C" int sg_copy_rows(int device, void* stream, void* w, int rowlen, const long long* pairs, int npairs) {
@@ -687,7 +730,8 @@ extern "C" int sg_r2_stats(int device, void* stream, const void* w, int nrows, i
     if (nchunks > 65535) return SG_ERR_LIMIT;
     float* rfa = (float*)scratch;
     double* part = (double*)((unsigned char*)scratch + ((size_t)nrows * 4 + 255) / 256 * 256);
-    k_r2_rowstat<<<(nrows + 3) / 4, 128, 0, st>>>((const unsigned short*)w, nrows, rowlen, rfi, rfa);
+    rc = row_chain(w, nrows, rowlen, RowRms{rfi, rfa, 0.0}, st);
+    if (rc != SG_OK) return rc;
     k_r2_colpart<<<dim3((rowlen + 31) / 32, nchunks), 256, 0, st>>>((const unsigned short*)w, nrows, rowlen, step, rfa, part);
     k_r2_colfinal<<<(rowlen + 255) / 256, 256, 0, st>>>(part, nchunks, nrows, rowlen, cfi, scl);
     return cuda_ok(cudaGetLastError());

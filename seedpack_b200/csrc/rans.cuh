@@ -42,8 +42,12 @@ struct ByteWriterDown {
         bits += n8;
     }
     SG_DEVINL unsigned oldest() const { return __byte_perm(__funnelshift_rc(lo, hi, 64 - bits), 0, 0x0123); }       // bits >= 32
-    SG_DEVINL void drain() {
-        if (bits >= 32) { p -= 4; *reinterpret_cast<unsigned*>(p) = oldest(); bits -= 32; }
+    SG_DEVINL void drain() {                                   // (a predicated store: a branch would end the block of independent steps)
+        const bool four = bits >= 32;
+        uint8_t* q = p - 4;
+        asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.u32 t, %0, 0;\n\t@t st.global.u32 [%1], %2;\n\t}" ::"r"((unsigned)four), "l"(q), "r"(oldest()) : "memory");
+        p = four ? q : p;
+        bits -= four ? 32 : 0;
     }
     SG_DEVINL bool bad() const { return minf == 0; }
     // bytes written so far end at this address (the lowest written byte)
@@ -157,7 +161,7 @@ struct RingReader {
 };
 
 // ---- coder steps -------------------------------------------------------------------------------------
-// The chain from state to state: two comparisons, a shift, the reciprocal's high product, a shift, one multiply-add.  What
+// The chain from state to state: a shift, the reciprocal's high product, a shift, one multiply-add, two selects.  What
 // depends on the entry alone (xm, the shift, the bias) is off it.  f = 1: the reciprocal 2^32 - 1 gives x - 1, made up
 // for in the bias.
 // Segments per warp of a kernel with one lane per segment: its time is that of one lane's chain, so a warp takes more than 8
@@ -176,12 +180,15 @@ template <int PB> SG_DEVINL RansStep rans_step_of(const RansSym e) {
 }
 template <class W>
 SG_DEVINL void rans_put(unsigned& x, W& w, const RansStep t) {
-    // x < 2^31 and xm >= 2^(31 - PB) for f >= 1: at most two bytes leave per symbol (PB <= 15)
-    const int n8 = (x >> 8) >= t.xm ? 16 : x >= t.xm ? 8 : 0;
-    w.push(x, n8);
-    x >>= n8;
-    const unsigned q = __umulhi(x, t.rcp) >> (t.sh_comp & 31u);
-    x = q * (t.sh_comp >> 5) + (x + t.bias);
+    // x < 2^31 and xm >= 2^(31 - PB) for f >= 1: at most two bytes leave per symbol (PB <= 15).  The step is worked out for no,
+    // one and two bytes side by side and chosen at the end, so that the comparisons are not on the chain
+    const unsigned y1 = x >> 8, y2 = x >> 16, sh = t.sh_comp & 31u, comp = t.sh_comp >> 5;
+    const bool one = x >= t.xm, two = y1 >= t.xm;
+    const unsigned r0 = (__umulhi(x, t.rcp) >> sh) * comp + (x + t.bias);
+    const unsigned r1 = (__umulhi(y1, t.rcp) >> sh) * comp + (y1 + t.bias);
+    const unsigned r2 = (__umulhi(y2, t.rcp) >> sh) * comp + (y2 + t.bias);
+    w.push(x, two ? 16 : one ? 8 : 0);
+    x = two ? r2 : one ? r1 : r0;
 }
 // one symbol, or two with one look at the pending bytes
 template <int PB, class W>

@@ -113,3 +113,37 @@ def test_base_codec_round_trip(rows, cols, spread):
     bits = ctypes.c_int(0)
     _lib.check(L.sg_status_fetch(torch.cuda.current_device(), st, ctypes.byref(bits)), "sg_status_fetch")
     assert bits.value == 0 and torch.equal(back, w)
+
+
+@pytest.mark.parametrize("rows,cols,off", [(1, 1, 0), (33, 64, 0), (31, 72, 0), (40, 130, 0), (5, 1001, 0), (32, 256, 2), (7, 256, 1)])
+def test_row_recurrences(rows, cols, off):
+    """row fingerprints and row statistics against the recurrences in Python (integers; float64 sums in order), for rows whose
+    length and address allow 16-byte copies, 4-byte copies and none"""
+    import ctypes
+
+    import torch
+    from seedpack_b200 import _lib
+    L = _lib.lib()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    rng = np.random.default_rng(rows * cols)
+    w32 = (rng.standard_normal((rows, cols)) * 0.02).astype(np.float32)
+    bits = (w32.view(np.uint32) >> 16).astype(np.uint16)
+    buf = torch.zeros(off + rows * cols + 8, dtype=torch.int16, device="cuda")
+    w = buf[off:off + rows * cols]
+    w.copy_(torch.from_numpy(bits.view(np.int16).reshape(-1)))
+    h = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    _lib.check(L.sg_row_hash(0, st, p(w), rows, cols, p(h)), "sg_row_hash")
+    rfi, cfi = torch.zeros(rows, dtype=torch.int16, device="cuda"), torch.zeros(cols, dtype=torch.int16, device="cuda")
+    scl, scratch = torch.zeros(cols, dtype=torch.int8, device="cuda"), torch.zeros(L.sg_r2_stats_scratch_bytes(rows, cols), dtype=torch.uint8, device="cuda")
+    _lib.check(L.sg_r2_stats(0, st, p(w), rows, cols, p(rfi), p(cfi), p(scl), p(scratch), scratch.numel()), "sg_r2_stats")
+    for r in range(rows):
+        a, s = 1469598103934665603, 0.0
+        for v in bits[r].tolist():
+            a = ((a ^ v) * 1099511628211) & (2 ** 64 - 1)
+            a ^= a >> 29
+        for v in (bits[r].astype(np.uint32) << 16).view(np.float32).astype(np.float64).tolist():
+            s += v * v
+        assert int(h[r]) & (2 ** 64 - 1) == a
+        lg = 8 * np.log2(np.sqrt(s / cols) + 1e-30)
+        assert abs(int(rfi[r]) - lg) <= 0.5 + 1e-9            # round to nearest; log2 to well below 1e-9
