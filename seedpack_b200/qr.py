@@ -8,6 +8,7 @@ the slot-doubling retry (qr.py:1043-1053).  Arrays are torch CUDA tensors (or ho
 """
 import ctypes
 import struct
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import torch
@@ -327,9 +328,11 @@ class QRCodec:
         return lens_h.astype(np.uint32), stream
 
     @staticmethod
-    def finish(freq, used, lens, stream, mv=MODEL):
-        """the batch as the archive holds it (seedpack/qr.py:1058-1061): tables, segment lengths, streams, model byte"""
-        out = {"t": store_tables(freq, used), "l": zstd.compress(np.asarray(lens, np.uint32).tobytes(), 19), "s": bytes(stream)}
+    def finish(freq, used, lens, stream, mv=MODEL, tables=None):
+        """the batch as the archive holds it (seedpack/qr.py:1058-1061): tables, segment lengths, streams, model byte;
+        `tables`: a future of store_tables(freq, used) where the caller has one"""
+        packed_lens = zstd.compress(np.asarray(lens, np.uint32).tobytes(), 19)
+        out = {"t": store_tables(freq, used) if tables is None else tables.result(), "l": packed_lens, "s": bytes(stream)}
         if mv != 1:
             out["v"] = bytes([mv])
         return pack(out)
@@ -339,8 +342,11 @@ class QRCodec:
         offset])] of one batch, all of ggml type T -> bytes of the coded batch (seedpack/qr.py:1007-1061)"""
         state, counts = self.hist(T, items, seed_dev, imx_dev, mv)
         freq, used = normalize(counts)
-        lens, stream = self.code(state, freq, used)
-        return self.finish(freq, used, lens, stream, state["mv"])
+        # compressing the tables (some 7 ms at level 19, and the library call leaves the interpreter free) beside the coder
+        with ThreadPoolExecutor(1) as pool:
+            tables = pool.submit(store_tables, freq, used)
+            lens, stream = self.code(state, freq, used)
+            return self.finish(freq, used, lens, stream, state["mv"], tables)
 
     def decode(self, T, buf, items, seed_dev, imx_dev=None):
         """items: [(predicted bytes, seed byte offset, seed type[, weights per row, imatrix offset])] -> device uint8

@@ -1,8 +1,8 @@
 """Segment-parallel rANS codec over a symbol stream with per-block context tables - host side.
 
 Mirrors the framing of the reference's QR batches (seedpack/qr.py:1007-1090): histogram on the device, table
-normalisation on the host (`normalize`, copied from seedpack/qr.py:904-923 - fifteen lines of host NumPy whose every
-tie-break decides archive bytes; with the reference bound through seedpack_b200.refbind its own copy runs), encode into per-segment slots with the doubling retry of seedpack/qr.py:1043-1053, prefix sum +
+normalisation on the host (`normalize`, as seedpack/qr.py:904-923 does it: every tie-break decides archive bytes; with the
+reference bound through seedpack_b200.refbind its own copy runs), encode into per-segment slots with the doubling retry of seedpack/qr.py:1043-1053, prefix sum +
 gather, and the inverse.  All coding runs in libseedgrow.so; there is no CPU coder here.
 """
 import ctypes
@@ -19,22 +19,25 @@ SEG = 16384          # symbols per segment (seedpack/qr.py:952-954: max(16, 1638
 def normalize(counts, scale=1 << PB):
     """counts (T, 256) int -> (uint16 freqs of the used rows, used row ids): every row sums to `scale`, every
     seen symbol keeps at least 1; the rounding deficit / surplus goes to the largest entry (first maximum).
-    Copied from the reference (seedpack/qr.py:904-923) with NumPy arrays in and out: the format is defined by it."""
+    Same result as the reference's row loop (seedpack/qr.py:904-923), whose tie-breaks define the format, for all rows at
+    once; a row whose largest entry cannot give all of its surplus goes on by itself."""
     c = np.asarray(counts).astype(np.int64).reshape(-1, 256)
     tot = c.sum(1)
     used = np.flatnonzero(tot)
-    f = np.zeros((len(used), 256), np.int64)
-    for k, r in enumerate(used):
-        row = c[r]
-        fr = np.where(row > 0, np.maximum(1, row * scale // tot[r]), 0)
-        diff = scale - int(fr.sum())
-        while diff != 0:
-            j = int(np.argmax(fr))
-            step = diff if diff > 0 else -min(-diff, int(fr[j]) - 1)
-            if step == 0:
-                j = int(np.flatnonzero(fr > 1)[0]); step = -1
-            fr[j] += step; diff -= step
-        f[k] = fr
+    c, tot = c[used], tot[used, None]
+    f = np.where(c > 0, np.maximum(1, c * scale // tot), 0)
+    at = np.arange(len(used))
+    diff, top = scale - f.sum(1), f.argmax(1)
+    step = np.maximum(diff, 1 - f[at, top])
+    f[at, top] += step
+    for k in np.flatnonzero(diff != step):
+        row, d = f[k], int(diff[k] - step[k])
+        while d != 0:                                 # d < 0
+            j = int(np.argmax(row))
+            s = -min(-d, int(row[j]) - 1)
+            if s == 0:
+                j = int(np.flatnonzero(row > 1)[0]); s = -1
+            row[j] += s; d -= s
     return f.astype(np.uint16), used.astype(np.int32)
 
 

@@ -52,3 +52,38 @@ def test_port_decode_flags_truncation():
     off2 = off.copy(); off2[-1] -= 3
     _, rc = orans.decode(stream, off2, G[f"{name}_block_tab"], BL, len(G[f"{name}_sym"]), SEG, _full(name))
     assert rc == 1
+
+
+def test_normalize_equals_the_row_loop():
+    """all rows at once against the row-by-row definition of the format: deficits, surpluses that one entry cannot give,
+    ties for the largest entry, single symbols, unused rows"""
+    from seedpack_b200.rans import normalize
+
+    def loop(c, scale):
+        f = np.zeros_like(c)
+        for k, row in enumerate(c):
+            fr = np.where(row > 0, np.maximum(1, row * scale // row.sum()), 0)
+            diff = scale - int(fr.sum())
+            while diff != 0:
+                j = int(np.argmax(fr))
+                step = diff if diff > 0 else -min(-diff, int(fr[j]) - 1)
+                if step == 0:
+                    j = int(np.flatnonzero(fr > 1)[0]); step = -1
+                fr[j] += step; diff -= step
+            f[k] = fr
+        return f
+
+    rng = np.random.default_rng(0)
+    rows = [np.zeros(256, np.int64) for _ in range(4)]
+    rows[1][7] = 1
+    rows[2][:] = 1
+    rows[3][:] = 1; rows[3][9] = 10 ** 9                         # 255 symbols of frequency 1, all surplus from one entry
+    for _ in range(300):
+        c = rng.integers(0, 2 ** rng.integers(1, 40, 256)) * (rng.random(256) < rng.random())
+        c[rng.integers(0, 256)] += 1
+        rows.append(c.astype(np.int64))
+    c = np.stack(rows)
+    for scale in (1 << 8, 1 << 12, 1 << 14, 1 << 15):            # (at 2^8 with 256 symbols every frequency ends at 1)
+        f, used = normalize(c, scale)
+        assert used.tolist() == [k for k in range(len(c)) if c[k].any()] and f.dtype == np.uint16
+        assert np.array_equal(f, loop(c[used], scale))
