@@ -144,16 +144,15 @@ SG_DEVINL int qkx_cand_code(float iscale, float mn, int nmax, float xi) {
     return clampi(nearest_int(v), 0, nmax);
 }
 
-// the same code as a float.  V3: the value that goes into nearest_int lies in (0, nmax], where the rounding add of
-// nearest_int yields the integer's float directly (v + 1.5 * 2^23 - 1.5 * 2^23), with no integer detour.
+// the same code as a float, without a conversion (a quarter of the lanes' rate).  V3: the value that goes into nearest_int
+// lies in [0, nmax], where the rounding add of nearest_int yields the integer's float directly (v + 1.5 * 2^23 - 1.5 * 2^23);
+// v <= 0 and NaN give 0.  Else, for any v: the clamp works on the mantissa that nearest_int reads, the integer plus 2^22.
 template <int N, bool V3>
 SG_DEVINL float qkx_cand_level(float iscale, float mn, int nmax, float xi) {
-    if (V3) {
-        const float v = fmul(iscale, fsub(xi, mn));
-        const float r = fsub(fadd(fminf(v, (float)nmax), 12582912.f), 12582912.f);
-        return v > 0.f ? r : 0.f;
-    }
-    return (float)qkx_cand_code<N, V3>(iscale, mn, nmax, xi);
+    const float v = fmul(iscale, fsub(xi, mn));
+    if (V3) return fsub(fadd(fminf(fmaxf(v, 0.f), (float)nmax), 12582912.f), 12582912.f);
+    const int m = clampi(__float_as_int(fadd(v, 12582912.f)) & 0x007fffff, 0x00400000, 0x00400000 + nmax);
+    return fsub(__int_as_float(0x4b000000 | m), 12582912.f);
 }
 
 template <int N, bool V3>
