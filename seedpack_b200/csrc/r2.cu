@@ -488,7 +488,7 @@ struct RowRms {
         rfi[r] = (short)fmin(fmax(rint(rf * 8.0), -32768.0), 32767.0);
     }
 };
-template <int CP, class Op>                                       // CP: bytes per asynchronous copy, what the rows are aligned to
+template <int CP, class Op>                                       // CP: bytes per copy, what the rows are aligned to (2: plain loads)
 __global__ void __launch_bounds__(128) k_row_chain(const unsigned short* __restrict__ w, int nrows, int rowlen, Op op) {
     __shared__ __align__(16) uint4 tile[RC_STAGES][RC_ROWS][RC_PITCH];
     constexpr int PER = 128 / CP;                                 // copies per row and tile
@@ -500,7 +500,8 @@ __global__ void __launch_bounds__(128) k_row_chain(const unsigned short* __restr
                 if (r0 + r < nrows && col < rowlen) {
                     const unsigned dst = (unsigned)__cvta_generic_to_shared(reinterpret_cast<unsigned char*>(&tile[t % RC_STAGES][r][0]) + i % PER * CP);
                     const unsigned short* src = w + (size_t)(r0 + r) * rowlen + col;
-                    if (CP == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+                    if (CP == 2) reinterpret_cast<unsigned short*>(&tile[t % RC_STAGES][r][0])[i % PER] = *src;
+                    else if (CP == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
                     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
                 }
             }
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(128) k_row_chain(const unsigned short* __restr
         ask(t + RC_STAGES - 1);
         if (threadIdx.x < 32 && r0 + lane < nrows) {
             const uint4* p = tile[t % RC_STAGES][lane];
-            const int n = min(64, rowlen - t * 64);               // (even: the rows are 4-byte aligned)
+            const int n = min(64, rowlen - t * 64);
             if (n == 64) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -523,28 +524,17 @@ __global__ void __launch_bounds__(128) k_row_chain(const unsigned short* __restr
 #pragma unroll
                     for (int k = 0; k < 4; ++k) { op.step(v[k] & 0xffffu); op.step(v[k] >> 16); }
                 }
-            } else for (int i = 0; i < n / 2; ++i) { const unsigned v = reinterpret_cast<const unsigned*>(p)[i]; op.step(v & 0xffffu); op.step(v >> 16); }
+            } else for (int i = 0; i < n; ++i) op.step(reinterpret_cast<const unsigned short*>(p)[i]);
         }
     }
     if (threadIdx.x < 32 && r0 + lane < nrows) op.done(r0 + lane, rowlen);
-}
-// rows of an odd length or alignment: straight from global memory
-template <class Op>
-__global__ void __launch_bounds__(32) k_row_chain_any(const unsigned short* __restrict__ w, int nrows, int rowlen, Op op) {
-    const int r = blockIdx.x * 32 + threadIdx.x;
-    if (r >= nrows) return;
-    const unsigned short* p = w + (size_t)r * rowlen;
-    op.init();
-#pragma unroll 8
-    for (int j = 0; j < rowlen; ++j) op.step(p[j]);
-    op.done(r, rowlen);
 }
 template <class Op> static int row_chain(const void* w, int nrows, int rowlen, Op op, cudaStream_t st) {
     const unsigned grid = (unsigned)((nrows + RC_ROWS - 1) / RC_ROWS);
     const unsigned short* p = (const unsigned short*)w;
     if (rowlen % 8 == 0 && (uintptr_t)w % 16 == 0) k_row_chain<16><<<grid, 128, 0, st>>>(p, nrows, rowlen, op);
     else if (rowlen % 2 == 0 && (uintptr_t)w % 4 == 0) k_row_chain<4><<<grid, 128, 0, st>>>(p, nrows, rowlen, op);
-    else k_row_chain_any<<<grid, 32, 0, st>>>(p, nrows, rowlen, op);
+    else k_row_chain<2><<<grid, 128, 0, st>>>(p, nrows, rowlen, op);
     return cuda_ok(cudaGetLastError());
 }
 
