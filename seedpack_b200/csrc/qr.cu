@@ -267,55 +267,35 @@ __global__ void __launch_bounds__(QR_TPB) k_qr_enc(const Args a, const RansSym* 
 // are decoded first.  So the warp decodes flag and fields in lockstep (every lane runs the same chain on the same
 // bytes, which costs what one lane would), then its lanes work out contexts and predictions of the block's weights
 // side by side into shared memory, the chain runs over the staged contexts, and the lanes put the codes together.
-// Table lookups for symbol 0 (by far the most frequent: cum = 0, freq from a small table in shared memory) stay off
-// global memory.
+// Table lookups for the symbols 0 and 1 (by far the most frequent) stay off global memory.
 constexpr int DW_WARPS = 4;
 struct __align__(8) DecWarpSmem {
+    unsigned ring[RING_ROWS + 1];           // (a word more: the arrays below are read eight bytes at a time)
     unsigned fblk[56], pblk[56];            // the block being rebuilt / its prediction (block sizes <= 210 bytes)
     unsigned short ctx[256];
     short pred[256];
     signed char sgn[256];
     uchar sym[256];
 };
-// the decoder's state and byte source: bytes come through a 64-bit register refilled every 8 bytes, reads past the
-// end give zeros and set `over`
-struct WarpDec {
-    unsigned x;
-    unsigned long long buf; int nbuf;
-    const uchar* p; const uchar* end; bool over;
-    const RansSym* enc; const uchar* lut; const unsigned short* f0;
-    SG_DEVINL void fill() {
-        buf = 0;
-        const long long left = end - p;
-        if (left <= 0) { over = true; nbuf = 8; return; }
-        const int n = left < 8 ? (int)left : 8;
-        for (int i = 0; i < n; ++i) buf |= (unsigned long long)p[i] << (56 - 8 * i);
-        p += n; nbuf = n;
-    }
-    SG_DEVINL unsigned byte() {
-        if (nbuf == 0) fill();
-        const unsigned b = (unsigned)(buf >> 56);
-        buf <<= 8; --nbuf;
-        return b;
-    }
-    SG_DEVINL void init(const uchar* b, const uchar* e) {
-        p = b; end = e; over = false; nbuf = 0; buf = 0; x = 0;
-        for (int i = 0; i < 4; ++i) x = (x << 8) | byte();
-    }
-    SG_DEVINL bool finished() const { return !over && x == RANS_L && p - nbuf == end; }
-    SG_DEVINL int get(int tab) {
-        const unsigned slot = x & 4095u, f = f0[tab];
-        int s = 0;
-        if (slot < f) x = f * (x >> 12) + slot;                  // symbol 0: cum = 0
-        else {
+// a segment's decoder, run by several lanes in lockstep over one ring
+struct QrDec {
+    unsigned x; RingReader<1> r; const RansSym* enc; const uchar* lut; const unsigned* f01;
+    // w = f01[tab].  Symbols 0 and 1 without a load
+    SG_DEVINL int step(int tab, unsigned w) {
+        const unsigned slot = x & 4095u, f0 = w & 0xffffu, f1 = w >> 16;
+        const bool one = slot >= f0;
+        int s = one;
+        unsigned f = one ? f1 : f0, d = one ? slot - f0 : slot;
+        if (slot >= f0 + f1) {
             s = lut[((size_t)tab << 12) + slot];
             const unsigned fc = enc[tab * 256 + s].fc;
-            x = (fc & 0xffffu) * (x >> 12) + slot - (fc >> 16);
+            f = fc & 0xffffu; d = slot - (fc >> 16);
         }
-#pragma unroll 1
-        for (int guard = 0; guard < 4 && x < RANS_L; ++guard) x = (x << 8) | byte();
+        x = f * (x >> 12) + d;
+        r.renorm(x);
         return s;
     }
+    SG_DEVINL int get(int tab) { return step(tab, f01[tab]); }
 };
 SG_DEVINL void or_byte(unsigned* blk, int i, unsigned v) { atomicOr(blk + (i >> 2), (v & 255u) << (8 * (i & 3))); }
 // put_code with the bits OR-ed into a zeroed block in shared memory, safe for lanes that share a byte
@@ -333,43 +313,47 @@ SG_DEVINL void put_code_shared(int T, unsigned* blk, int w, int q) {
 // small W wastes fewer issue slots on the lockstep parts, a large W spreads the per-weight work wider.  The warp's
 // control flow is kept uniform (every segment of the warp is at its j-th block; segments whose block equals its
 // prediction, or that have ended, sit the phases out), so the lane groups stay converged.
-template <int W>
+template <int T, int W>
 __global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
                                                                const RansSym* __restrict__ enc, const uchar* __restrict__ lut,
                                                                uchar* __restrict__ F, int* __restrict__ status) {
     constexpr int SPW = 32 / W;
-    __shared__ unsigned short f0[NTAB2];
+    constexpr int qk = qk_of(T), bs = bs_of(T), nf = nfield(T), sublen = sublen_of(T);
+    __shared__ unsigned f01[NTAB2];
     __shared__ DecWarpSmem wsm[DW_WARPS * SPW];
-    for (int t = threadIdx.x; t < NTAB2; t += blockDim.x) f0[t] = (unsigned short)(enc[t * 256].fc & 0xffffu);
+    for (int t = threadIdx.x; t < NTAB2; t += blockDim.x) f01[t] = (enc[t * 256].fc & 0xffffu) | (enc[t * 256 + 1].fc << 16);
     __syncthreads();
     const int lane = threadIdx.x & 31, sub = lane % W, grp = (threadIdx.x >> 5) * SPW + lane / W;
     const int s = blockIdx.x * (DW_WARPS * SPW) + grp;
     const bool have = s < a.nseg;
     DecWarpSmem& m = wsm[grp];
-    const int T = a.T, mv = a.mv;
+    const int mv = a.mv;
+    const unsigned group = (W == 32 ? 0xffffffffu : (1u << (W & 31)) - 1u) << (lane / W * W);
     const Setup u = setup(T, a.seed, a.tm, a.sg, have ? s : a.nseg - 1);
-    WarpDec c; c.enc = enc; c.lut = lut; c.f0 = f0;
-    if (have) c.init(in + off[s], in + off[s + 1]);
-    else { c.init(in, in); c.x = RANS_L; c.over = false; }
+    QrDec c; c.enc = enc; c.lut = lut; c.f01 = f01;
+    if (have) { c.r.init(in + off[s], in + off[s + 1], m.ring); c.x = c.r.state(); }
+    else { c.r.init(in, in, m.ring); c.x = RANS_L; }
+    // (the ring is one for the segment's lanes: none runs ahead into a top-up)
+    auto top_up = [&]() { __syncwarp(group); c.r.top_up(); };
     uchar* fb = reinterpret_cast<uchar*>(m.fblk);
     const uchar* pbs = reinterpret_cast<const uchar*>(m.pblk);
     const int nb = have ? u.g.nb : 0;
     const int nbmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)nb);
     int prev = 1;
     for (int j = 0; j < nbmax; ++j) {
-        const bool live = j < nb && !c.over;
+        const bool live = j < nb && !c.r.over();
         const long long b = u.g.b0 + j;
-        const uchar* pg = a.P + b * u.bs;
-        uchar* fg = F + b * u.bs;
+        const uchar* pg = a.P + b * bs;
+        uchar* fg = F + b * bs;
         int eq = 1;
-        if (live) { eq = c.get(FLAG + prev); prev = eq; }
-        if (live && eq) for (int i = sub; i < u.bs; i += W) fg[i] = pg[i];
+        if (live) { top_up(); eq = c.get(FLAG + prev); prev = eq; }
+        if (live && eq) for (int i = sub; i < bs; i += W) fg[i] = pg[i];
         const bool code = live && !eq;
         if (!__any_sync(0xffffffffu, code)) continue;
         __syncwarp();
         if (code) {
             for (int i = sub; i < 56; i += W) m.fblk[i] = 0;
-            for (int i = sub; i < u.bs; i += W) reinterpret_cast<uchar*>(m.pblk)[i] = pg[i];
+            for (int i = sub; i < bs; i += W) reinterpret_cast<uchar*>(m.pblk)[i] = pg[i];
         }
         __syncwarp();
         int tv[MAXF];
@@ -377,7 +361,9 @@ __global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, con
             int pv[MAXF];
             unpack_fields(T, pbs, pv);
             int any = 0;
-            for (int k = 0; k < u.nf; ++k) {
+#pragma unroll
+            for (int k = 0; k < nf; ++k) {
+                if ((k & 3) == 0) top_up();
                 const int kd = fkind(T, k);
                 const int pr = fpred(T, mv, pv, k, k > 0 ? tv[0] : 0, k > 1 ? tv[1] : 0);
                 const int sym = c.get(fctx(kd, any));
@@ -392,11 +378,11 @@ __global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, con
             }
             if (sub == 0) pack_fields(T, fb, tv);
             // contexts and predictions of the block's weights, side by side
-            const long long gw0 = (b - u.m.blk0) * u.qk;
+            const long long gw0 = (b - u.m.blk0) * qk;
             const long long col0 = u.m.cols > 0 ? gw0 % u.m.cols : 0;
             int tsub = -1; float ta = 0.f, tc = 0.f;
-            for (int w = sub; w < u.qk; w += W) {
-                if (w / u.sublen != tsub) { tsub = w / u.sublen; wscale(T, tv, tsub, ta, tc); }
+            for (int w = sub; w < qk; w += W) {
+                if (w / sublen != tsub) { tsub = w / sublen; wscale(T, tv, tsub, ta, tc); }
                 float xv, hv; seed_val(u.m.seed_type, u.sbase, gw0 + w, xv, hv, u.m.cols);
                 int r, sgn, ctx; predict_code(T, ta, tc, pbs, w, xv, hv, u.hboff, r, sgn, ctx, mv, pos8(col0 + w, u.m.cols));
                 m.ctx[w] = (unsigned short)ctx; m.pred[w] = (short)r; m.sgn[w] = (signed char)sgn;
@@ -405,7 +391,8 @@ __global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, con
         __syncwarp();
         if (code) {
 #pragma unroll 1
-            for (int w = 0; w < u.qk; w += 4) {          // four contexts per load, four symbols per store
+            for (int w = 0; w < qk; w += 4) {          // four contexts per load, four symbols per store
+                if ((w & 15) == 0) top_up();
                 const uint2 cx = *reinterpret_cast<const uint2*>(m.ctx + w);
                 unsigned sy = (unsigned)c.get((int)(cx.x & 0xffffu));
                 sy |= (unsigned)c.get((int)(cx.x >> 16)) << 8;
@@ -416,16 +403,16 @@ __global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, con
         }
         __syncwarp();
         if (code) {
-            for (int w = sub; w < u.qk; w += W) {
+            for (int w = sub; w < qk; w += W) {
                 int q = m.pred[w] + m.sgn[w] * (int)(signed char)m.sym[w];
                 if (T == 8) q = (int)(signed char)(q & 255);
                 put_code_shared(T, m.fblk, w, q);
             }
         }
         __syncwarp();
-        if (code) for (int i = sub; i < u.bs; i += W) fg[i] = fb[i];
+        if (code) for (int i = sub; i < bs; i += W) fg[i] = fb[i];
     }
-    if (have && sub == 0 && !c.finished()) atomicOr(status, SG_ST_CORRUPT);
+    if (have && sub == 0 && (c.r.over() || c.x != RANS_L || !c.r.at_end())) atomicOr(status, SG_ST_CORRUPT);
 }
 
 // ---- decoder of the lattice types: a CTA per segment -------------------------------------------------------------------
@@ -453,25 +440,6 @@ struct GridSmem {
     unsigned short tg[64];
     int tv[MAXF];
     int eq;
-};
-struct GridDec {
-    unsigned x; RingReader<1> r; const RansSym* enc; const uchar* lut; const unsigned* f01;
-    // w = f01[tab].  Symbols 0 and 1 without a load
-    SG_DEVINL int step(int tab, unsigned w) {
-        const unsigned slot = x & 4095u, f0 = w & 0xffffu, f1 = w >> 16;
-        const bool one = slot >= f0;
-        int s = one;
-        unsigned f = one ? f1 : f0, d = one ? slot - f0 : slot;
-        if (slot >= f0 + f1) {
-            s = lut[((size_t)tab << 12) + slot];
-            const unsigned fc = enc[tab * 256 + s].fc;
-            f = fc & 0xffffu; d = slot - (fc >> 16);
-        }
-        x = f * (x >> 12) + d;
-        r.renorm(x);
-        return s;
-    }
-    SG_DEVINL int get(int tab) { return step(tab, f01[tab]); }
 };
 template <int N> SG_DEVINL float point_dist_w(const float* tab, unsigned key) {
     constexpr int B = N == 8 ? 2 : 3, E = 1 << (2 * B);
@@ -596,7 +564,7 @@ __global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uch
     fetch(0, 0);
     __syncthreads();
     if (warp == 1) sum_squares(0);
-    GridDec c; c.enc = enc; c.lut = lut; c.f01 = m.f01;
+    QrDec c; c.enc = enc; c.lut = lut; c.f01 = m.f01;
     int prev = 1;
     if (warp == 0) { c.r.init(in + off[s], in + off[s + 1], m.ring); c.x = c.r.state(); }
     uchar* fb = reinterpret_cast<uchar*>(m.fblk);
@@ -949,8 +917,25 @@ extern "C" int sg_qr_decode(int device, void* stream, int T, const unsigned char
     else
     {
         constexpr int W = 8, per_cta = DW_WARPS * (32 / W);
-        k_qr_dec_warp<W><<<(nseg + per_cta - 1) / per_cta, DW_WARPS * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F,
-                                                                                                  status_word(device));
+        auto run = [&](auto kernel) {
+            kernel<<<(nseg + per_cta - 1) / per_cta, DW_WARPS * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F, status_word(device));
+        };
+        switch (T) {
+            case 2: run(k_qr_dec_warp<2, W>); break;
+            case 3: run(k_qr_dec_warp<3, W>); break;
+            case 6: run(k_qr_dec_warp<6, W>); break;
+            case 7: run(k_qr_dec_warp<7, W>); break;
+            case 8: run(k_qr_dec_warp<8, W>); break;
+            case 10: run(k_qr_dec_warp<10, W>); break;
+            case 11: run(k_qr_dec_warp<11, W>); break;
+            case 12: run(k_qr_dec_warp<12, W>); break;
+            case 13: run(k_qr_dec_warp<13, W>); break;
+            case 14: run(k_qr_dec_warp<14, W>); break;
+            case 20: run(k_qr_dec_warp<20, W>); break;
+            case 23: run(k_qr_dec_warp<23, W>); break;
+            case 42: run(k_qr_dec_warp<42, W>); break;
+            default: return SG_ERR_TYPE;
+        }
     }
     return cuda_ok(cudaGetLastError());
 }
