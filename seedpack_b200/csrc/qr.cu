@@ -464,8 +464,9 @@ template <int N, bool SGN> SG_DEVINL void group_tables(float* tab, const GridSme
 SG_DEVINL unsigned ordered_bits(float d) { const unsigned u = __float_as_uint(d); return u ^ ((unsigned)((int)u >> 31) | 0x80000000u); }
 
 // Closest GTOP points of one group in the order (distance, index), and its gap context.  Every lane keeps the closest of
-// its own points (lane, lane + 32, ...; met in index order, so that on equal distances the earlier one stays ahead);
-// the warp's next one is then an arg-min over the lanes' lists.  Points at infinite distance never come up.
+// its own points (lane, lane + 32, ...; met in index order): a point goes in before the first one that is further away, so
+// after its equals, and what stands there moves down one place, whatever the distances.  The warp's next one is then an
+// arg-min over the lanes' lists.  Points at infinite distance never come up.
 template <int N, bool SGN> SG_DEVINL void rank_group(GridSmem& m, float* tab, int gs, int w0, float gdl, int lane, unsigned short* top, unsigned char* gap) {
     const float inf = __int_as_float(0x7f800000);
     __syncwarp();
@@ -478,12 +479,13 @@ template <int N, bool SGN> SG_DEVINL void rank_group(GridSmem& m, float* tab, in
     for (int k0 = 0; k0 < gs; k0 += 32) {
         float d = point_dist_w<N>(tab, m.gk[k0 + lane]);
         int k = k0 + lane;
+        bool in = false;                           // from here on d, k are the one that was moved out of the place before
 #pragma unroll
         for (int l = 0; l < GTOP; ++l) {
-            const bool lt = d < D[l];
+            in = in || d < D[l];
             const float dm = D[l]; const int km = K[l];
-            D[l] = lt ? d : dm; K[l] = lt ? k : km;
-            d = lt ? dm : d; k = lt ? km : k;
+            D[l] = in ? d : dm; K[l] = in ? k : km;
+            d = in ? dm : d; k = in ? km : k;
         }
     }
     float d1 = inf, d2 = inf;

@@ -147,3 +147,31 @@ def test_row_recurrences(rows, cols, off):
         assert int(h[r]) & (2 ** 64 - 1) == a
         lg = 8 * np.log2(np.sqrt(s / cols) + 1e-30)
         assert abs(int(rfi[r]) - lg) <= 0.5 + 1e-9            # round to nearest; log2 to well below 1e-9
+
+
+@pytest.mark.parametrize("t", [16, 17, 18, 19, 21, 22, 29])
+def test_lattice_points_at_equal_distances(t):
+    """residual batches of the lattice types come back bit for bit where many of a group's lattice points lie equally far from the
+    seed: weights of few magnitudes, zeros among them, columns without importance.  Every rank occurs, the ones that
+    the decoder ranks ahead and the ones that it looks up."""
+    import torch
+    from seedpack_b200.gpuquant import GPUQuant
+    from seedpack_b200.qr import QRCodec
+    rows, cols = 96, 3072
+    g = torch.Generator(device="cuda").manual_seed(t)
+    pick = lambda n, values, p: torch.tensor(values, device="cuda")[torch.multinomial(torch.tensor(p), n, replacement=True, generator=torch.Generator().manual_seed(t)).cuda()]
+    x = pick(rows * cols, [-2.0, -1.0, 0.0, 1.0, 2.0], [0.1, 0.35, 0.1, 0.35, 0.1]) * 0.0625
+    x[:cols] = 0.0625                                            # a row of one value, and one of zeros
+    x[cols:2 * cols] = 0
+    x = x.to(torch.bfloat16)
+    imx = pick(cols, [0.0, 1.0], [0.1, 0.9]).float()
+    gq, codec = GPUQuant(), QRCodec()
+    pred = gq.quantize_tensors(t, [(x, cols)], [imx], device=True)[0]
+    noise = torch.where(torch.rand(rows * cols, generator=g, device="cuda") < 0.3, torch.randn(rows * cols, generator=g, device="cuda") * 0.05, 0)
+    file = gq.quantize_tensors(t, [((x.float() + noise).to(torch.bfloat16), cols)], [torch.ones_like(imx)], device=True)[0].clone()
+    seed = x.view(torch.uint8)
+    _, counts = codec.hist(t, [(file, pred, 0, 30, cols, 0)], seed, imx)
+    ranks = counts[214:230].sum(0)                               # the tables of the ranks; 16: a rank past the list's end
+    assert (ranks[:5] > 50).all() and ranks[4:16].sum() > 100 and ranks[16] > 50, ranks[:17]
+    buf = codec.encode(t, [(file, pred, 0, 30, cols, 0)], seed, imx)
+    assert torch.equal(codec.decode(t, buf, [(pred, 0, 30, cols, 0)], seed, imx), file)
