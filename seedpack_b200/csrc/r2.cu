@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
     __syncthreads();
     const bool staged = T.tab == cta_tab && !m.bad;
     const int nbatch = (m.nmax + DB - 1) / DB;
-    DecRing rd; rd.pos = rd.len = 0;
+    DecRing rd; rd.pos = rd.have = 0; rd.left = 0;
     unsigned x = RANS_L;
     bool bad = false;
     if (chain && live) { rd.init(in + in_off[s], in + in_end[s], m.ring + grp); x = rd.state(); }
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
                 const unsigned e = cx[w];
                 const int pe = e & 511, sc = (e >> 9) & 15, pred = (int)e >> 16;
                 const unsigned x0 = x, top0 = rd.top;
-                const int pos0 = rd.pos;
+                const unsigned pos0 = rd.pos;
                 const bool near = staged && (unsigned)(pe - pe0) < (unsigned)D_ECTX;
                 const uint8_t* te = m.expo + (near ? pe - pe0 : 0) * D_EP;
                 bool miss = !near;

@@ -111,7 +111,8 @@ struct RingReader {
     const uint8_t* end;
     uint4 c0, c1;                  // the 32 bytes asked for last
     unsigned* ring;
-    int pos, have, len;            // bits from the aligned start: taken, put into the ring, in the stream
+    unsigned pos, have;            // bits from the aligned start, modulo 2^32: taken, put into the ring (`have` is never far ahead)
+    long long left;                // bits of the stream that are not in the ring yet; negative: it holds some past the end
     unsigned top;                  // the next four bytes, the first one highest
     SG_DEVINL void fetch() {
         c0 = c1 = make_uint4(0, 0, 0, 0);
@@ -120,35 +121,37 @@ struct RingReader {
         src += 32;
     }
     SG_DEVINL void top_up() {
-        if (have - pos <= 8 * (4 * RING_WORDS - 32)) {
-            const int w = (have >> 5) & (RING_WORDS - 1);      // a multiple of 8
+        if ((int)(have - pos) <= 8 * (4 * RING_WORDS - 32)) {
+            const unsigned w = (have >> 5) & (RING_WORDS - 1); // a multiple of 8
             unsigned* r = ring + w * P;
             const unsigned a[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
             for (int i = 0; i < 8; ++i) r[i * P] = __byte_perm(a[i], 0, 0x0123);
             if (w == 0) ring[RING_WORDS * P] = __byte_perm(a[0], 0, 0x0123);
             have += 256;
+            left -= 256;
             fetch();
         }
     }
     SG_DEVINL void look() {
-        const unsigned off = (P >= 8 ? (unsigned)pos * (P / 8) : (unsigned)pos / (8 / P)) & ((RING_WORDS - 1) * P * 4);
+        const unsigned off = (P >= 8 ? pos * (P / 8) : pos / (8 / P)) & ((RING_WORDS - 1) * P * 4);
         const unsigned* r = reinterpret_cast<const unsigned*>(reinterpret_cast<const char*>(ring) + off);
         top = __funnelshift_l(r[P], r[0], pos);                // (the shift counts modulo 32)
     }
     SG_DEVINL void init(const uint8_t* begin, const uint8_t* e, unsigned* r) {
         ring = r;
         src = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(begin) & ~(uintptr_t)15);
-        pos = 8 * (int)(begin - src); have = 0;
+        pos = 8 * (unsigned)(begin - src); have = 0;
         end = e > begin ? e : begin;
-        len = 8 * (int)min((long long)(end - src), 1LL << 27); // (a segment's symbols take far less)
+        left = 8LL * (end - src);
         if (end == begin) end = src;                           // nothing to read
         fetch();
         top_up(); top_up(); top_up();
         look();
     }
-    SG_DEVINL bool over() const { return pos > len; }
-    SG_DEVINL bool at_end() const { return pos == len; }
+    // (a stream may be longer than 2^32 bits: only distances are compared)
+    SG_DEVINL bool over() const { return (int)(pos - have) > left; }
+    SG_DEVINL bool at_end() const { return (int)(pos - have) == left; }
     // x after a step: the bytes that bring it to 2^23 or more.  A coder's state is 2^23 or more before a step, hence 2^8 or
     // more after it: two bytes at most.  (A damaged stream may leave it smaller; it is found out at the segment's end.)
     SG_DEVINL void renorm(unsigned& x) {

@@ -117,3 +117,21 @@ def test_reciprocal_division_is_exact():
     full = np.zeros((3, 256), np.uint16); full[r["used"]] = r["freq"]
     want, woff = orans.encode(sym, bt, 32, 16384, full)
     assert np.array_equal(r["stream"].cpu().numpy()[:r["total"]], want)
+
+
+def test_segment_of_more_than_128_mib():
+    """one segment of 9.0e7 symbols of 12 bits each (135 MB of stream) there and back: positions in a segment are not bounded by
+    what the archive formats' 16 K symbols take"""
+    import torch
+    from seedpack_b200.rans import RansCodec
+    n = 90_177_536
+    c = RansCodec()
+    sym = torch.randint(1, 256, (n,), dtype=torch.uint8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    bt = torch.zeros(n // 32, dtype=torch.int16, device="cuda")
+    freq = np.ones((1, 256), np.uint16)
+    freq[0, 0] = 4096 - 255
+    enc, _ = c.tables(freq, lut=False)
+    stream, off, total = c.encode_with(sym, bt, 32, enc, seg_len=n, cap=(n * 3 // 2 + 4096) // 16 * 16)
+    assert 1 << 27 < total < n * 8 // 5
+    back = c.decode(stream, off, bt, 32, n, freq, np.array([0]), 1, seg_len=n)
+    assert c.status() == 0 and torch.equal(back, sym)
