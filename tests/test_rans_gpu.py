@@ -135,3 +135,26 @@ def test_segment_of_more_than_128_mib():
     assert 1 << 27 < total < n * 8 // 5
     back = c.decode(stream, off, bt, 32, n, freq, np.array([0]), 1, seg_len=n)
     assert c.status() == 0 and torch.equal(back, sym)
+
+
+def test_compact_tables_leave_nothing_unwritten():
+    """the compact table (pb = 15) of an unused row is zero, whatever its memory held: the decoder stages the rows of a whole role"""
+    import ctypes
+
+    import torch
+    from seedpack_b200 import _lib
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    f = np.zeros((3, 256), np.uint16)
+    f[1, :200] = 163
+    f[1, 7] += 32768 - int(f[1].sum(dtype=np.int64))
+    enc = torch.empty(3 * 512, dtype=torch.int32, device="cuda")
+    lut = torch.full((3 * 1280,), 255, dtype=torch.uint8, device="cuda")
+    _lib.check(_lib.lib().sg_rans_tables(0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), p(_dev(f)), 3, 15, p(enc), p(lut)), "sg_rans_tables")
+    l = lut.cpu().numpy().reshape(3, 1280)
+    assert not l[0].any() and not l[2].any()
+    cum = np.cumsum(f[1], dtype=np.int64) - f[1]
+    words = np.frombuffer(l[1, 256:].tobytes(), np.uint32)
+    assert np.array_equal(words, (f[1] | cum << 16).astype(np.uint32))
+    for b in range(256):                                       # the symbol whose range holds slot 128 b
+        s = l[1, b]
+        assert cum[s] <= 128 * b < cum[s] + f[1, s]
