@@ -115,10 +115,11 @@ def test_base_codec_round_trip(rows, cols, spread):
     assert bits.value == 0 and torch.equal(back, w)
 
 
-@pytest.mark.parametrize("rows,cols,off", [(1, 1, 0), (33, 64, 0), (31, 72, 0), (40, 130, 0), (5, 1001, 0), (32, 256, 2), (7, 256, 1)])
+@pytest.mark.parametrize("rows,cols,off", [(1, 1, 0), (33, 64, 0), (31, 72, 0), (40, 130, 0), (5, 1001, 0), (32, 256, 2), (7, 256, 1),
+                                           (1, 1, 1), (2, 2, 1), (3, 63, 1), (9, 65, 7), (34, 127, 1), (4, 4033, 3), (9, 8, 4), (9, 7, 0)])
 def test_row_recurrences(rows, cols, off):
     """row fingerprints and row statistics against the recurrences in Python (integers; float64 sums in order), for rows whose
-    length and address allow 16-byte copies, 4-byte copies and none"""
+    length and address are multiples of 16 bytes, and for rows that begin and end anywhere within them"""
     import ctypes
 
     import torch
