@@ -313,8 +313,11 @@ SG_DEVINL void put_code_shared(int T, unsigned* blk, int w, int q) {
 // small W wastes fewer issue slots on the lockstep parts, a large W spreads the per-weight work wider.  The warp's
 // control flow is kept uniform (every segment of the warp is at its j-th block; segments whose block equals its
 // prediction, or that have ended, sit the phases out), so the lane groups stay converged.
-template <int T, int W>
-__global__ void __launch_bounds__(DW_WARPS * 32) k_qr_dec_warp(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
+// B CTAs per SM at least.  6 (80 registers) once the segments fill five per SM: with its 93 - 96 registers a kernel of Q2_K, Q4_K,
+// Q5_K or Q2_0 gets five, and a last wave of a few CTAs took as long as all others (Q4_K, 12288 segments: 8.0 ms against 5.7).
+// 1 below, where the registers are worth 4 % (2048 segments: 3.47 against 3.60 ms).
+template <int T, int W, int B>
+__global__ void __launch_bounds__(DW_WARPS * 32, B) k_qr_dec_warp(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
                                                                const RansSym* __restrict__ enc, const uchar* __restrict__ lut,
                                                                uchar* __restrict__ F, int* __restrict__ status) {
     constexpr int SPW = 32 / W;
@@ -922,20 +925,12 @@ extern "C" int sg_qr_decode(int device, void* stream, int T, const unsigned char
         auto run = [&](auto kernel) {
             kernel<<<(nseg + per_cta - 1) / per_cta, DW_WARPS * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F, status_word(device));
         };
+        const bool crowded = nseg > 148 * 5 * per_cta;
         switch (T) {
-            case 2: run(k_qr_dec_warp<2, W>); break;
-            case 3: run(k_qr_dec_warp<3, W>); break;
-            case 6: run(k_qr_dec_warp<6, W>); break;
-            case 7: run(k_qr_dec_warp<7, W>); break;
-            case 8: run(k_qr_dec_warp<8, W>); break;
-            case 10: run(k_qr_dec_warp<10, W>); break;
-            case 11: run(k_qr_dec_warp<11, W>); break;
-            case 12: run(k_qr_dec_warp<12, W>); break;
-            case 13: run(k_qr_dec_warp<13, W>); break;
-            case 14: run(k_qr_dec_warp<14, W>); break;
-            case 20: run(k_qr_dec_warp<20, W>); break;
-            case 23: run(k_qr_dec_warp<23, W>); break;
-            case 42: run(k_qr_dec_warp<42, W>); break;
+#define SG_DEC(t) case t: if (crowded) run(k_qr_dec_warp<t, W, 6>); else run(k_qr_dec_warp<t, W, 1>); break;
+            SG_DEC(2) SG_DEC(3) SG_DEC(6) SG_DEC(7) SG_DEC(8) SG_DEC(10) SG_DEC(11)
+            SG_DEC(12) SG_DEC(13) SG_DEC(14) SG_DEC(20) SG_DEC(23) SG_DEC(42)
+#undef SG_DEC
             default: return SG_ERR_TYPE;
         }
     }

@@ -176,3 +176,33 @@ def test_lattice_points_at_equal_distances(t):
     assert (ranks[:5] > 50).all() and ranks[4:16].sum() > 100 and ranks[16] > 50, ranks[:17]
     buf = codec.encode(t, [(file, pred, 0, 30, cols, 0)], seed, imx)
     assert torch.equal(codec.decode(t, buf, [(pred, 0, 30, cols, 0)], seed, imx), file)
+
+
+def _quantised_pair(t, n, cols, seed, importance=None):
+    """n weights, and their blocks of type t as a prediction and as a file made from slightly other weights"""
+    import torch
+    from seedpack_b200.gpuquant import GPUQuant
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = (torch.randn(n, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    y = torch.where(torch.rand(n, generator=g, device="cuda") < 0.1, x + torch.randn(n, generator=g, device="cuda") * 0.01, x.float()).to(torch.bfloat16)
+    pred, file = (GPUQuant().quantize_tensors(t, [(v, cols)], [importance], device=True)[0].clone() for v in (x, y))
+    return x, pred, file
+
+
+@pytest.mark.parametrize("t", [2, 3, 6, 7, 8, 10, 11, 12, 13, 14, 20, 23, 42])
+def test_residual_decoder_with_many_segments(t):
+    """more segments than five CTAs a SM take, of one and two blocks (a tensor each), the last CTA partly filled"""
+    import torch
+    from seedpack_b200.qr import BS, QK, QRCodec
+    nseg, qk, bs = 148 * 5 * 16 + 5, QK[t], BS[t]
+    nb = nseg + nseg // 3
+    x, pred, file = _quantised_pair(t, nb * qk, qk, t)
+    items, b = [], 0
+    for i in range(nseg):
+        k = 2 if i < nseg // 3 else 1
+        items.append((file[b * bs:(b + k) * bs], pred[b * bs:(b + k) * bs], 2 * b * qk, 30, qk))
+        b += k
+    codec, seed = QRCodec(), x.view(torch.uint8)
+    assert 0.05 < (file.view(nb, bs) != pred.view(nb, bs)).any(1).float().mean() <= 1
+    buf = codec.encode(t, items, seed)
+    assert torch.equal(codec.decode(t, buf, [it[1:] for it in items], seed), file)
