@@ -421,24 +421,26 @@ __global__ void __launch_bounds__(DW_WARPS * 32, B) k_qr_dec_warp(const Args a, 
 // ---- decoder of the lattice types: a CTA per segment -------------------------------------------------------------------
 // What makes these blocks expensive is the ordering of all 256 - 2048 lattice points by their weighted distance to the
 // seed, once per group of 4 / 8 weights.  It depends on the seed and on the block's scale fields only, so that once the
-// fields are decoded the eight warps rank all groups of the block side by side (four units of 8 weights each): the closest
-// four points and the gap context of every group go to shared memory.  The first warp then runs the chain - ranks and
-// signs - over them, all lanes in lockstep, while the others fetch the next block and sum its squares.  A rank beyond the
-// fourth is looked up when it occurs.  (One warp per segment that ranked a group when the chain came to it: 6100 cycles
-// a group, 13.2 ms for the 1024 x 3072 weights of an IQ3_S tensor.)
-constexpr int GW = 8, GTOP = 4;                    // warps per CTA; ranked points kept per group
-struct GridSmem {
+// fields are decoded the CTA's warps rank all groups of the block side by side, four units of 8 weights at a time: the closest
+// points and the gap context of every group go to shared memory.  The first warp then runs the chain - ranks and signs - over
+// them, all lanes in lockstep, while the others fetch the next block and sum its squares.  A rank that is not among the
+// closest four is looked up when it occurs; so is the group's order where IQ1_M's shift bit is not the prediction's, on which the
+// level offset hangs.  (One warp per segment that ranked a group when the chain came to it: 13.2 ms for the 1024 x 3072
+// weights of an IQ3_S tensor against 4.9, 60 ms for 2 x 4096 x 12288 against 39.)
+// Bound by the chain with few segments, by the issue of the ranking with many: B CTAs per SM, that is 64 registers a thread.
+constexpr int GTOP = 4;                            // ranked points kept per group
+template <int T, int GW> struct GridSmem {           // GW: warps per CTA
     unsigned f01[NTAB2];                           // per table: frequency of symbol 0 | of symbol 1 << 16
     unsigned ring[RING_ROWS];
     unsigned fblk[28], pblk[2][28];                // block sizes <= 110 bytes
     float xs[2][256];                              // the block's seed values; this block and the next
     float sx2[2];
     float tab[GW][128];                            // pair tables of the group a warp ranks: [pair][levels]
-    float dist[2048];                              // distance of every lattice point (ranks beyond GTOP)
+    float dist[grid_size(T)];                      // distance of every lattice point (ranks beyond GTOP)
     float gu[256], gw[256];                        // per weight: seed value over the unit's scale (sign-folded), search weight
-    unsigned short gk[2048];                       // the lattice's points
-    unsigned short top[2][64][GTOP];               // [IQ1_M's shift bit][group]: closest points in order, 0xffff: none
-    unsigned char gap[2][64];
+    unsigned short gk[grid_size(T)];               // the lattice's points
+    unsigned short top[64][GTOP];                  // per group: closest points in order, NOPOINT, NOTKNOWN
+    unsigned char gap[64];
     unsigned char pn[32], neg[32], shift[32];      // per unit: negative seed values; decoded sign symbols, shift bit
     unsigned short tg[64];
     int tv[MAXF];
@@ -449,10 +451,10 @@ template <int N> SG_DEVINL float point_dist_w(const float* tab, unsigned key) {
     float d = 0.f;
 #pragma unroll
     for (int p = 0; p < N / 2; ++p) d = d + tab[p * E + ((key >> (2 * B * p)) & (E - 1))];
-    return isnan(d) ? __int_as_float(0x7f800000) : d;
+    return fminf(d, __int_as_float(0x7f800000));   // (NaN: infinity)
 }
 // pair tables of the group of weights w0 .. w0 + N - 1, entries spread over the lanes
-template <int N, bool SGN> SG_DEVINL void group_tables(float* tab, const GridSmem& m, int w0, float gdl, int lane) {
+template <int N, bool SGN, class S> SG_DEVINL void group_tables(float* tab, const S& m, int w0, float gdl, int lane) {
     constexpr int B = N == 8 ? 2 : 3, L = 1 << B, E = L * L;
 #pragma unroll
     for (int e = lane; e < (N / 2) * E; e += 32) {
@@ -466,58 +468,70 @@ template <int N, bool SGN> SG_DEVINL void group_tables(float* tab, const GridSme
 // a float's bits in an unsigned order (no NaN comes here)
 SG_DEVINL unsigned ordered_bits(float d) { const unsigned u = __float_as_uint(d); return u ^ ((unsigned)((int)u >> 31) | 0x80000000u); }
 
-// Closest GTOP points of one group in the order (distance, index), and its gap context.  Every lane keeps the closest of
+// The lattice's points in shared memory: a word holds the points k and k + 32 of every 64
+SG_DEVINL int gk_at(int k) { return (k & ~63) + 2 * (k & 31) + ((k >> 5) & 1); }
+
+// Closest GTOP points of one group in the order (distance, index), and its gap context.  Every lane keeps the closest two of
 // its own points (lane, lane + 32, ...; met in index order): a point goes in before the first one that is further away, so
 // after its equals, and what stands there moves down one place, whatever the distances.  The warp's next one is then an
-// arg-min over the lanes' lists.  Points at infinite distance never come up.
-template <int N, bool SGN> SG_DEVINL void rank_group(GridSmem& m, float* tab, int gs, int w0, float gdl, int lane, unsigned short* top, unsigned char* gap) {
+// arg-min over the lanes' lists.  Points at infinite distance never come up.  A lane that has given both of its points leaves
+// the ranks after them unknown: looked up where one is coded.  (Lists of four cost as much as the distances themselves: IQ1_S
+// 24576 segments 187 ms, with lists of two 142.)
+constexpr int NOPOINT = 0xffff, NOTKNOWN = 0xfffe, LLEN = 2;
+template <int N, bool SGN, int gs, class S> SG_DEVINL void rank_group(S& m, float* tab, int w0, float gdl, int lane, unsigned short* top, unsigned char* gap) {
     const float inf = __int_as_float(0x7f800000);
     __syncwarp();
     group_tables<N, SGN>(tab, m, w0, gdl, lane);
     __syncwarp();
-    float D[GTOP]; int K[GTOP];
+    float D[LLEN]; int K[LLEN];
 #pragma unroll
-    for (int l = 0; l < GTOP; ++l) { D[l] = inf; K[l] = 0xffff; }
+    for (int l = 0; l < LLEN; ++l) { D[l] = inf; K[l] = NOPOINT; }
+    auto insert = [&](float d, int k) {
+        bool lt[LLEN];
+#pragma unroll
+        for (int l = 0; l < LLEN; ++l) lt[l] = d < D[l];
+#pragma unroll
+        for (int l = LLEN - 1; l > 0; --l) { D[l] = fminf(fmaxf(d, D[l - 1]), D[l]); K[l] = lt[l - 1] ? K[l - 1] : lt[l] ? k : K[l]; }
+        D[0] = fminf(d, D[0]); K[0] = lt[0] ? k : K[0];
+    };
+    const unsigned* gk2 = reinterpret_cast<const unsigned*>(m.gk) + lane;
 #pragma unroll 4
-    for (int k0 = 0; k0 < gs; k0 += 32) {
-        float d = point_dist_w<N>(tab, m.gk[k0 + lane]);
-        int k = k0 + lane;
-        bool in = false;                           // from here on d, k are the one that was moved out of the place before
-#pragma unroll
-        for (int l = 0; l < GTOP; ++l) {
-            in = in || d < D[l];
-            const float dm = D[l]; const int km = K[l];
-            D[l] = in ? d : dm; K[l] = in ? k : km;
-            d = in ? dm : d; k = in ? km : k;
-        }
+    for (int k = 0; k < gs; k += 64) {
+        const unsigned kk = gk2[k / 2];
+        insert(point_dist_w<N>(tab, kk & 0xffffu), k + lane);
+        insert(point_dist_w<N>(tab, kk >> 16), k + 32 + lane);
     }
     float d1 = inf, d2 = inf;
+    int given = 0;
+    bool known = true;
 #pragma unroll
     for (int j = 0; j < GTOP; ++j) {
         const unsigned key = ordered_bits(D[0]), best = __reduce_min_sync(0xffffffffu, key);
-        const unsigned bk = __reduce_min_sync(0xffffffffu, key == best ? (unsigned)K[0] : 0xffffu);
-        if (lane == 0) top[j] = (unsigned short)bk;
+        const unsigned bk = __reduce_min_sync(0xffffffffu, key == best ? (unsigned)K[0] : (unsigned)NOPOINT);
+        if (lane == 0) top[j] = (unsigned short)(known ? bk : NOTKNOWN);
         if (j < 2) {
             const float d = __uint_as_float(best ^ ((best >> 31) ? 0x80000000u : 0xffffffffu));
             if (j == 0) d1 = d; else d2 = d;
         }
-        if (key == best && (unsigned)K[0] == bk) {
+        if (key == best && (unsigned)K[0] == bk && bk != NOPOINT) {
 #pragma unroll
-            for (int l = 0; l + 1 < GTOP; ++l) { D[l] = D[l + 1]; K[l] = K[l + 1]; }
-            D[GTOP - 1] = inf; K[GTOP - 1] = 0xffff;
+            for (int l = 0; l + 1 < LLEN; ++l) { D[l] = D[l + 1]; K[l] = K[l + 1]; }
+            D[LLEN - 1] = inf; K[LLEN - 1] = NOPOINT;
+            ++given;
         }
+        if (j + 1 >= LLEN && j + 1 < GTOP) known = known && !__any_sync(0xffffffffu, given == LLEN);
     }
     if (lane == 0) *gap = (unsigned char)gapctx(d1, d2);
 }
-// the point of rank r >= GTOP, by the first warp: distances to shared memory, then r + 1 rounds of an arg-min
-template <int N, bool SGN> SG_DEVINL int deep_rank(GridSmem& m, int gs, int w0, float gdl, int r, int lane) {
+// the point of rank r, by the first warp: distances to shared memory, then r + 1 rounds of an arg-min
+template <int N, bool SGN, int gs, class S> SG_DEVINL int deep_rank(S& m, int w0, float gdl, int r, int lane) {
     const float inf = __int_as_float(0x7f800000);
     __syncwarp();
     group_tables<N, SGN>(m.tab[0], m, w0, gdl, lane);
     __syncwarp();
     float md = inf; int mk = 0x7fffffff;
     for (int k = lane; k < gs; k += 32) {
-        const float d = point_dist_w<N>(m.tab[0], m.gk[k]);
+        const float d = point_dist_w<N>(m.tab[0], m.gk[gk_at(k)]);
         m.dist[k] = d;
         if (d < md) { md = d; mk = k; }
     }
@@ -540,25 +554,28 @@ template <int N, bool SGN> SG_DEVINL int deep_rank(GridSmem& m, int gs, int w0, 
     return bk == 0x7fffffff ? r : bk;              // slots beyond the points at finite distance keep their own number
 }
 
-template <int T>
-__global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
+template <int T, int GW, int B>
+__global__ void __launch_bounds__(GW * 32, B) k_qr_dec_grid(const Args a, const uchar* __restrict__ in, const unsigned long long* __restrict__ off,
                                                          const RansSym* __restrict__ enc, const uchar* __restrict__ lut,
                                                          uchar* __restrict__ F, int* __restrict__ status) {
-    constexpr int N = T == 18 || T == 21 ? 4 : 8, ng = 8 / N, B = N == 8 ? 2 : 3, gs = grid_size(T), bs = bs_of(T), nf = nfield(T);
+    constexpr int N = T == 18 || T == 21 ? 4 : 8, ng = 8 / N, LB = N == 8 ? 2 : 3, gs = grid_size(T), bs = bs_of(T), nf = nfield(T);
     constexpr bool SGN = T != 19 && T != 29, par = parity_type(T);
-    __shared__ __align__(16) GridSmem m;
+    __shared__ __align__(16) GridSmem<T, GW> m;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.x, mv = a.mv;
     const Setup u = setup(T, a.seed, a.tm, a.sg, s);
     const float* im = u.m.imx_off >= 0 ? a.imx + u.m.imx_off : nullptr;
     for (int t = threadIdx.x; t < NTAB2; t += GW * 32) m.f01[t] = (enc[t * 256].fc & 0xffffu) | (enc[t * 256 + 1].fc << 16);
-    for (int k = threadIdx.x; k < gs; k += GW * 32) m.gk[k] = a.gk[k];
-    // block j of the segment into buffer j & 1, by the threads of warps w0 .. GW - 1
+    for (int k = threadIdx.x; k < gs; k += GW * 32) m.gk[gk_at(k)] = a.gk[k];
+    // prediction / seed values of block j of the segment into buffer j & 1, by the warps w0 .. GW - 1
     auto fetch = [&](int j, int w0) {
-        const int t = (int)threadIdx.x - 32 * w0;
-        if (t < 0 || j >= u.g.nb) return;
-        const long long b = u.g.b0 + j, gw0 = (b - u.m.blk0) * 256;
-        for (int i = t; i < bs; i += 32 * (GW - w0)) reinterpret_cast<uchar*>(m.pblk[j & 1])[i] = a.P[b * bs + i];
-        for (int i = t; i < 256; i += 32 * (GW - w0)) { float xv, hv; seed_val(u.m.seed_type, u.sbase, gw0 + i, xv, hv, u.m.cols); m.xs[j & 1][i] = xv; }
+        const long long b = u.g.b0 + j;
+        if (j < u.g.nb) for (int i = (int)threadIdx.x - 32 * w0; i < bs; i += 32 * (GW - w0)) reinterpret_cast<uchar*>(m.pblk[j & 1])[i] = a.P[b * bs + i];
+    };
+    auto fetch_seed = [&](int j, int w0) {
+        const long long gw0 = (u.g.b0 + j - u.m.blk0) * 256;
+        for (int i = (int)threadIdx.x - 32 * w0; i < 256; i += 32 * (GW - w0)) {
+            float xv, hv; seed_val(u.m.seed_type, u.sbase, gw0 + i, xv, hv, u.m.cols); m.xs[j & 1][i] = xv;
+        }
     };
     auto sum_squares = [&](int j) {                // in order; one warp, every lane the same
         float sx2 = 0.f;
@@ -568,7 +585,7 @@ __global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uch
     };
     fetch(0, 0);
     __syncthreads();
-    if (warp == 1) sum_squares(0);
+    bool ahead = false;                            // block j's seed values are there
     QrDec c; c.enc = enc; c.lut = lut; c.f01 = m.f01;
     int prev = 1;
     if (warp == 0) { c.r.init(in + off[s], in + off[s + 1], m.ring); c.x = c.r.state(); }
@@ -614,44 +631,53 @@ __global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uch
         const int eq = m.eq;
         if (eq == 2) break;
         const long long col0 = u.m.cols > 0 ? gw0 % u.m.cols : 0;
+        if (eq == 0 && !ahead) {
+            fetch_seed(j, 0);
+            __syncthreads();
+            if (warp == 1) sum_squares(j);
+            __syncthreads();
+        }
         if (eq == 0) {
-            // this warp's four units, a weight per lane: search weight, sign folding with the parity repair, value over scale
-            const int un = 4 * warp + (lane >> 3), i = lane & 7, w = 32 * warp + lane;
-            const float sx2 = m.sx2[j & 1], sigma2 = (T == 16 || T == 17) ? sx2 * (1.0f / 256.f) : 2.f * sx2 * (1.0f / 256.f);
-            float gs_, gdl;
-            gscale(T, fb, m.tv, un, gs_, gdl);     // (the scale does not depend on IQ1_M's shift bit)
-            const float x = m.xs[j & 1][w];
-            float wi = sqrtf(sigma2 + x * x);
-            if (im) wi = wi * im[(gw0 + w) % u.m.cols];
-            float v = SGN ? fabsf(x) : x;
-            unsigned pnb = (__ballot_sync(0xffffffffu, x < 0.f) >> (8 * (lane >> 3))) & 255u;
-            if (SGN && par) {                      // an odd number of negatives: the least weighty one flips back
-                const float e = wi * x * x;
-                int imin = 0; float mn = __shfl_sync(0xffffffffu, e, 0, 8);
+            // four units at a time, a weight per lane: search weight, sign folding with the parity repair, value over scale
+#pragma unroll 1
+            for (int part = warp; part < 8; part += GW) {
+                const int un = 4 * part + (lane >> 3), i = lane & 7, w = 32 * part + lane;
+                const float sx2 = m.sx2[j & 1], sigma2 = (T == 16 || T == 17) ? sx2 * (1.0f / 256.f) : 2.f * sx2 * (1.0f / 256.f);
+                float gs_, gdl;
+                gscale(T, fb, m.tv, un, gs_, gdl); // (the scale does not depend on IQ1_M's shift bit)
+                const float x = m.xs[j & 1][w];
+                float wi = sqrtf(sigma2 + x * x);
+                if (im) wi = wi * im[(gw0 + w) % u.m.cols];
+                float v = SGN ? fabsf(x) : x;
+                unsigned pnb = (__ballot_sync(0xffffffffu, x < 0.f) >> (8 * (lane >> 3))) & 255u;
+                if (SGN && par) {                  // an odd number of negatives: the least weighty one flips back
+                    const float e = wi * x * x;
+                    int imin = 0; float mn = __shfl_sync(0xffffffffu, e, 0, 8);
 #pragma unroll
-                for (int q = 1; q < 8; ++q) { const float o = __shfl_sync(0xffffffffu, e, q, 8); if (o < mn) { mn = o; imin = q; } }
-                if (__popc(pnb) & 1) { pnb ^= 1u << imin; if (i == imin) v = -v; }
-            }
-            m.gu[w] = v / gs_; m.gw[w] = wi;
-            if (i == 0) m.pn[un] = (unsigned char)pnb;
-            __syncwarp();
+                    for (int q = 1; q < 8; ++q) { const float o = __shfl_sync(0xffffffffu, e, q, 8); if (o < mn) { mn = o; imin = q; } }
+                    if (__popc(pnb) & 1) { pnb ^= 1u << imin; if (i == imin) v = -v; }
+                }
+                m.gu[w] = v / gs_; m.gw[w] = wi;
+                if (i == 0) m.pn[un] = (unsigned char)pnb;
+                __syncwarp();
 #pragma unroll 1
-            for (int q = 0; q < 4 * ng; ++q) {
-                const int g = 4 * ng * warp + q;
-                float sc, dl;
-                gscale(T, fb, m.tv, g / ng, sc, dl);
-                if (T != 29) rank_group<N, SGN>(m, m.tab[warp], gs, N * g, dl, lane, m.top[0][g], &m.gap[0][g]);
-                else {                             // the level offset hangs on a shift bit that the chain decodes: both are ranked
-#pragma unroll 1
-                    for (int h = 0; h < 2; ++h) rank_group<N, SGN>(m, m.tab[warp], gs, N * g, h ? -0.125f : 0.125f, lane, m.top[h][g], &m.gap[h][g]);
+                for (int q = 0; q < 4 * ng; ++q) {
+                    const int g = 4 * ng * part + q;
+                    float sc, dl;
+                    gscale(T, fb, m.tv, g / ng, sc, dl);
+                    if (T == 29) dl = get_shift(pbs, g) ? -0.125f : 0.125f;      // (the chain decodes whether the shift bit is the prediction's)
+                    rank_group<N, SGN, gs>(m, m.tab[warp], N * g, dl, lane, m.top[g], &m.gap[g]);
                 }
             }
         }
         __syncthreads();
         if (warp > 0) {
             fetch(j + 1, 1);
-            asm volatile("bar.sync 1, %0;" ::"n"((GW - 1) * 32) : "memory");
-            if (warp == 1 && j + 1 < u.g.nb) sum_squares(j + 1);
+            if (eq == 0 && j + 1 < u.g.nb) {       // after a block that differs the next one is expected to differ as well
+                fetch_seed(j + 1, 1);
+                asm volatile("bar.sync 1, %0;" ::"n"((GW - 1) * 32) : "memory");
+                if (warp == 1) sum_squares(j + 1);
+            }
         } else if (eq) {
             for (int i = lane; i < bs; i += 32) F[b * bs + i] = pbs[i];
         } else {
@@ -665,22 +691,26 @@ __global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uch
                 int h = 0;
                 float gs_, gdl;
                 gscale(T, fb, m.tv, un, gs_, gdl);
-                if (T == 29) { h = (c.get(GRID_SHIFT) ^ get_shift(pbs, un)) != 0; gdl = h ? -0.125f : 0.125f; }
+                if (T == 29) {
+                    const int sp = get_shift(pbs, un);
+                    h = (c.get(GRID_SHIFT) ^ sp) != 0; gdl = h ? -0.125f : 0.125f;
+                    if (h != sp) { rank_group<N, SGN, gs>(m, m.tab[0], N * un, gdl, lane, m.top[un], &m.gap[un]); __syncwarp(); }
+                }
                 int tg[2] = {0, 0};
 #pragma unroll
                 for (int gg = 0; gg < ng; ++gg) {
                     const int g = un * ng + gg;
-                    const int r = c.get(rank0 + m.gap[h][g]);
-                    int t;
+                    const int r = c.get(rank0 + m.gap[g]);
+                    int t = r < GTOP ? m.top[g][r] : NOTKNOWN;
                     if (r >= TOPK) { const int lo = c.get(FESC_LO), hi = c.get(FESC_HI); t = (lo | (hi << 8)) % gs; }
-                    else if (r < GTOP) { t = m.top[h][g][r]; if (t == 0xffff) t = r; }
-                    else t = deep_rank<N, SGN>(m, gs, N * g, gdl, r, lane);
+                    else if (t == NOTKNOWN) t = deep_rank<N, SGN, gs>(m, N * g, gdl, r, lane);
+                    else if (t == NOPOINT) t = r;
                     tg[gg] = t;
                 }
                 unsigned neg = 0;
                 if (SGN) {
                     // lane j works out the context of sign j; the chain then takes the contexts' tables from the lanes
-                    const int j8 = lane & 7, lev = (m.gk[ng == 2 && j8 >= 4 ? tg[1] : tg[0]] >> (B * (j8 % N))) & ((1 << B) - 1);
+                    const int j8 = lane & 7, lev = (m.gk[gk_at(ng == 2 && j8 >= 4 ? tg[1] : tg[0])] >> (LB * (j8 % N))) & ((1 << LB) - 1);
                     const float m4 = fabsf(m.gu[8 * un + j8]) * 4.f;
                     const int sctx = sign0 + (lev == 0) * 8 + (m4 < 7.f ? (int)m4 : 7);
                     const unsigned sw = m.f01[sctx], pn = m.pn[un];
@@ -707,6 +737,7 @@ __global__ void __launch_bounds__(GW * 32) k_qr_dec_grid(const Args a, const uch
             __syncwarp();
             for (int i = lane; i < bs; i += 32) F[b * bs + i] = fb[i];
         }
+        ahead = eq == 0;
         __syncthreads();
     }
     if (threadIdx.x == 0 && (c.r.over() || c.x != RANS_L || !c.r.at_end())) atomicOr(status, SG_ST_CORRUPT);
@@ -908,15 +939,15 @@ extern "C" int sg_qr_decode(int device, void* stream, int T, const unsigned char
     rc = use_device(device);
     if (rc != SG_OK) return rc;
     if (qr::is_grid(T)) {
-        auto run = [&](auto kernel) { kernel<<<nseg, GW * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F, status_word(device)); };
+        // up to four CTAs per SM: eight warps rank a block the faster; beyond, twice the segments side by side count for more (IQ1_S:
+        // 384 segments 3.97 ms with eight warps and 4.09 with four, 768 segments 6.96 and 6.40, 6144 segments 42.7 and 36.9)
+        auto run = [&](auto kernel, int warps) {
+            kernel<<<nseg, warps * 32, 0, (cudaStream_t)stream>>>(a, in, off, (const RansSym*)enc_tab, lut, F, status_word(device));
+        };
         switch (T) {
-            case 16: run(k_qr_dec_grid<16>); break;
-            case 17: run(k_qr_dec_grid<17>); break;
-            case 18: run(k_qr_dec_grid<18>); break;
-            case 19: run(k_qr_dec_grid<19>); break;
-            case 21: run(k_qr_dec_grid<21>); break;
-            case 22: run(k_qr_dec_grid<22>); break;
-            default: run(k_qr_dec_grid<29>);
+#define SG_DEC(t) case t: if (nseg <= 148 * 4) run(k_qr_dec_grid<t, 8, 4>, 8); else run(k_qr_dec_grid<t, 4, 8>, 4); break;
+            SG_DEC(16) SG_DEC(17) SG_DEC(18) SG_DEC(19) SG_DEC(21) SG_DEC(22) SG_DEC(29)
+#undef SG_DEC
         }
     }
     else

@@ -206,3 +206,28 @@ def test_residual_decoder_with_many_segments(t):
     assert 0.05 < (file.view(nb, bs) != pred.view(nb, bs)).any(1).float().mean() <= 1
     buf = codec.encode(t, items, seed)
     assert torch.equal(codec.decode(t, buf, [it[1:] for it in items], seed), file)
+
+
+@pytest.mark.parametrize("t", [16, 17, 18, 19, 21, 22, 29])
+def test_lattice_decoder_with_many_segments(t):
+    """more segments than the kernel of eight warps is used for, of one to three blocks (a tensor each); blocks that equal their
+    prediction and blocks that do not follow one another in every order"""
+    import torch
+    from seedpack_b200.qr import BS, QRCodec
+    nseg, bs = 148 * 4 + 1, BS[t]
+    sizes = [1 + i % 3 for i in range(nseg)]
+    nb = sum(sizes)
+    imx = torch.linspace(0.5, 2.0, 256, device="cuda")
+    x, pred, file = _quantised_pair(t, nb * 256, 256, t, imx)
+    keep = torch.rand(nb, generator=torch.Generator(device="cuda").manual_seed(t), device="cuda") < 0.5
+    file = torch.where(keep[:, None], pred.view(nb, bs), file.view(nb, bs)).reshape(-1)
+    items, b = [], 0
+    for k in sizes:
+        items.append((file[b * bs:(b + k) * bs], pred[b * bs:(b + k) * bs], 2 * b * 256, 30, 256, 0))
+        b += k
+    codec, seed = QRCodec(), x.view(torch.uint8)
+    buf = codec.encode(t, items, seed, imx)
+    assert torch.equal(codec.decode(t, buf, [it[1:] for it in items], seed, imx), file)
+    one = [(file, pred, 0, 30, 256, 0)]                          # the same blocks in few segments
+    buf = codec.encode(t, one, seed, imx)
+    assert torch.equal(codec.decode(t, buf, [it[1:] for it in one], seed, imx), file)
