@@ -246,68 +246,142 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
 
 // Decoder.  A segment is one rANS chain by format, but what a weight's symbols are decoded WITH - the exponent's and the
 // sign's tables, the prediction the mantissa's table is picked by - depends on its row and column only.  A CTA (one per SM)
-// takes up to 64 segments, as few as fill the SMs: eight warps run the chains, a segment per lane, over contexts that eight
-// more warps (four lanes a segment) stage for the next 32 weights while they store the 32 weights before.  A chain warp and
+// takes a piece of up to 96 segments of one role: up to twelve warps run the chains, a segment per lane, over contexts that as
+// many warps (four lanes a segment) stage for the next 32 weights while they store the 32 weights before.  A chain warp and
 // its staging warp wait for each other only; few lanes to a chain warp, since one lane's walk through a bucket or top-up
 // of its ring holds up the others (four chain warps behind one barrier: 10.7 ms for 2 x 4096 x 12288 weights).
 // The chain is three table searches per weight, and what they cost is the memory the tables are in: 656 tables do not fit
-// the L1.  In shared memory are, of the role of the CTA's first segment, the 128 mantissa tables, 16 sign tables and the
-// exponent tables of 128 contexts (16 octaves) around that segment's first weight, each as the cumulated frequencies plus
-// the symbol that holds every 128th slot; anything else goes through the tables in global memory.
-constexpr int DB = 32, DSEG = 64, DG = 4, DW = DB / DG;          // weights per batch, segments per CTA, staging lanes per segment and their weights
-constexpr int D_CHAIN = 256, D_THREADS = D_CHAIN + DG * DSEG;
-constexpr int D_ECTX = 128, D_MCTX = 128, D_MP = 256 + 260, D_EP = 256 + 516;       // bytes per table: 256 coarse, 130 / 258 cumulated
+// the L1.  In shared memory are, of the piece's role, the 128 mantissa tables, 16 sign tables and, of the exponent tables of
+// 128 contexts (16 octaves) around the piece's first weight, 64 exponents each, as the cumulated frequencies plus the symbol
+// that holds every 128th slot; anything else goes through the tables in global memory.
+// Pieces: the segments come in runs of one role, cut evenly.  A CTA of two roles, one of them without tables, took three times
+// as long (28 layers of seven projections, layer by layer: 36.6 ms; 22.5 with no tables in shared memory at all).  Runs that are
+// too short for that are decoded from global memory, four lanes a segment, 192 segments a CTA: see dec_plan().
+constexpr int DB = 32, DG = 4, DW = DB / DG;                     // weights per batch, lanes per segment in the staging warps and their weights
+constexpr int D_PAIRS = 12, DSEG = 8 * D_PAIRS, D_THREADS = 2 * 32 * D_PAIRS, D_RING = 128;
+constexpr int D_ECTX = 128, D_ESYM = 64, D_MCTX = 128, D_MP = 256 + 260, D_EP = 256 + 132;     // bytes per table: 256 coarse, 130 / 66 cumulated
+constexpr int GSEG = D_THREADS / DG, G_RING = 256;               // segments of a CTA that decodes from global memory
+constexpr int D_RUNS = 1024;
 struct DecSmem {
-    unsigned ring[RING_ROWS * DSEG];
-    unsigned ctx[2][DSEG][DB + 1];                               // pe | sc << 9 | pred << 16; rows padded
-    unsigned sign[16];                                           // frequency of symbol 0 | of symbol 1 << 16
-    unsigned short out[2][DSEG][DB + 2];
-    uint8_t mant[D_MCTX * D_MP], expo[D_ECTX * D_EP];
-    int nmax, pe0, bad;
+    int runs[D_RUNS + 1], warp_sum[D_THREADS / 32], pieces[4], first, count;
+    int nmax, pe0, ex0, bad;
+    union {
+        struct {
+            unsigned ring[RING_ROWS * D_RING];
+            unsigned ctx[2][DSEG][DB + 1];                       // pe | sc << 9 | pred << 16; rows padded
+            unsigned sign[16];                                   // frequency of symbol 0 | of symbol 1 << 16
+            unsigned short out[2][DSEG][DB + 2];
+            uint8_t mant[D_MCTX * D_MP], expo[D_ECTX * D_EP];
+        };
+        struct {
+            unsigned g_ring[RING_ROWS * G_RING];
+            unsigned g_ctx[GSEG][DB + 1];
+            unsigned short g_out[GSEG][DB + 2];
+        };
+    };
 };
-// stage a compact table; false: it has symbols from `nsym` on, or is not a whole distribution (an unused one)
-SG_DEVINL void stage_table(const uint8_t* __restrict__ ct, uint8_t* dst, int nsym, int lane, int& bad) {
+static_assert(sizeof(DecSmem) <= 227 * 1024, "one CTA per SM");
+typedef RingReader<D_RING> DecRing;
+// (mctx() is constant outside of +-4000)
+SG_DEVINL unsigned pack_ctx(int pred, int pe, int sc) { return (unsigned)pe | (unsigned)sc << 9 | (unsigned)clampi(pred, -4000, 4000) << 16; }
+
+// How the segments are cut, the same in every CTA: the pieces' number and size; a negative size: pieces of any roles.  A wave of
+// pieces takes 4.9 ms with 21 segments each and 6.4 ms with 83, so what counts is the number of waves: a larger piece is
+// taken where that saves one.  Segments of any roles, from global memory: 19.7 ms for 6000, 23 for 26000 (in runs of ten).
+SG_DEVINL int dec_plan(DecSmem& m, const TB* __restrict__ tb, const SG* __restrict__ sg, int nseg, int& per) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int chunk = (nseg + D_THREADS - 1) / D_THREADS;
+    const int i0 = (int)min((long long)threadIdx.x * chunk, (long long)nseg), i1 = (int)min((long long)i0 + chunk, (long long)nseg);
+    auto starts = [&](auto&& f) {
+        int prev = i0 > 0 && i0 < i1 ? sg[i0 - 1].t : -1;
+#pragma unroll 4
+        for (int i = i0; i < i1; ++i) {
+            const int t = sg[i].t;
+            if (prev < 0 || (t != prev && tb[t].tab != tb[prev].tab)) f(i);
+            prev = t;
+        }
+    };
+    int n = 0;
+    starts([&](int) { ++n; });
+    int incl = n;
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+    if (lane == 31) m.warp_sum[warp] = incl;
+    if (threadIdx.x < 4) m.pieces[threadIdx.x] = 0;
+    __syncthreads();
+    int at = incl - n, nruns = 0;
+    for (int w = 0; w < D_THREADS / 32; ++w) { if (w < warp) at += m.warp_sum[w]; nruns += m.warp_sum[w]; }
+    const int gwaves = (nseg + 148 * GSEG - 1) / (148 * GSEG), gper = min(GSEG, ((nseg + 148 * gwaves - 1) / (148 * gwaves) + 7) / 8 * 8);
+    const int gpieces = (nseg + gper - 1) / gper;
+    per = -gper;
+    if (nruns > D_RUNS) return gpieces;
+    starts([&](int i) { m.runs[at++] = i; });
+    if (threadIdx.x == 0) m.runs[nruns] = nseg;
+    __syncthreads();
+    const int waves0 = (nseg + 148 * DSEG - 1) / (148 * DSEG), even = (nseg + 148 * waves0 - 1) / (148 * waves0);
+    const int size[4] = {even, min(DSEG, even * 5 / 4), min(DSEG, even * 3 / 2), min(DSEG, even * 2)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        int p = 0;
+        for (int r = threadIdx.x; r < nruns; r += D_THREADS) p += (m.runs[r + 1] - m.runs[r] + size[k] - 1) / size[k];
+        if (p) atomicAdd(&m.pieces[k], p);
+    }
+    __syncthreads();
+    int waves = 0x7fffffff, total = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int w = (m.pieces[k] + 147) / 148;
+        if (w < waves) { waves = w; per = size[k]; total = m.pieces[k]; }
+    }
+    if (60LL * waves > 185 + nseg / 548) { per = -gper; return gpieces; }
+    return total;
+}
+
+// stage the cumulated frequencies and coarse entries of NSYM symbols of a compact table from s0 on; a coarse entry outside of them
+// becomes the nearest of them
+template <int NSYM> SG_DEVINL void stage_table(const uint8_t* __restrict__ ct, uint8_t* dst, int s0, int lane) {
     const unsigned* __restrict__ words = reinterpret_cast<const unsigned*>(ct + 256);
-    for (int i = lane; i < 64; i += 32) reinterpret_cast<unsigned*>(dst)[i] = reinterpret_cast<const unsigned*>(ct)[i];
+    for (int i = lane; i < 64; i += 32) {
+        const unsigned v = reinterpret_cast<const unsigned*>(ct)[i];
+        unsigned o = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o |= (unsigned)clampi((int)((v >> (8 * k)) & 255u) - s0, 0, NSYM - 1) << (8 * k);
+        reinterpret_cast<unsigned*>(dst)[i] = o;
+    }
     unsigned short* cum = reinterpret_cast<unsigned short*>(dst + 256);
-    for (int i = lane; i < nsym; i += 32) cum[i] = (unsigned short)(words[i] >> 16);
-    if (lane == 0) {
-        const unsigned w = words[nsym - 1];
-        const unsigned tot = (w >> 16) + (w & 0xffffu);
-        cum[nsym] = (unsigned short)tot;
-        cum[nsym + 1] = (unsigned short)tot;
-        if (tot != (1u << PB)) bad = 1;
+    for (int i = lane; i < NSYM + 2; i += 32) {
+        const unsigned w = words[min(s0 + i, 255)];
+        cum[i] = (unsigned short)((w >> 16) + (s0 + i > 255 ? w & 0xffffu : 0u));
     }
 }
-typedef RingReader<DSEG> DecRing;
 // The staged search stops at the second symbol of a bucket: a third one (rare symbols share a bucket) sets `miss`, and the
-// weight is decoded again with a walk.  So the usual steps have no branch.
-template <int NSYM> SG_DEVINL unsigned get_staged(unsigned& x, DecRing& r, const uint8_t* t, bool& miss) {
+// weight is decoded again with a walk.  So the usual steps have no branch.  BELOW: there may be symbols before the staged ones.
+template <bool BELOW> SG_DEVINL unsigned get_staged(unsigned& x, DecRing& r, const uint8_t* t, bool& miss) {
     const unsigned short* cum = reinterpret_cast<const unsigned short*>(t + 256);
     const unsigned slot = x & ((1u << PB) - 1), xs = x >> PB;
-    unsigned s = t[slot >> (PB - 8)];
-    if (NSYM < 256) s &= NSYM - 1;                               // (an unused table's place holds anything)
+    const unsigned s = t[slot >> (PB - 8)];
     const unsigned c0 = cum[s], c1 = cum[s + 1], c2 = cum[s + 2];
     const bool up = slot >= c1;
-    miss |= slot >= c2;
+    miss |= slot >= c2 || (BELOW && slot < c0);
     const unsigned lo = up ? c1 : c0, hi = up ? c2 : c1;
     x = (hi - lo) * xs + (slot - lo);
     r.renorm(x);
     return s + up;
 }
-template <int NSYM> SG_DEVINL unsigned get_walk(unsigned& x, DecRing& r, const uint8_t* t) {
+// false: the symbol is not among the staged ones
+template <int NSYM> SG_DEVINL bool get_walk(unsigned& x, DecRing& r, const uint8_t* t, unsigned& sym) {
     const unsigned short* cum = reinterpret_cast<const unsigned short*>(t + 256);
     const unsigned slot = x & ((1u << PB) - 1);
     unsigned s = t[slot >> (PB - 8)];
-    if (NSYM < 256) s &= NSYM - 1;
 #pragma unroll 1
-    while (slot >= cum[s + 1] && s < NSYM - 1) ++s;
-    const unsigned lo = cum[s];
-    x = (cum[s + 1] - lo) * (x >> PB) + (slot - lo);
+    while (slot >= cum[s + 1] && s < NSYM) ++s;
+    const unsigned lo = cum[s], hi = cum[s + 1];
+    if (slot < lo || slot >= hi) return false;
+    x = (hi - lo) * (x >> PB) + (slot - lo);
     r.renorm(x);
-    return s;
+    sym = s;
+    return true;
 }
-SG_DEVINL unsigned get_global(unsigned& x, DecRing& r, const uint8_t* __restrict__ ct) {
+template <class R> SG_DEVINL unsigned get_global(unsigned& x, R& r, const uint8_t* __restrict__ ct) {
     const unsigned* __restrict__ words = reinterpret_cast<const unsigned*>(ct + 256);
     const unsigned slot = x & ((1u << PB) - 1);
     unsigned s = ct[slot >> (PB - 8)];
@@ -318,64 +392,114 @@ SG_DEVINL unsigned get_global(unsigned& x, DecRing& r, const uint8_t* __restrict
     r.renorm(x);
     return s;
 }
-__global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __restrict__ in, const unsigned long long* __restrict__ in_off,
-                                                         const unsigned long long* __restrict__ in_end, unsigned char* __restrict__ dev,
-                                                         const TB* __restrict__ tb, const SG* __restrict__ sg, int nseg, int per, Ctx c,
-                                                         const unsigned char* __restrict__ lut, int* __restrict__ status) {
-    extern __shared__ __align__(16) unsigned char dsm[];
-    DecSmem& m = *reinterpret_cast<DecSmem*>(dsm);
-    const bool chain = threadIdx.x < D_CHAIN;
+// exponent, mantissa and the sign's frequencies from the role's tables in global memory
+template <class R> SG_DEVINL void weight_global(unsigned& x, R& r, const uint8_t* __restrict__ tl, int pe, int sc, int pred, unsigned& ex,
+                                                unsigned& man, unsigned& f01) {
+    ex = get_global(x, r, tl + (size_t)pe * RANS_COMPACT);
+    man = get_global(x, r, tl + (size_t)(512 + mctx((int)ex, pred)) * RANS_COMPACT);
+    const unsigned* sw = reinterpret_cast<const unsigned*>(tl + (size_t)(640 + sc) * RANS_COMPACT + 256);
+    f01 = (sw[0] & 0xffffu) | (sw[1] << 16);
+}
+template <class R> SG_DEVINL bool get_sign(unsigned& x, R& r, unsigned f01) {
+    const unsigned slot = x & ((1u << PB) - 1), f0 = f01 & 0xffffu;
+    const bool neg = slot >= f0;                                 // (two symbols: the second one starts where the first ends)
+    x = (neg ? f01 >> 16 : f0) * (x >> PB) + (slot - (neg ? f0 : 0u));
+    r.renorm(x);
+    return neg;
+}
+
+struct DecArgs {
+    const unsigned char* in; const unsigned long long* in_off; const unsigned long long* in_end;
+    unsigned char* dev; const TB* tb; const SG* sg; Ctx c; const unsigned char* lut; int* status;
+};
+// a piece of segments of one role
+SG_DEVINL void dec_staged(DecSmem& m, const DecArgs& a, int first, int count) {
+    const Ctx& c = a.c;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int first = blockIdx.x * per;
-    const int pair = warp & 7, grp = chain ? (lane < DSEG / 8 ? 8 * lane + pair : DSEG) : 8 * (lane / DG) + pair, gl = lane % DG;
+    const bool chain = warp < D_PAIRS;
+    // as many pairs as every scheduler of the SM gets alike: 21 segments in four pairs 4.86 ms, in five 5.31, seven 5.10, eleven 5.72;
+    // 42 in eight 5.47, in eleven 5.99
+    const int npair = count <= 24 ? 4 : count <= 48 ? 8 : D_PAIRS;
+    const int pair = chain ? warp : warp - D_PAIRS, sub = chain ? lane : lane / DG, grp = npair * sub + pair, gl = lane % DG;
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); };
     const int s = first + grp;
-    const bool live = grp < per && s < nseg;
+    const bool live = pair < npair && sub < 8 && grp < count;
     SG g; g.t = 0; g.n = 0; g.i0 = 0;
-    if (live) g = sg[s];
-    const TB T = tb[g.t];
-    const int cta_tab = tb[sg[first].t].tab;
+    if (live) g = a.sg[s];
+    const TB T = a.tb[g.t];
+    const uint8_t* tl = a.lut + (size_t)a.tb[a.sg[first].t].tab * RANS_COMPACT;
     if (threadIdx.x == 0) {
-        const SG f = sg[first];
-        const TB F = tb[f.t];
+        const SG f = a.sg[first];
+        const TB F = a.tb[f.t];
         const int rc = (int)(f.i0 / F.rowlen), j = (int)(f.i0 % F.rowlen);
         int pred, pe, sc; contexts(c, F, F.rmap >= 0 ? c.rowmap[F.rmap + rc] : rc, j, pred, pe, sc);
-        m.pe0 = min(max(pe - D_ECTX / 2, 0), 512 - D_ECTX);
+        m.pe0 = clampi(pe - D_ECTX / 2, 0, 512 - D_ECTX);
+        m.ex0 = clampi(((pred + 952 + 64) >> 3) - 44, 0, 256 - D_ESYM);    // weights mostly lie below the typical magnitude
         m.nmax = 0; m.bad = 0;
     }
     __syncthreads();
-    const int pe0 = m.pe0;
+    const int pe0 = m.pe0, ex0 = m.ex0;
     if (chain && live) atomicMax(&m.nmax, g.n);
     for (int t = warp; t < D_MCTX + D_ECTX; t += D_THREADS / 32) {
         if (t < D_MCTX) {
-            const uint8_t* ct = lut + (size_t)(cta_tab + 512 + t) * RANS_COMPACT;
-            int bad = 0;
-            stage_table(ct, m.mant + t * D_MP, 128, lane, bad);
-            // a used table whose distribution goes on past symbol 127 (no encoder writes one): this CTA stays with global memory
-            const unsigned w = reinterpret_cast<const unsigned*>(ct + 256)[255];
-            if (bad && (w >> 16) + (w & 0xffffu) == (1u << PB)) m.bad = 1;
-        } else {
-            int bad = 0;
-            stage_table(lut + (size_t)(cta_tab + pe0 + t - D_MCTX) * RANS_COMPACT, m.expo + (t - D_MCTX) * D_EP, 256, lane, bad);
-        }
+            const uint8_t* ct = tl + (size_t)(512 + t) * RANS_COMPACT;
+            stage_table<128>(ct, m.mant + t * D_MP, 0, lane);
+            // a distribution that goes on past symbol 127 (no encoder writes one): this CTA stays with global memory
+            const unsigned w = reinterpret_cast<const unsigned*>(ct + 256)[127], z = reinterpret_cast<const unsigned*>(ct + 256)[255];
+            if ((w >> 16) + (w & 0xffffu) != (z >> 16) + (z & 0xffffu)) m.bad = 1;
+        } else stage_table<D_ESYM>(tl + (size_t)(pe0 + t - D_MCTX) * RANS_COMPACT, m.expo + (t - D_MCTX) * D_EP, ex0, lane);
     }
     if (threadIdx.x < 16) {
-        const unsigned* w = reinterpret_cast<const unsigned*>(lut + (size_t)(cta_tab + 640 + threadIdx.x) * RANS_COMPACT + 256);
+        const unsigned* w = reinterpret_cast<const unsigned*>(tl + (size_t)(640 + threadIdx.x) * RANS_COMPACT + 256);
         m.sign[threadIdx.x] = (w[0] & 0xffffu) | (w[1] << 16);
     }
     __syncthreads();
-    const bool staged = T.tab == cta_tab && !m.bad;
+    const bool staged = !m.bad;
     const int nbatch = (m.nmax + DB - 1) / DB;
-    DecRing rd; rd.pos = rd.have = 0; rd.left = 0;
-    unsigned x = RANS_L;
-    bool bad = false;
-    if (chain && live) { rd.init(in + in_off[s], in + in_end[s], m.ring + grp); x = rd.state(); }
-    unsigned short* base = reinterpret_cast<unsigned short*>(dev + T.doff);
-    // a staging lane's first weight of the batch to stage and of the batch to store: compact row, column
-    int rc = 0, j = 0, orc = 0, oj = 0;
-    if (!chain && live) { const long long i = g.i0 + DW * gl; orc = rc = (int)(i / T.rowlen); oj = j = (int)(i % T.rowlen); }
-    for (int it = 0; it < nbatch + 2; ++it) {
-        if (!chain) {
+    if (chain) {
+        DecRing rd; rd.pos = rd.have = 0; rd.left = 0;
+        unsigned x = RANS_L;
+        bool bad = false;
+        if (live) { rd.init(a.in + a.in_off[s], a.in + a.in_end[s], m.ring + grp); x = rd.state(); }
+        pair_sync();
+        for (int it = 0; it < nbatch; ++it) {
+            if (live && !bad) {
+                const int n = min(DB, g.n - it * DB);
+                const unsigned* cx = m.ctx[it & 1][grp];
+                unsigned short* o = m.out[it & 1][grp];
+#pragma unroll 1
+                for (int w = 0; w < n; ++w) {
+                    if ((w & 3) == 0) rd.top_up();               // four weights take 24 bytes at most
+                    const unsigned e = cx[w];
+                    const int pe = e & 511, sc = (e >> 9) & 15, pred = (int)e >> 16;
+                    const unsigned x0 = x, top0 = rd.top, pos0 = rd.pos;
+                    const bool near = staged && (unsigned)(pe - pe0) < (unsigned)D_ECTX;
+                    const uint8_t* te = m.expo + (near ? pe - pe0 : 0) * D_EP;
+                    bool miss = !near;
+                    unsigned ex = ex0 + get_staged<true>(x, rd, te, miss);
+                    unsigned man = get_staged<false>(x, rd, m.mant + mctx((int)ex, pred) * D_MP, miss);
+                    unsigned f01 = m.sign[sc];
+                    if (miss) {
+                        x = x0; rd.top = top0; rd.pos = pos0;
+                        if (near && get_walk<D_ESYM>(x, rd, te, ex)) {
+                            ex += ex0;
+                            if (!get_walk<127>(x, rd, m.mant + mctx((int)ex, pred) * D_MP, man)) bad = true;     // (no table there: a damaged stream)
+                        } else weight_global(x, rd, tl, pe, sc, pred, ex, man, f01);
+                    }
+                    const bool neg = get_sign(x, rd, f01);
+                    o[w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
+                }
+                bad |= rd.over();
+            }
+            pair_sync();
+        }
+        if (live && (bad || rd.over() || x != RANS_L || !rd.at_end())) atomicOr(a.status, SG_ST_CORRUPT);
+    } else {
+        unsigned short* base = reinterpret_cast<unsigned short*>(a.dev + T.doff);
+        // a staging lane's first weight of the batch to stage and of the batch to store: compact row, column
+        int rc = 0, j = 0, orc = 0, oj = 0;
+        if (live) { const long long i = g.i0 + DW * gl; orc = rc = (int)(i / T.rowlen); oj = j = (int)(i % T.rowlen); }
+        for (int it = 0; it < nbatch + 2; ++it) {
             if (live && it >= 2) {                               // store the batch that was decoded in the last turn
                 int r = orc, col = oj, have = -1, orow = 0;
 #pragma unroll
@@ -401,8 +525,7 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
 #pragma unroll
                     for (int v = 0; v < DW; ++v) {
                         int pred, pe, sc; contexts(c, T, T.rmap >= 0 ? c.rowmap[T.rmap + r[v]] : r[v], col[v], pred, pe, sc);
-                        // (mctx() is constant outside of +-4000)
-                        e[v] = (unsigned)pe | (unsigned)sc << 9 | (unsigned)clampi(pred, -4000, 4000) << 16;
+                        e[v] = pack_ctx(pred, pe, sc);
                     }
 #pragma unroll
                     for (int v = 0; v < DW; ++v) m.ctx[it & 1][grp][DW * gl + v] = e[v];
@@ -410,47 +533,90 @@ __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const unsigned char* __
                 j += DB;
                 while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
             }
-        } else if (live && it >= 1 && !bad) {
-            const int n = min(DB, g.n - (it - 1) * DB);
-            const unsigned* cx = m.ctx[(it - 1) & 1][grp];
-            unsigned short* o = m.out[(it - 1) & 1][grp];
+            if (it <= nbatch) pair_sync();
+        }
+    }
+}
+// segments of any roles: for every 32 weights the four lanes of a segment look the contexts up side by side, the first of them runs
+// the chain over them, all four store
+SG_DEVINL void dec_general(DecSmem& m, const DecArgs& a, int first, int count) {
+    const Ctx& c = a.c;
+    const int grp = threadIdx.x / DG, gl = threadIdx.x % DG, s = first + grp;
+    const bool live = grp < count;
+    SG g; g.t = 0; g.n = 0; g.i0 = 0;
+    if (live) g = a.sg[s];
+    const TB T = a.tb[g.t];
+    const uint8_t* tl = a.lut + (size_t)T.tab * RANS_COMPACT;
+    const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(g.n, 0));
+    RingReader<G_RING> rd; rd.pos = rd.have = 0; rd.left = 0;
+    unsigned x = RANS_L;
+    if (live && gl == 0) { rd.init(a.in + a.in_off[s], a.in + a.in_end[s], m.g_ring + grp); x = rd.state(); }
+    unsigned short* base = reinterpret_cast<unsigned short*>(a.dev + T.doff);
+    int rc = 0, j = 0;                                           // this lane's first weight of the batch: compact row, column
+    if (live) { const long long i = g.i0 + DW * gl; rc = (int)(i / T.rowlen); j = (int)(i % T.rowlen); }
+    bool bad = false;
+    for (int k0 = 0; k0 < nmax; k0 += DB) {
+        size_t at[DW];
+        {
+            int r = rc, col = j, have = -1, orow = 0;
+#pragma unroll
+            for (int v = 0; v < DW; ++v) {
+                at[v] = 0;
+                if (k0 + DW * gl + v < g.n) {
+                    if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
+                    int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
+                    m.g_ctx[grp][DW * gl + v] = pack_ctx(pred, pe, sc);
+                    at[v] = (size_t)orow * T.rowlen + col;
+                    if (++col == T.rowlen) { col = 0; ++r; }
+                }
+            }
+        }
+        __syncwarp();
+        if (live && gl == 0 && !bad) {
+            const int n = min(DB, g.n - k0);
 #pragma unroll 1
             for (int w = 0; w < n; ++w) {
-                if ((w & 3) == 0) rd.top_up();                   // four weights take 24 bytes at most
-                const unsigned e = cx[w];
-                const int pe = e & 511, sc = (e >> 9) & 15, pred = (int)e >> 16;
-                const unsigned x0 = x, top0 = rd.top;
-                const unsigned pos0 = rd.pos;
-                const bool near = staged && (unsigned)(pe - pe0) < (unsigned)D_ECTX;
-                const uint8_t* te = m.expo + (near ? pe - pe0 : 0) * D_EP;
-                bool miss = !near;
-                unsigned ex = get_staged<256>(x, rd, te, miss);
-                unsigned man = get_staged<128>(x, rd, m.mant + mctx((int)ex, pred) * D_MP, miss);
-                unsigned f01 = m.sign[sc];
-                if (miss) {
-                    x = x0; rd.top = top0; rd.pos = pos0;
-                    if (near) {
-                        ex = get_walk<256>(x, rd, te);
-                        man = get_walk<128>(x, rd, m.mant + mctx((int)ex, pred) * D_MP);
-                    } else {
-                        const uint8_t* tl = lut + (size_t)T.tab * RANS_COMPACT;
-                        ex = get_global(x, rd, tl + (size_t)pe * RANS_COMPACT);
-                        man = get_global(x, rd, tl + (size_t)(512 + mctx((int)ex, pred)) * RANS_COMPACT);
-                        const unsigned* sw = reinterpret_cast<const unsigned*>(tl + (size_t)(640 + sc) * RANS_COMPACT + 256);
-                        f01 = (sw[0] & 0xffffu) | (sw[1] << 16);
-                    }
-                }
-                const unsigned slot = x & ((1u << PB) - 1), f0 = f01 & 0xffffu;
-                const bool neg = slot >= f0;                     // (two symbols: the second one starts where the first ends)
-                x = (neg ? f01 >> 16 : f0) * (x >> PB) + (slot - (neg ? f0 : 0u));
-                rd.renorm(x);
-                o[w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
+                if ((w & 3) == 0) rd.top_up();
+                const unsigned e = m.g_ctx[grp][w];
+                unsigned ex, man, f01;
+                weight_global(x, rd, tl, e & 511, (e >> 9) & 15, (int)e >> 16, ex, man, f01);
+                const bool neg = get_sign(x, rd, f01);
+                m.g_out[grp][w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
             }
             bad = rd.over();
         }
-        pair_sync();
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < DW; ++v)
+            if (k0 + DW * gl + v < g.n) base[at[v]] = m.g_out[grp][DW * gl + v];
+        j += DB;
+        if (live) while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
     }
-    if (chain && live && (bad || rd.over() || x != RANS_L || !rd.at_end())) atomicOr(status, SG_ST_CORRUPT);
+    if (live && gl == 0 && (bad || rd.over() || x != RANS_L || !rd.at_end())) atomicOr(a.status, SG_ST_CORRUPT);
+}
+__global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const DecArgs a, int nseg) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    DecSmem& m = *reinterpret_cast<DecSmem*>(dsm);
+    int per;
+    const int pieces = dec_plan(m, a.tb, a.sg, nseg, per);
+    for (int b = blockIdx.x; b < pieces; b += gridDim.x) {
+        if (per < 0) { dec_general(m, a, -per * b, min(-per, nseg + per * b)); continue; }       // (its warps are on their own)
+        if (threadIdx.x == 0) {
+            int at = 0, r = 0, k;
+            for (;; ++r) {
+                k = (m.runs[r + 1] - m.runs[r] + per - 1) / per;
+                if (b < at + k) break;
+                at += k;
+            }
+            const long long len = m.runs[r + 1] - m.runs[r];
+            m.first = m.runs[r] + (int)(len * (b - at) / k);
+            m.count = m.runs[r] + (int)(len * (b - at + 1) / k) - m.first;
+        }
+        __syncthreads();
+        const int first = m.first, count = m.count;
+        dec_staged(m, a, first, count);
+        __syncthreads();
+    }
 }
 
 // duplicate rows copied from their source rows after decoding (bf16v2.py:475-480): pairs = (dup row, source row)
@@ -698,16 +864,17 @@ extern "C" int sg_r2_decode(int device, void* stream, const unsigned char* in, c
     int rc = r2_common(dev, tb, sgp, nseg, rfi, cfi, scl);
     if (rc != SG_OK) return rc;
     if (!in || !in_off || !in_end || !enc_tab || !lut) return SG_ERR_ARG;
-    if ((uintptr_t)in % 16 || (uintptr_t)lut % 8) return SG_ERR_ALIGN;           // (the sign tables' two words are one 8-byte load)
+    if ((uintptr_t)in % 16 || (uintptr_t)lut % 8) return SG_ERR_ALIGN;
     if (nseg == 0) return SG_OK;
     rc = use_device(device);
     if (rc != SG_OK) return rc;
     Ctx c = {rfi, cfi, scl, rowmap};
     rc = cuda_ok(cudaFuncSetAttribute(k_r2_dec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecSmem)));
     if (rc != SG_OK) return rc;
-    const int want = (nseg + 147) / 148, per = want > DSEG ? DSEG : want;
-    k_r2_dec<<<(nseg + per - 1) / per, D_THREADS, sizeof(DecSmem), (cudaStream_t)stream>>>(in, in_off, in_end, dev, (const TB*)tb, (const SG*)sgp,
-                                                                                           nseg, per, c, lut, status_word(device));
+    // the number of pieces is known to the kernel only: twice what segments of one role need, the CTAs without a piece end at once
+    const long long grid = 2LL * 148 * ((nseg + 148LL * DSEG - 1) / (148 * DSEG));
+    k_r2_dec<<<(unsigned)(grid < nseg ? grid : nseg), D_THREADS, sizeof(DecSmem), (cudaStream_t)stream>>>(
+        DecArgs{in, in_off, in_end, dev, (const TB*)tb, (const SG*)sgp, c, lut, status_word(device)}, nseg);
     return cuda_ok(cudaGetLastError());
 }
 

@@ -231,3 +231,80 @@ def test_lattice_decoder_with_many_segments(t):
     one = [(file, pred, 0, 30, 256, 0)]                          # the same blocks in few segments
     buf = codec.encode(t, one, seed, imx)
     assert torch.equal(codec.decode(t, buf, [it[1:] for it in one], seed, imx), file)
+
+
+# how the base decoder cuts its segments: one wave of CTAs with several chains a warp, two waves, runs of two roles, runs too short to
+# be decoded with the role's tables staged (three waves of them; more runs than the kernel lists), a table the stage has no room for
+BASE_CUTS = {
+    "one role": (12000, lambda i: 0, None), "two waves": (15000, lambda i: 0, None), "runs": (9001, lambda i: i // 700 % 3, None),
+    "short runs": (500, lambda i: i % 2, None), "many runs": (1100, lambda i: i % 2, None), "symbol past 127": (600, lambda i: i // 300, 200),
+}
+
+
+@pytest.mark.parametrize("name", BASE_CUTS)
+def test_base_decoder_cuts(name):
+    """many segments of 1 to 100 weights, rows over several octaves and some zeros: the weights come back bit for bit"""
+    import ctypes
+
+    import torch
+    from seedpack_b200 import _lib
+    from seedpack_b200.rans import normalize
+    nseg, role, extra = BASE_CUTS[name]
+    L, dev = _lib.lib(), torch.device("cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    call = lambda fn, *a: _lib.check(getattr(L, fn)(0, st, *a), fn)
+    rng = np.random.default_rng(len(name))
+    ns = rng.integers(1, 101, nseg)
+    roles = np.array([role(i) for i in range(nseg)])
+    starts = np.flatnonzero(np.r_[True, roles[1:] != roles[:-1]])                # a tensor per run of one role, of 37 columns
+    ends = np.r_[starts[1:], nseg]
+    cols, sizes = 37, np.array([int(ns[a:b].sum()) for a, b in zip(starts, ends)])
+    rows = -(-sizes // cols)
+    rowbase = np.r_[0, np.cumsum(rows)]
+    at = int(rowbase[-1]) * cols
+    tb = np.zeros(len(sizes), np.dtype([("doff", "<i8"), ("rowlen", "<i4"), ("rowbase", "<i4"), ("colbase", "<i4"), ("tab", "<i4"), ("rmap", "<i4"), ("pad", "<i4")]))
+    segs = []
+    for t, (a, b) in enumerate(zip(starts, ends)):
+        tb[t] = (2 * rowbase[t] * cols, cols, rowbase[t], t * cols, roles[a] * 656, -1, 0)
+        segs += list(zip([t] * (b - a), ns[a:b].tolist(), (np.cumsum(ns[a:b]) - ns[a:b]).tolist()))
+    sg = np.array(segs, np.dtype([("t", "<i4"), ("n", "<i4"), ("i0", "<i8")]))
+    tb, sg = torch.from_numpy(tb.view(np.uint8)).cuda(), torch.from_numpy(sg.view(np.uint8)).cuda()
+    g = torch.Generator(device="cuda").manual_seed(nseg)
+    w = torch.randn(at, generator=g, device=dev) * torch.exp2(torch.randint(-3, 4, (at // cols, 1), generator=g, device=dev).float()).expand(-1, cols).reshape(-1)
+    w = torch.where(torch.rand(at, generator=g, device=dev) < 0.01, 0, w).to(torch.bfloat16).view(torch.int16)
+    # side information from the weights: whole eighths of an octave a row and a column, a class a column
+    rfi = torch.randint(-24, 25, (at // cols,), generator=g, device=dev).to(torch.int16)
+    cfi = torch.randint(-8, 9, (cols * len(sizes),), generator=g, device=dev).to(torch.int16)
+    scl = torch.randint(0, 16, (cols * len(sizes),), generator=g, device=dev).to(torch.int8)
+    none = torch.zeros(1, dtype=torch.int32, device=dev)
+    side = (p(rfi), p(cfi), p(scl), p(none))
+    ntab = 656 * (int(roles.max()) + 1)
+    counts = torch.zeros(ntab * 256, dtype=torch.int32, device=dev)
+    call("sg_r2_hist", p(w), p(tb), p(sg), nseg, *side, p(counts))
+    assert int(counts.sum()) == 3 * int(ns.sum())
+    freq, used = normalize(counts.cpu().numpy().reshape(ntab, 256), 1 << 15)
+    full = np.zeros((ntab, 256), np.uint16)
+    full[used] = freq
+    if extra is not None:
+        row = full[512 + np.flatnonzero(full[512:640].any(1))[0]]
+        row[int(row.argmax())] -= 5
+        row[extra] = 5
+    f = torch.from_numpy(full.view(np.int16)).cuda()
+    enc, lut = torch.empty(ntab * 512, dtype=torch.int32, device=dev), torch.empty(ntab * 1280, dtype=torch.uint8, device=dev)
+    call("sg_rans_tables", p(f), ntab, 15, p(enc), p(lut))
+    cap = 1024
+    slots, lens = torch.empty(nseg * cap, dtype=torch.uint8, device=dev), torch.empty(nseg, dtype=torch.int32, device=dev)
+    call("sg_r2_encode", p(w), p(tb), p(sg), nseg, *side, p(enc), p(slots), cap, p(lens))
+    total = int(lens.sum(dtype=torch.int64))
+    assert int(lens.min()) >= 4 and total < nseg * cap
+    stream, off = torch.zeros((total + 31) // 16 * 16, dtype=torch.uint8, device=dev), torch.empty(nseg + 1, dtype=torch.int64, device=dev)
+    call("sg_scan_gather", p(slots), cap, p(lens), nseg, p(stream), total, p(off))
+    back = torch.full_like(w, -1)
+    call("sg_r2_decode", p(stream), p(off), p(off[1:]), p(back), p(tb), p(sg), nseg, *side, p(enc), p(lut))
+    bits = ctypes.c_int(0)
+    _lib.check(L.sg_status_fetch(0, st, ctypes.byref(bits)), "sg_status_fetch")
+    coded = torch.zeros(at, dtype=torch.bool, device=dev)                        # (a tensor's last row may reach past its segments)
+    for r, k in zip(rowbase, sizes):
+        coded[int(r) * cols:int(r) * cols + int(k)] = True
+    assert bits.value == 0 and torch.equal(back[coded], w[coded]) and bool((back[~coded] == -1).all())
