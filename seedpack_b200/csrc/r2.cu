@@ -47,38 +47,87 @@ SG_DEVINL void contexts(const Ctx& c, const TB& T, int orow, int j, int& pred, i
 }
 SG_DEVINL int mctx(int ex, int pred) { return clampi(8 * ex - pred - 1016 + 64, 0, 127); }
 
+// The exponent context whose neighbourhood of 64 to either side holds the most of the first weights of the segments first .. first
+// + n - 1 (those of the role `tab`; n <= WIN_MAX): one of them alone may lie in a row of zeros.  By the whole CTA.
+constexpr int WIN_MAX = 96;
+struct WinSmem { int pe[WIN_MAX], best; };
+SG_DEVINL int window_of(WinSmem& m, const Ctx& c, const TB* __restrict__ tb, const SG* __restrict__ sg, int first, int n, int tab) {
+    const int t = threadIdx.x;
+    __syncthreads();
+    if (t == 0) m.best = 0;
+    if (t < n) {
+        const SG g = sg[first + t];
+        const TB T = tb[g.t];
+        int pred, pe = -1024, sc;
+        if (T.tab == tab && g.n > 0) {
+            const int rc = (int)(g.i0 / T.rowlen), j = (int)(g.i0 % T.rowlen);
+            contexts(c, T, T.rmap >= 0 ? c.rowmap[T.rmap + rc] : rc, j, pred, pe, sc);
+        }
+        m.pe[t] = pe;
+    }
+    __syncthreads();
+    if (t < n && m.pe[t] >= 0) {
+        int k = 0;
+        for (int j = 0; j < n; ++j) k += (unsigned)(m.pe[j] - m.pe[t] + 64) < 128u;
+        atomicMax(&m.best, k << 9 | m.pe[t]);
+    }
+    __syncthreads();
+    return m.best & 511;
+}
+// the lowest of 64 exponents to keep at hand around such a context: weights mostly lie below the typical magnitude
+SG_DEVINL int window_exponent(int pe) { return ((pe - 256 + 1016) >> 3) - 44; }
+// add to global memory, once for the lanes that come with the same counter (rows of zeros do)
+SG_DEVINL void hadd(unsigned* counts, unsigned key) {
+    const unsigned m = __match_any_sync(__activemask(), key);
+    if ((threadIdx.x & 31) == (unsigned)(__ffs(m) - 1)) atomicAdd(counts + key, (unsigned)__popc(m));
+}
+
 // Counts do not depend on the order of the weights.  A CTA takes `per` segments, as few as give two CTAs per SM their share,
 // and its 16 warps walk through a segment together (coalesced reads, four weights per lane in flight).  Bound by the shared
 // memory's atomics, three per weight.  Mantissa symbols are spread over 128 x 128 counters per role, which a CTA collects in
-// shared memory (64 KB) and adds to global memory at its end; so are the exponent symbols inside a window of 128 contexts x
-// 64 exponents around the CTA's first weight (weights of one tensor keep to a few octaves; what falls outside the window
-// goes to global memory directly).  Of the sign's 32 counters every lane has its own copy: they would collide on every step.
-constexpr int R2H_THREADS = 512, R2H_U = 4;
+// shared memory (64 KB) and adds to global memory when the role changes and at its end (about the time of a segment); so are
+// the exponent symbols inside a window of 128 contexts x 64 exponents (weights of one tensor keep to a few octaves; what falls
+// outside the window goes to global memory directly).  Of the sign's 32 counters every lane has its own
+// copy: they would collide on every step.
+constexpr int R2H_THREADS = 512, R2H_U = 4, R2H_OWN = 4096;
 constexpr int R2H_SMEM = (128 * 128 + 128 * 64 + 32 * 32) * 4;
 __global__ void __launch_bounds__(R2H_THREADS, 2) k_r2_hist(const unsigned char* __restrict__ dev, const TB* __restrict__ tb,
                                                             const SG* __restrict__ sg, int nseg, int per, Ctx c, unsigned* __restrict__ counts) {
-    extern __shared__ unsigned mhist[];            // [128 contexts][128 symbols] of the role of the CTA's first segment
+    extern __shared__ unsigned mhist[];            // [128 contexts][128 symbols] of the role `tab`
+    __shared__ WinSmem win;
     unsigned* ehist = mhist + 128 * 128;           // [128 contexts from pe0][64 exponents from ex0] of the same role
     unsigned* shist = ehist + 128 * 64;            // [16 classes x sign][lane] of the same role
-    __shared__ int win[2];
     for (int i = threadIdx.x; i < R2H_SMEM / 4; i += R2H_THREADS) mhist[i] = 0;
     const int lane = threadIdx.x & 31, first = blockIdx.x * per;
-    const int cta_tab = tb[sg[first].t].tab;
-    if (threadIdx.x == 0) {
-        const SG g = sg[first];
-        const TB T = tb[g.t];
-        const int rc = (int)(g.i0 / T.rowlen), j = (int)(g.i0 % T.rowlen);
-        const int orow = T.rmap >= 0 ? c.rowmap[T.rmap + rc] : rc;
-        const unsigned u = reinterpret_cast<const unsigned short*>(dev + T.doff)[(size_t)orow * T.rowlen + j];
-        int pred, pe, sc; contexts(c, T, orow, j, pred, pe, sc);
-        win[0] = pe - 64; win[1] = (int)((u >> 7) & 255) - 40;      // weights mostly lie below the typical magnitude
-    }
-    __syncthreads();
-    const int pe0 = win[0], ex0 = win[1];
+    int tab = -1, pe0 = 0, ex0 = 0;
+    auto add_up = [&]() {                          // what was collected to global memory, the counters back to zero
+        __syncthreads();
+        unsigned* gt = counts + (size_t)tab * 256;
+        for (int i = threadIdx.x; i < 128 * 128; i += R2H_THREADS) {
+            const unsigned v = mhist[i];
+            if (v) { atomicAdd(gt + (512 + (i >> 7)) * 256 + (i & 127), v); mhist[i] = 0; }
+        }
+        for (int i = threadIdx.x; i < 128 * 64; i += R2H_THREADS) {
+            const unsigned v = ehist[i];
+            if (v) { atomicAdd(gt + (pe0 + (i >> 6)) * 256 + ex0 + (i & 63), v); ehist[i] = 0; }
+        }
+        for (int i = threadIdx.x >> 5; i < 32; i += R2H_THREADS / 32) {
+            const unsigned v = __reduce_add_sync(0xffffffffu, shist[i * 32 + lane]);
+            if (v && lane == 0) atomicAdd(gt + (640 + (i >> 1)) * 256 + (i & 1), v);
+            shist[i * 32 + lane] = 0;
+        }
+    };
     for (int s = first; s < min(nseg, first + per); ++s) {
         const SG g = sg[s];
         const TB T = tb[g.t];
-        const bool local = T.tab == cta_tab;
+        // another role: its own counters, unless the segment is too small to be worth clearing them
+        if (T.tab != tab && (tab < 0 || g.n >= R2H_OWN)) {
+            if (tab >= 0) add_up();
+            tab = T.tab;
+            const int pe = window_of(win, c, tb, sg, s, min(WIN_MAX, min(nseg, first + per) - s), tab);
+            pe0 = pe - 64; ex0 = window_exponent(pe);
+        }
+        const bool local = T.tab == tab;
         unsigned* gt = counts + (size_t)T.tab * 256;
         // this lane's weight: compact row rc, column j; a CTA's width further every time (no division inside the loop)
         const int dr = R2H_THREADS / T.rowlen, dj = R2H_THREADS % T.rowlen;
@@ -102,31 +151,18 @@ __global__ void __launch_bounds__(R2H_THREADS, 2) k_r2_hist(const unsigned char*
                 if (k0 + v * R2H_THREADS >= g.n) break;
                 const int ex = (u[v] >> 7) & 255, man = u[v] & 127, sgn = u[v] >> 15, mc = mctx(ex, pred[v]);
                 if (local && (unsigned)(pe[v] - pe0) < 128u && (unsigned)(ex - ex0) < 64u) atomicAdd(ehist + (pe[v] - pe0) * 64 + (ex - ex0), 1u);
-                else atomicAdd(gt + pe[v] * 256 + ex, 1u);
+                else hadd(gt, pe[v] * 256 + ex);
                 if (local) {
                     atomicAdd(mhist + mc * 128 + man, 1u);
                     atomicAdd(shist + (sc[v] * 2 + sgn) * 32 + lane, 1u);
                 } else {
-                    atomicAdd(gt + (512 + mc) * 256 + man, 1u);
-                    atomicAdd(gt + (640 + sc[v]) * 256 + sgn, 1u);
+                    hadd(gt, (512 + mc) * 256 + man);
+                    hadd(gt, (640 + sc[v]) * 256 + sgn);
                 }
             }
         }
     }
-    __syncthreads();
-    unsigned* gt = counts + (size_t)cta_tab * 256;
-    for (int i = threadIdx.x; i < 128 * 128; i += R2H_THREADS) {
-        const unsigned v = mhist[i];
-        if (v) atomicAdd(gt + (512 + (i >> 7)) * 256 + (i & 127), v);
-    }
-    for (int i = threadIdx.x; i < 128 * 64; i += R2H_THREADS) {
-        const unsigned v = ehist[i];
-        if (v) atomicAdd(gt + (pe0 + (i >> 6)) * 256 + ex0 + (i & 63), v);
-    }
-    for (int i = threadIdx.x >> 5; i < 32; i += R2H_THREADS / 32) {
-        const unsigned v = __reduce_add_sync(0xffffffffu, shist[i * 32 + lane]);
-        if (v && lane == 0) atomicAdd(gt + (640 + (i >> 1)) * 256 + (i & 1), v);
-    }
+    add_up();
 }
 
 // Encoder.  What a weight's three symbols are coded with depends on the data only, not on the coder state, and a segment's
