@@ -26,20 +26,6 @@ struct Ctx {
     const short* rfi; const short* cfi; const signed char* scl; const int* rowmap;
 };
 
-// position of a lane inside its tensor: compact row rc (after duplicate-row removal), column j, original row
-struct Cursor {
-    TB T; int rc, j, orow; const unsigned short* w;
-    SG_DEVINL void seek(const unsigned char* dev, const TB& t, long long i, const int* rowmap) {
-        T = t; rc = (int)(i / T.rowlen); j = (int)(i % T.rowlen);
-        orow = T.rmap >= 0 ? rowmap[T.rmap + rc] : rc;
-        w = reinterpret_cast<const unsigned short*>(dev + T.doff) + (size_t)orow * T.rowlen;
-    }
-    SG_DEVINL void row(const unsigned char* dev, const int* rowmap) {
-        orow = T.rmap >= 0 ? rowmap[T.rmap + rc] : rc;
-        w = reinterpret_cast<const unsigned short*>(dev + T.doff) + (size_t)orow * T.rowlen;
-    }
-};
-
 SG_DEVINL void contexts(const Ctx& c, const TB& T, int orow, int j, int& pred, int& pe, int& sc) {
     pred = c.rfi[T.rowbase + orow] + c.cfi[T.colbase + j];
     pe = clampi(pred + 256, 0, 511);
@@ -292,29 +278,31 @@ __global__ void __launch_bounds__(E_THREADS) k_r2_enc(const unsigned char* __res
 // that holds every 128th slot; anything else goes through the tables in global memory.
 // Pieces: the segments come in runs of one role, cut evenly.  A CTA of two roles, one of them without tables, took three times
 // as long (28 layers of seven projections, layer by layer: 36.6 ms; 22.5 with no tables in shared memory at all).  Runs that are
-// too short for that are decoded from global memory, four lanes a segment, 192 segments a CTA: see dec_plan().
+// too short for that are decoded by k_r2_dec_any from global memory, four lanes a segment: see dec_plan().
 constexpr int DB = 32, DG = 4, DW = DB / DG;                     // weights per batch, lanes per segment in the staging warps and their weights
 constexpr int D_PAIRS = 12, DSEG = 8 * D_PAIRS, D_THREADS = 2 * 32 * D_PAIRS, D_RING = 128;
 constexpr int D_ECTX = 128, D_ESYM = 64, D_MCTX = 128, D_MP = 256 + 260, D_EP = 256 + 132;     // bytes per table: 256 coarse, 130 / 66 cumulated
 constexpr int GSEG = D_THREADS / DG, G_RING = 256;               // segments of a CTA that decodes from global memory
 constexpr int D_RUNS = 1024;
-struct DecSmem {
+struct PlanSmem {
     int runs[D_RUNS + 1], warp_sum[D_THREADS / 32], pieces[4], first, count;
-    int nmax, pe0, ex0, bad;
-    union {
-        struct {
-            unsigned ring[RING_ROWS * D_RING];
-            unsigned ctx[2][DSEG][DB + 1];                       // pe | sc << 9 | pred << 16; rows padded
-            unsigned sign[16];                                   // frequency of symbol 0 | of symbol 1 << 16
-            unsigned short out[2][DSEG][DB + 2];
-            uint8_t mant[D_MCTX * D_MP], expo[D_ECTX * D_EP];
-        };
-        struct {
-            unsigned g_ring[RING_ROWS * G_RING];
-            unsigned g_ctx[GSEG][DB + 1];
-            unsigned short g_out[GSEG][DB + 2];
-        };
-    };
+    int v_pe[D_THREADS], v_tab[D_THREADS], v_best[64];
+};
+struct DecSmem {
+    PlanSmem plan;
+    WinSmem win;
+    int nmax, bad;
+    unsigned ring[RING_ROWS * D_RING];
+    unsigned ctx[2][DSEG][DB + 1];                               // pe | sc << 9 | pred << 16; rows padded
+    unsigned sign[16];                                           // frequency of symbol 0 | of symbol 1 << 16
+    unsigned short out[2][DSEG][DB + 2];
+    uint8_t mant[D_MCTX * D_MP], expo[D_ECTX * D_EP];
+};
+struct AnySmem {
+    PlanSmem plan;
+    unsigned ring[RING_ROWS * G_RING];
+    unsigned ctx[GSEG][DB + 1];
+    unsigned short out[GSEG][DB + 2];
 };
 static_assert(sizeof(DecSmem) <= 227 * 1024, "one CTA per SM");
 typedef RingReader<D_RING> DecRing;
@@ -323,8 +311,10 @@ SG_DEVINL unsigned pack_ctx(int pred, int pe, int sc) { return (unsigned)pe | (u
 
 // How the segments are cut, the same in every CTA: the pieces' number and size; a negative size: pieces of any roles.  A wave of
 // pieces takes 4.9 ms with 21 segments each and 6.4 ms with 83, so what counts is the number of waves: a larger piece is
-// taken where that saves one.  Segments of any roles, from global memory: 19.7 ms for 6000, 23 for 26000 (in runs of ten).
-SG_DEVINL int dec_plan(DecSmem& m, const TB* __restrict__ tb, const SG* __restrict__ sg, int nseg, int& per) {
+// taken where that saves one.  Segments of any roles, from global memory: 14.3 ms for 6000 in runs of ten, 17.7 for 26000, the
+// same again for every further 28416 (192 an SM).  They are decoded that way too if the rows' magnitudes are spread over more
+// contexts than a piece has room for (rows over 40 octaves: 8.1 ms for 6144 segments, 13.6 in pieces).
+SG_DEVINL int dec_plan(PlanSmem& m, const Ctx& c, const TB* __restrict__ tb, const SG* __restrict__ sg, int nseg, int& per) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int chunk = (nseg + D_THREADS - 1) / D_THREADS;
     const int i0 = (int)min((long long)threadIdx.x * chunk, (long long)nseg), i1 = (int)min((long long)i0 + chunk, (long long)nseg);
@@ -368,7 +358,37 @@ SG_DEVINL int dec_plan(DecSmem& m, const TB* __restrict__ tb, const SG* __restri
         const int w = (m.pieces[k] + 147) / 148;
         if (w < waves) { waves = w; per = size[k]; total = m.pieces[k]; }
     }
-    if (60LL * waves > 185 + nseg / 548) { per = -gper; return gpieces; }
+    __syncthreads();
+    // and how many weights' contexts a piece's window would hold: twelve segments of each of 64 stretches as long as a piece
+    const int q = threadIdx.x / 12, i = min((int)((long long)q * nseg / 64) + (int)(threadIdx.x % 12) * per / 12, nseg - 1);
+    {
+        const SG g = sg[i];
+        const TB T = tb[g.t];
+        int pred, pe = -1024, sc;
+        if (g.n > 0) {
+            const int rc = (int)(g.i0 / T.rowlen), j = (int)(g.i0 % T.rowlen);
+            contexts(c, T, T.rmap >= 0 ? c.rowmap[T.rmap + rc] : rc, j, pred, pe, sc);
+        }
+        m.v_pe[threadIdx.x] = pe; m.v_tab[threadIdx.x] = T.tab;
+        if (threadIdx.x < 64) m.v_best[threadIdx.x] = 0;
+        if (threadIdx.x < 2) m.pieces[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    {
+        int held = 0, same = 0;
+        for (int k = 12 * q; k < 12 * q + 12; ++k) {
+            const bool of_role = m.v_tab[k] == m.v_tab[threadIdx.x];
+            same += of_role;
+            held += of_role && (unsigned)(m.v_pe[k] - m.v_pe[threadIdx.x] + 64) < 128u;
+        }
+        atomicMax(&m.v_best[q], held << 8 | same);
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) { atomicAdd(&m.pieces[0], m.v_best[threadIdx.x] >> 8); atomicAdd(&m.pieces[1], m.v_best[threadIdx.x] & 255); }
+    __syncthreads();
+    // (a lane outside the window holds up its warp: with 16 of 17 inside 9.9 ms, from global memory 8.1)
+    if (64LL * waves > 133LL * gwaves + nseg / 600 || 20 * m.pieces[0] < 19 * m.pieces[1]) { per = -gper; total = gpieces; }
+    __syncthreads();
     return total;
 }
 
@@ -463,18 +483,11 @@ SG_DEVINL void dec_staged(DecSmem& m, const DecArgs& a, int first, int count) {
     SG g; g.t = 0; g.n = 0; g.i0 = 0;
     if (live) g = a.sg[s];
     const TB T = a.tb[g.t];
-    const uint8_t* tl = a.lut + (size_t)a.tb[a.sg[first].t].tab * RANS_COMPACT;
-    if (threadIdx.x == 0) {
-        const SG f = a.sg[first];
-        const TB F = a.tb[f.t];
-        const int rc = (int)(f.i0 / F.rowlen), j = (int)(f.i0 % F.rowlen);
-        int pred, pe, sc; contexts(c, F, F.rmap >= 0 ? c.rowmap[F.rmap + rc] : rc, j, pred, pe, sc);
-        m.pe0 = clampi(pe - D_ECTX / 2, 0, 512 - D_ECTX);
-        m.ex0 = clampi(((pred + 952 + 64) >> 3) - 44, 0, 256 - D_ESYM);    // weights mostly lie below the typical magnitude
-        m.nmax = 0; m.bad = 0;
-    }
-    __syncthreads();
-    const int pe0 = m.pe0, ex0 = m.ex0;
+    const int tab = a.tb[a.sg[first].t].tab;
+    const uint8_t* tl = a.lut + (size_t)tab * RANS_COMPACT;
+    if (threadIdx.x == 0) { m.nmax = 0; m.bad = 0; }
+    const int pe_mid = window_of(m.win, c, a.tb, a.sg, first, count, tab);
+    const int pe0 = clampi(pe_mid - D_ECTX / 2, 0, 512 - D_ECTX), ex0 = clampi(window_exponent(pe_mid), 0, 256 - D_ESYM);
     if (chain && live) atomicMax(&m.nmax, g.n);
     for (int t = warp; t < D_MCTX + D_ECTX; t += D_THREADS / 32) {
         if (t < D_MCTX) {
@@ -575,7 +588,7 @@ SG_DEVINL void dec_staged(DecSmem& m, const DecArgs& a, int first, int count) {
 }
 // segments of any roles: for every 32 weights the four lanes of a segment look the contexts up side by side, the first of them runs
 // the chain over them, all four store
-SG_DEVINL void dec_general(DecSmem& m, const DecArgs& a, int first, int count) {
+SG_DEVINL void dec_any(AnySmem& m, const DecArgs& a, int first, int count) {
     const Ctx& c = a.c;
     const int grp = threadIdx.x / DG, gl = threadIdx.x % DG, s = first + grp;
     const bool live = grp < count;
@@ -586,7 +599,7 @@ SG_DEVINL void dec_general(DecSmem& m, const DecArgs& a, int first, int count) {
     const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(g.n, 0));
     RingReader<G_RING> rd; rd.pos = rd.have = 0; rd.left = 0;
     unsigned x = RANS_L;
-    if (live && gl == 0) { rd.init(a.in + a.in_off[s], a.in + a.in_end[s], m.g_ring + grp); x = rd.state(); }
+    if (live && gl == 0) { rd.init(a.in + a.in_off[s], a.in + a.in_end[s], m.ring + grp); x = rd.state(); }
     unsigned short* base = reinterpret_cast<unsigned short*>(a.dev + T.doff);
     int rc = 0, j = 0;                                           // this lane's first weight of the batch: compact row, column
     if (live) { const long long i = g.i0 + DW * gl; rc = (int)(i / T.rowlen); j = (int)(i % T.rowlen); }
@@ -601,7 +614,7 @@ SG_DEVINL void dec_general(DecSmem& m, const DecArgs& a, int first, int count) {
                 if (k0 + DW * gl + v < g.n) {
                     if (r != have) { orow = T.rmap >= 0 ? c.rowmap[T.rmap + r] : r; have = r; }
                     int pred, pe, sc; contexts(c, T, orow, col, pred, pe, sc);
-                    m.g_ctx[grp][DW * gl + v] = pack_ctx(pred, pe, sc);
+                    m.ctx[grp][DW * gl + v] = pack_ctx(pred, pe, sc);
                     at[v] = (size_t)orow * T.rowlen + col;
                     if (++col == T.rowlen) { col = 0; ++r; }
                 }
@@ -613,46 +626,59 @@ SG_DEVINL void dec_general(DecSmem& m, const DecArgs& a, int first, int count) {
 #pragma unroll 1
             for (int w = 0; w < n; ++w) {
                 if ((w & 3) == 0) rd.top_up();
-                const unsigned e = m.g_ctx[grp][w];
+                const unsigned e = m.ctx[grp][w];
                 unsigned ex, man, f01;
                 weight_global(x, rd, tl, e & 511, (e >> 9) & 15, (int)e >> 16, ex, man, f01);
                 const bool neg = get_sign(x, rd, f01);
-                m.g_out[grp][w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
+                m.out[grp][w] = (unsigned short)(((unsigned)neg << 15) | (ex << 7) | man);
             }
             bad = rd.over();
         }
         __syncwarp();
 #pragma unroll
         for (int v = 0; v < DW; ++v)
-            if (k0 + DW * gl + v < g.n) base[at[v]] = m.g_out[grp][DW * gl + v];
+            if (k0 + DW * gl + v < g.n) base[at[v]] = m.out[grp][DW * gl + v];
         j += DB;
         if (live) while (j >= T.rowlen) { j -= T.rowlen; ++rc; }
     }
     if (live && gl == 0 && (bad || rd.over() || x != RANS_L || !rd.at_end())) atomicOr(a.status, SG_ST_CORRUPT);
 }
+// Which of the two ways it is depends on the records, which only the device sees: both kernels are launched, work it out and the one
+// that has nothing to do ends (some 10 us).  They are two so that the tables of the second find the L1 that the first's shared
+// memory takes from it (rows over 40 octaves: 14.9 ms with both in one, 8.1).
 __global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec(const DecArgs a, int nseg) {
     extern __shared__ __align__(16) unsigned char dsm[];
     DecSmem& m = *reinterpret_cast<DecSmem*>(dsm);
+    PlanSmem& pl = m.plan;
     int per;
-    const int pieces = dec_plan(m, a.tb, a.sg, nseg, per);
+    const int pieces = dec_plan(pl, a.c, a.tb, a.sg, nseg, per);
+    if (per < 0) return;
     for (int b = blockIdx.x; b < pieces; b += gridDim.x) {
-        if (per < 0) { dec_general(m, a, -per * b, min(-per, nseg + per * b)); continue; }       // (its warps are on their own)
         if (threadIdx.x == 0) {
             int at = 0, r = 0, k;
             for (;; ++r) {
-                k = (m.runs[r + 1] - m.runs[r] + per - 1) / per;
+                k = (pl.runs[r + 1] - pl.runs[r] + per - 1) / per;
                 if (b < at + k) break;
                 at += k;
             }
-            const long long len = m.runs[r + 1] - m.runs[r];
-            m.first = m.runs[r] + (int)(len * (b - at) / k);
-            m.count = m.runs[r] + (int)(len * (b - at + 1) / k) - m.first;
+            const long long len = pl.runs[r + 1] - pl.runs[r];
+            pl.first = pl.runs[r] + (int)(len * (b - at) / k);
+            pl.count = pl.runs[r] + (int)(len * (b - at + 1) / k) - pl.first;
         }
         __syncthreads();
-        const int first = m.first, count = m.count;
+        const int first = pl.first, count = pl.count;
         dec_staged(m, a, first, count);
         __syncthreads();
     }
+}
+__global__ void __launch_bounds__(D_THREADS, 1) k_r2_dec_any(const DecArgs a, int nseg) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    AnySmem& m = *reinterpret_cast<AnySmem*>(dsm);
+    int per;
+    const int pieces = dec_plan(m.plan, a.c, a.tb, a.sg, nseg, per);
+    if (per > 0) return;
+    per = -per;
+    for (int b = blockIdx.x; b < pieces; b += gridDim.x) dec_any(m, a, b * per, min(per, nseg - b * per));     // (its warps are on their own)
 }
 
 // duplicate rows copied from their source rows after decoding (bf16v2.py:475-480): pairs = (dup row, source row)
@@ -907,10 +933,15 @@ extern "C" int sg_r2_decode(int device, void* stream, const unsigned char* in, c
     Ctx c = {rfi, cfi, scl, rowmap};
     rc = cuda_ok(cudaFuncSetAttribute(k_r2_dec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecSmem)));
     if (rc != SG_OK) return rc;
+    rc = cuda_ok(cudaFuncSetAttribute(k_r2_dec_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AnySmem)));
+    if (rc != SG_OK) return rc;
+    const DecArgs args = {in, in_off, in_end, dev, (const TB*)tb, (const SG*)sgp, c, lut, status_word(device)};
     // the number of pieces is known to the kernel only: twice what segments of one role need, the CTAs without a piece end at once
-    const long long grid = 2LL * 148 * ((nseg + 148LL * DSEG - 1) / (148 * DSEG));
-    k_r2_dec<<<(unsigned)(grid < nseg ? grid : nseg), D_THREADS, sizeof(DecSmem), (cudaStream_t)stream>>>(
-        DecArgs{in, in_off, in_end, dev, (const TB*)tb, (const SG*)sgp, c, lut, status_word(device)}, nseg);
+    const long long grid = 2LL * 148 * ((nseg + 148LL * DSEG - 1) / (148 * DSEG)), any = 148LL * ((nseg + 148LL * GSEG - 1) / (148 * GSEG));
+    k_r2_dec<<<(unsigned)(grid < nseg ? grid : nseg), D_THREADS, sizeof(DecSmem), (cudaStream_t)stream>>>(args, nseg);
+    rc = cuda_ok(cudaGetLastError());
+    if (rc != SG_OK) return rc;
+    k_r2_dec_any<<<(unsigned)(any < nseg ? any : nseg), D_THREADS, sizeof(AnySmem), (cudaStream_t)stream>>>(args, nseg);
     return cuda_ok(cudaGetLastError());
 }
 

@@ -234,10 +234,12 @@ def test_lattice_decoder_with_many_segments(t):
 
 
 # how the base decoder cuts its segments: one wave of CTAs with several chains a warp, two waves, runs of two roles, runs too short to
-# be decoded with the role's tables staged (three waves of them; more runs than the kernel lists), a table the stage has no room for
+# be decoded with the role's tables staged (four waves of them; more runs than the kernel lists), a table the stage has no room for,
+# rows over more octaves than it has room for
 BASE_CUTS = {
-    "one role": (12000, lambda i: 0, None), "two waves": (15000, lambda i: 0, None), "runs": (9001, lambda i: i // 700 % 3, None),
-    "short runs": (500, lambda i: i % 2, None), "many runs": (1100, lambda i: i % 2, None), "symbol past 127": (600, lambda i: i // 300, 200),
+    "one role": (12000, lambda i: 0, None, 24), "two waves": (15000, lambda i: 0, None, 24), "runs": (9001, lambda i: i // 700 % 3, None, 24),
+    "short runs": (500, lambda i: i % 2, None, 24), "many runs": (1100, lambda i: i % 2, None, 24),
+    "symbol past 127": (600, lambda i: i // 300, 200, 24), "many octaves": (5000, lambda i: i // 1000, None, 200),
 }
 
 
@@ -249,7 +251,7 @@ def test_base_decoder_cuts(name):
     import torch
     from seedpack_b200 import _lib
     from seedpack_b200.rans import normalize
-    nseg, role, extra = BASE_CUTS[name]
+    nseg, role, extra, spread = BASE_CUTS[name]
     L, dev = _lib.lib(), torch.device("cuda")
     p = lambda t: ctypes.c_void_p(t.data_ptr())
     st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
@@ -274,7 +276,8 @@ def test_base_decoder_cuts(name):
     w = torch.randn(at, generator=g, device=dev) * torch.exp2(torch.randint(-3, 4, (at // cols, 1), generator=g, device=dev).float()).expand(-1, cols).reshape(-1)
     w = torch.where(torch.rand(at, generator=g, device=dev) < 0.01, 0, w).to(torch.bfloat16).view(torch.int16)
     # side information from the weights: whole eighths of an octave a row and a column, a class a column
-    rfi = torch.randint(-24, 25, (at // cols,), generator=g, device=dev).to(torch.int16)
+    rfi = torch.randint(-spread, spread + 1, (at // cols,), generator=g, device=dev).to(torch.int16)
+    rfi[torch.rand(at // cols, generator=g, device=dev) < 0.03] = -797           # (what a row of zeros has)
     cfi = torch.randint(-8, 9, (cols * len(sizes),), generator=g, device=dev).to(torch.int16)
     scl = torch.randint(0, 16, (cols * len(sizes),), generator=g, device=dev).to(torch.int8)
     none = torch.zeros(1, dtype=torch.int32, device=dev)
