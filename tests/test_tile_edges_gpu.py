@@ -44,6 +44,19 @@ def test_dequantize_values():
     assert np.array_equal(gq.dequantize(2, torch.from_numpy(y).cuda()).cpu().numpy().reshape(-1, 32), want)
 
 
+@pytest.mark.parametrize("t", [2, 3, 6, 7, 8, 10, 11, 12, 13, 14, 16, 17, 18, 19, 20, 21, 22, 23, 29, 42])
+def test_dequantize_equals_the_formulas(t):
+    """random blocks against the layouts and formulas in NumPy, exact (NaN where the scale is one)"""
+    import torch
+    from seedpack_b200.gpuquant import GPUQuant
+    from seedpack_b200.requant import QFUN
+    from tests.dequant_model import dequantize
+    _, qk, bs = QFUN[t]
+    y = np.random.default_rng(100 + t).integers(0, 256, (4096 // qk + 300) * bs, dtype=np.uint8)
+    got = GPUQuant().dequantize(t, torch.from_numpy(y).cuda()).cpu().numpy()
+    assert np.array_equal(got.reshape(-1, qk), dequantize(t, y, bs), equal_nan=True)
+
+
 R2_SHAPES = [(1, 1, 0), (5, 37, 0), (3, 16384, 0), (64, 1000, 1), (700, 4099, 1)]
 
 
