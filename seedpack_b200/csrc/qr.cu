@@ -298,7 +298,8 @@ struct QrDec {
     SG_DEVINL int get(int tab) { return step(tab, f01[tab]); }
 };
 SG_DEVINL void or_byte(unsigned* blk, int i, unsigned v) { atomicOr(blk + (i >> 2), (v & 255u) << (8 * (i & 3))); }
-// put_code with the bits OR-ed into a zeroed block in shared memory, safe for lanes that share a byte
+// a code's bits OR-ed into a zeroed block in shared memory, safe for lanes that share a byte (4-bit single-part codes go in
+// unmasked, qr.py:156-175)
 SG_DEVINL void put_code_shared(int T, unsigned* blk, int w, int q) {
     const CodeLoc L = code_loc(T, w);
     if (T == 8) { or_byte(blk, L.lo_byte, (unsigned)q); return; }

@@ -52,8 +52,6 @@ SG_DEVINL float h2fv(unsigned h) {
     return __uint_as_float(f);
 }
 SG_DEVINL int u16(const uchar* b) { return b[0] | (b[1] << 8); }
-SG_DEVINL unsigned u32(const uchar* b) { return b[0] | (b[1] << 8) | (b[2] << 16) | ((unsigned)b[3] << 24); }
-SG_DEVINL float h2f(const uchar* p) { return h2fv((unsigned)u16(p)); }
 
 constexpr __host__ SG_DEVINL int qk_of(int T) { return (T == 2 || T == 3 || T == 6 || T == 7 || T == 8 || T == 20) ? 32 : T == 42 ? 64 : 256; }
 constexpr __host__ SG_DEVINL int bs_of(int T) {
@@ -116,16 +114,6 @@ SG_DEVINL int get_code(int T, const uchar* b, int w) {
     int q = (b[L.lo_byte] >> L.lo_shift) & ((1 << L.lo_bits) - 1);
     if (L.hi_bits) q |= ((b[L.hi_byte] >> L.hi_shift) & ((1 << L.hi_bits) - 1)) << L.lo_bits;
     return q;
-}
-// bits are OR-ed in: the code bytes must be zero before
-SG_DEVINL void put_code(int T, uchar* b, int w, int q) {
-    const CodeLoc L = code_loc(T, w);
-    if (T == 8) { b[L.lo_byte] = (uchar)q; return; }
-    if (L.hi_bits) {
-        b[L.lo_byte] |= (uchar)((q & ((1 << L.lo_bits) - 1)) << L.lo_shift);
-        b[L.hi_byte] |= (uchar)(((q >> L.lo_bits) & ((1 << L.hi_bits) - 1)) << L.hi_shift);
-    } else if (L.lo_bits == 2) b[L.lo_byte] |= (uchar)((q & 3) << L.lo_shift);
-    else b[L.lo_byte] |= (uchar)(q << L.lo_shift);           // 4-bit single-part codes are OR-ed in unmasked (qr.py:156-175)
 }
 
 // ---- scale fields ------------------------------------------------------------------------------------------
