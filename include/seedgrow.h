@@ -242,7 +242,8 @@ SG_API int sg_qr_decode(int device, void *stream, int T, const unsigned char *in
  * dev = buffer holding the tensors (TB.doff = byte offset), rfi / cfi / scl = side information (int16 per row, int16 and
  * int8 per column), rowmap = compact-to-original row numbers of tensors with duplicate rows removed (TB.rmap >= 0).
  * Tables are addressed by raw id (role * 656 + context): counts has nroles * 656 * 256 entries; enc_tab / lut come
- * from sg_rans_tables(..., pb = 15).  sg_r2_decode takes the first and one-past-last stream byte of every segment.
+ * from sg_rans_tables(..., pb = 15).  sg_r2_decode takes the first and one-past-last stream byte of every segment; it does not
+ * read enc_tab (lut holds the frequencies too), which must be given all the same.
  * sg_r2_stats writes rfi[nrows], cfi[rowlen], scl[rowlen] of one tensor; scratch from sg_r2_stats_scratch_bytes. */
 SG_API int sg_r2_hist(int device, void *stream, const unsigned char *dev, const void *tb, const void *sg, int nseg,
                       const short *rfi, const short *cfi, const signed char *scl, const int *rowmap, unsigned *counts);
