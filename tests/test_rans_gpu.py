@@ -158,3 +158,17 @@ def test_compact_tables_leave_nothing_unwritten():
     for b in range(256):                                       # the symbol whose range holds slot 128 b
         s = l[1, b]
         assert cum[s] <= 128 * b < cum[s] + f[1, s]
+
+
+@pytest.mark.parametrize("nseg", [148 * 256 + 77, 148 * 64 + 1])
+def test_many_segments(nseg):
+    """more segments of 64 symbols than the decoder's CTAs and the encoder's warps take in one wave, the last ones partly filled"""
+    from seedpack_b200.rans import RansCodec
+    c = RansCodec()
+    sym, bt = synth_stream(nseg * 64 - 32, 32, 294, seed=nseg)
+    r = c.encode(_dev(sym), _dev(bt), 32, 294, seg_len=64)
+    full = np.zeros((294, 256), np.uint16); full[r["used"]] = r["freq"]
+    want, woff = orans.encode(sym, bt, 32, 64, full)
+    assert np.array_equal(r["off"].cpu().numpy().astype(np.uint64), woff) and np.array_equal(r["stream"].cpu().numpy()[:r["total"]], want)
+    out = c.decode(r["stream"], r["off"], _dev(bt), 32, len(sym), r["freq"], r["used"], 294, seg_len=64)
+    assert c.status() == 0 and np.array_equal(out.cpu().numpy(), sym)
